@@ -1258,7 +1258,8 @@ static int batch_layout(ct_fan_batch *b) {
         io += npx;
         so += nr;
         fb += (nr + b->fp_block - 1) / b->fp_block;
-        bb += (npx + b->bp_block - 1) / b->bp_block;
+        const int per = fan_batch_bp_pixels(b->bp_block);
+        bb += (npx + per - 1) / per;
     }
     CT_REQUIRE(fb < (1LL << 31) && bb < (1LL << 31), "batch too large for one launch");
     b->img_total = io;

@@ -1,7 +1,7 @@
 // fan2d.cu -- single-slice 2D fan- and parallel-beam projectors and
 // backprojectors (device code in fan2d_dev.cuh).  One thread per ray for the
-// forward projectors, one thread per pixel (all views, sum in a register,
-// written once) for the backprojectors.
+// forward projectors; for the backprojectors one thread per pixel and run of
+// views, the runs' sums added in a fixed order and each pixel written once.
 #include "fan2d_dev.cuh"
 
 namespace ct {
@@ -39,19 +39,20 @@ fan_fp_kernel(const FanGeom g, const float *__restrict__ img, OutT *__restrict__
     }
 }
 
+constexpr int F2_BP_BLOCK = 256;
+// blocks per SM the registers aim at: 4 (64 registers)
 template <int WMODE, bool UPDATE>
-__global__ void __launch_bounds__(F2_BLOCK)
+__global__ void __launch_bounds__(F2_BP_BLOCK, 4)
 fan_bp_kernel(const FanGeom g, const float *__restrict__ R, float *__restrict__ img,
               const float *__restrict__ colsum, float eps, float lambda, float lo, float hi) {
-    const int i = blockIdx.x * F2_BLOCK + threadIdx.x;
-    if (i >= g.nt * g.ns) return;
-    const float acc = fan_pixel_sum<WMODE>(g, R, i);
-    if (UPDATE) {
-        const float x = img[i] + lambda * acc / (colsum[i] + eps);
-        img[i] = fminf(fmaxf(x, lo), hi);
-    } else {
-        img[i] = acc;
-    }
+    fan_bp_block<WMODE>(g, R, (int)blockIdx.x * fan_bp_pixels(F2_BP_BLOCK), [&](int i, float acc) {
+        if (UPDATE) {
+            const float x = img[i] + lambda * acc / (colsum[i] + eps);
+            img[i] = fminf(fmaxf(x, lo), hi);
+        } else {
+            img[i] = acc;
+        }
+    });
 }
 
 }  // namespace
@@ -107,8 +108,9 @@ int fan_bp_launch(const FanGeom &g0, const float *R, float *img, int wmode, cons
     FanGeom g = g0;
     fan_geom_derive(g);
     CT_REQUIRE(g.np >= 2, "fan_bp: at least 2 detector bins");
-    const unsigned blocks = (unsigned)((g.nt * g.ns + F2_BLOCK - 1) / F2_BLOCK);
-#define CT_F2_CASE(W, U) fan_bp_kernel<W, U><<<blocks, F2_BLOCK, 0, st>>>(g, R, img, colsum, eps, lambda, lo, hi)
+    const int per = fan_bp_pixels(F2_BP_BLOCK);
+    const unsigned blocks = (unsigned)(((long long)g.nt * g.ns + per - 1) / per);
+#define CT_F2_CASE(W, U) fan_bp_kernel<W, U><<<blocks, F2_BP_BLOCK, 0, st>>>(g, R, img, colsum, eps, lambda, lo, hi)
     if (update) {
         if (wmode == 0) CT_F2_CASE(BP2_BACKPROJ, true);
         else if (wmode == 1) CT_F2_CASE(BP2_FBPFAN, true);

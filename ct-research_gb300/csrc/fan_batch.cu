@@ -70,29 +70,26 @@ fan_batch_fp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__r
     }
 }
 
-// blocks of 512 threads per SM the batched backprojection's registers aim at:
-// 3 (40 registers, a few bytes spilled by the chord weighting) measured 11.06 ms
-// per backprojection with update on 64 uneven slices, against 11.28 ms at 4
-// and 11.50 ms with the compiler's own choice (64 registers)
-#ifndef CT_FANB_BP_MINB
-#define CT_FANB_BP_MINB 3
-#endif
+// blocks of 512 threads per SM the batched backprojection's registers aim at: 2
+// (64 registers): a SIRT iteration of 64 uneven slices 12.2 ms; 12.4 ms with 112
+// registers, 22 ms with 40 (3 blocks: the loop spills)
 template <int WMODE, bool UPDATE>
-__global__ void __launch_bounds__(512, CT_FANB_BP_MINB)
+__global__ void __launch_bounds__(512, 2)
 fan_batch_bp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__restrict__ R, float *__restrict__ img,
                     const float *__restrict__ colsum, float eps, float lambda, float lo, float hi) {
     const int k = find_slice(sl, nsl, true);
-    const FanGeom g = sl[k].g;
-    const int i = (int)(blockIdx.x - sl[k].pix_blk0) * blockDim.x + threadIdx.x;
-    if (i >= g.nt * g.ns) return;
-    const float acc = fan_pixel_sum<WMODE>(g, R + sl[k].sino_off, i);
-    const long long o = sl[k].img_off + i;
-    if (UPDATE) {
-        const float x = img[o] + lambda * acc / (colsum[o] + eps);
-        img[o] = fminf(fmaxf(x, lo), hi);
-    } else {
-        img[o] = acc;
-    }
+    const FanGeom &g = sl[k].g;
+    const long long img_off = sl[k].img_off;
+    const int pix0 = (int)(blockIdx.x - sl[k].pix_blk0) * fan_bp_pixels(blockDim.x);
+    fan_bp_block<WMODE>(g, R + sl[k].sino_off, pix0, [&](int i, float acc) {
+        const long long o = img_off + i;
+        if (UPDATE) {
+            const float x = img[o] + lambda * acc / (colsum[o] + eps);
+            img[o] = fminf(fmaxf(x, lo), hi);
+        } else {
+            img[o] = acc;
+        }
+    });
 }
 
 }  // namespace
@@ -109,6 +106,8 @@ int fan_batch_fp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block,
     CT_LAUNCH_CHECK("fan_batch_fp_kernel");
     return fan_batch_fixup_launch(d_sl, nsl, img, out, b, rowsum, eps, norms, mode, gl, st);
 }
+
+int fan_batch_bp_pixels(int block) { return fan_bp_pixels(block); }
 
 int fan_batch_bp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block, const float *R, float *img, int wmode,
                         const float *colsum, float eps, float lambda, float lo, float hi, bool update,

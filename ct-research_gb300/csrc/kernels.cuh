@@ -25,6 +25,9 @@ struct FanGeom {
     // near-boundary recompute, so that it runs no FP64
     double ires[2], ext[2];
     float2 res_ff[2], hsize_ff[2], D_ff, ipint_ff;
+    // distance of a bin boundary, in bins, within which the backprojector's FP32
+    // detector coordinate does not decide the bin
+    float near_q;
     // the walk set-up of every ray (fan_ray_table_launch), or null: computed per ray
     const struct FanRay *ray_tab;
 };
@@ -55,6 +58,25 @@ inline void fan_geom_derive(FanGeom &g) {
     }
     g.D_ff = ff_split_host(g.D);
     g.ipint_ff = ff_split_host(1.0 / (double)g.pint);
+    // Error of the FP32 coordinate P Rscan / (Rscan - S) of a pixel within the half
+    // diagonal hd, in units of 2^-24: 2.5 E from P (E the mean extent) times the
+    // largest magnification, and of |Pd| <= Rscan hd / sqrt(Rscan^2 - hd^2) the
+    // product, the reciprocal and Rscan - S's three roundings; a quarter more for
+    // safety.  Then the quotient's: its constants and its own rounding, np bins at
+    // most.  Domains the implied grid does not cover take the float-float path
+    // everywhere (so does a scan whose source is inside the half diagonal).
+    const double hd = 0.5 * std::sqrt(g.size[0] * g.size[0] + g.size[1] * g.size[1]);
+    const double E = 0.5 * (g.size[0] + g.size[1]);
+    const double ulp = 1.0 / 16777216.0;
+    double err = 1.25 * (2.5 * E + hd);
+    if (!g.parallel) {
+        const double far = g.D - hd;
+        err = far > 0.0 ? 1.25 * (2.5 * E * g.D / far + g.D * hd / std::sqrt(far * (g.D + hd)) * (2.5 + 1.5 * (g.D + hd) / far))
+                        : 1e30;
+    }
+    const double q = err * ulp / g.pint + 2.0 * ulp * g.np;
+    const bool grid = g.np <= (1 << 22) && (double)g.maxp - g.minp <= ((double)g.np - 0.5) * g.pint;
+    g.near_q = grid && q < 0.5 ? (float)q : 1.0f;
 }
 
 // Detector-row filter job (filter.cu).
@@ -189,6 +211,8 @@ struct BatchSlice {
 int fan_batch_fp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block, const float *img, float *out,
                         const float *b, const float *rowsum, float eps, double *norms, int mode, const GrazeList &gl,
                         cudaStream_t st);
+// pixels a block of `block` threads of the batched backprojection covers
+int fan_batch_bp_pixels(int block);
 int fan_batch_bp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block, const float *R, float *img, int wmode,
                         const float *colsum, float eps, float lambda, float lo, float hi, bool update,
                         cudaStream_t st);

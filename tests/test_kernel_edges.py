@@ -1,0 +1,48 @@
+"""Kernels at the sizes where their tiles, groups and rules change, against the
+oracle (FP32 against the reference's FP64 arithmetic: rel-L2 <= 1e-5)."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5
+
+
+# (nt, ns), views, bins, detector half width over the image half width, descending, first spacing over the rest
+FAN_BP = [
+    ((5, 3), 1, 2, 1.6, False, 1.0),          # fewer views than groups, one bin pair
+    ((8, 4), 7, 3, 1.6, True, 1.0),
+    ((33, 1), 8, 4, 1.6, False, 1.0),         # two pixel tiles, the second of one lane
+    ((31, 33), 37, 50, 1.6, False, 1.0),
+    ((64, 65), 40, 333, 0.7, True, 1.0),      # truncated detector: off-detector pixels and edge bins
+    ((64, 64), 64, 90, 1.6, False, 1.02),     # uneven samples
+    ((48, 96), 128, 70, 1.6, False, 1.0),     # views on the diagonals: ties of the pixel edges
+]
+
+
+@pytest.mark.parametrize("shape,views,bins,width,down,first", FAN_BP)
+def test_fan_backprojection_groups_and_edges(oracle, shape, views, bins, width, down, first):
+    import torch
+    from ctgb.device import FanPlan
+    from ctgb.geometry import FanGeometry
+    nt, ns = shape
+    rng = np.random.default_rng(nt * views + bins)
+    half = width * 0.5 * max(nt, ns)
+    step = np.full(bins - 1, 1.0)
+    step[0] = first
+    P = np.concatenate([[0.0], np.cumsum(step)])
+    P = (P / P[-1] * 2 - 1) * half
+    P = P[::-1].copy() if down else P
+    beta = np.arange(1, views + 1) * (2 * np.pi / views)
+    size, D = np.array([float(nt), float(ns)]), 2.5 * max(nt, ns)
+    # smooth rows: the FP32 detector coordinate (~1e-7 of the scan's extent) then costs
+    # ~1e-6; on white noise it costs its error in bins, 1.3e-5 at these 0.14 mm bins
+    phase = rng.uniform(0, 6, (views, 1))
+    R = (1.5 + np.cos(phase + np.linspace(0, 5, bins)[None, :])).astype(np.float32)
+    b32, p32 = beta.astype(np.float32), P.astype(np.float32)
+    plan = FanPlan(FanGeometry(nt, ns, tuple(size), beta, P, D))
+    d = torch.from_numpy(R).cuda()
+    assert rel_l2(plan.bp(d).cpu().numpy(), oracle.fan_bp(R, b32, p32, size, (ns, nt), D)) <= TOL
+    filt = oracle.fbpfan_filter(R, p32, D, mode=0)
+    assert rel_l2(plan.fbp(d, filter_mode=0).cpu().numpy(), oracle.fbpfan_bp(filt, b32, p32, size, (ns, nt), D)) <= TOL
