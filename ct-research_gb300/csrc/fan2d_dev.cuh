@@ -267,8 +267,8 @@ __device__ __noinline__ float fan_view_exact(const FanGeom &g, const float *__re
         return val * fan_chord(dx, dy, fan_side_t(dx, a1, a2), ht, hs, __fmul_rn(2.0f, Rs));
     }
     if (WMODE == BP2_FBPFAN) {
-        const float ir = rcp_approx(__fmaf_rn(it, sb, __fmaf_rn(-is, cb, Rs)));
-        return val * __fmul_rn(ir, ir);
+        const float lr = __fmul_rn(rcp_approx(__fsub_rn(Rs, __fmaf_rn(is, cb, -__fmul_rn(it, sb)))), Rs);
+        return val * __fmul_rn(lr, lr);
     }
     return val;
 }
@@ -296,7 +296,7 @@ constexpr int kFanUnroll = 4;
 // Issue-bound: 46 instructions per pixel-view (FBP) and 60 (chord weight), 67%
 // of the issue slots, against ~160 and 132 of the form this replaced, which divided in IEEE and
 // built the unit direction of the line.  One approximate reciprocal of
-// Rscan - S serves P / U and the FBP weight 1 / U^2 (its constants multiply the
+// Rscan - S serves P / U and the FBP weight 1 / U^2 (the constants multiply the
 // sum once, at the end); the floor is an addition rounded down.  Every rounding
 // is written out and the order of the sum depends only on the pixels of the
 // warp and the views, so the single-slice and the batched builds give
@@ -380,7 +380,8 @@ __device__ __forceinline__ float fan_warp_sum(const FanGeom &g, const float *__r
                 w[u] = fan_chord(dx, dy, fan_side_t(dx, a1, a2), ht, hs, R2s);
                 odd[u] = odd[u] || tie[u];
             } else {
-                w[u] = __fmul_rn(ir, ir);
+                const float lr = __fmul_rn(ir, Rs);                              // 1 / U
+                w[u] = __fmul_rn(lr, lr);
             }
             const unsigned pc = min((unsigned)p1[u], inner);                     // for the reads only
             const float *__restrict__ r = Rv + ((long long)(v + u) * np + pc);
@@ -416,13 +417,12 @@ __device__ __forceinline__ float fan_warp_sum(const FanGeom &g, const float *__r
 }
 
 // The view-independent factor of fan_warp_sum's terms: 1 / PInt of the weights,
-// and 2 (chord), dbeta Rscan^2 (of dbeta / U^2) or dtheta.
+// and 2 (chord), dbeta or dtheta.
 template <int WMODE>
 __device__ __forceinline__ float fan_scale(const FanGeom &g) {
     const float ipint = 1.0f / g.pint;
     if (WMODE == BP2_BACKPROJ) return __fmul_rn(2.0f, ipint);
-    if (WMODE == BP2_FBPPAR) return __fmul_rn(ipint, g.bint);
-    return __fmul_rn(__fmul_rn(__fmul_rn(ipint, g.bint), g.D_ff.x), g.D_ff.x);
+    return __fmul_rn(ipint, g.bint);
 }
 
 // Backprojection of the block's pixels pix0 .. pix0 + fan_bp_pixels(blockDim.x):

@@ -46,3 +46,44 @@ def test_fan_backprojection_groups_and_edges(oracle, shape, views, bins, width, 
     assert rel_l2(plan.bp(d).cpu().numpy(), oracle.fan_bp(R, b32, p32, size, (ns, nt), D)) <= TOL
     filt = oracle.fbpfan_filter(R, p32, D, mode=0)
     assert rel_l2(plan.fbp(d, filter_mode=0).cpu().numpy(), oracle.fbpfan_bp(filt, b32, p32, size, (ns, nt), D)) <= TOL
+
+
+# bins around the 4-output groups, the P-tiles (128 fan, 256 cone) and the longest single-pass row; views around the
+# residual row tile of 128
+@pytest.mark.parametrize("views,bins", [(1, 2), (3, 5), (130, 127), (128, 130), (2, 1023), (2, 1024), (2, 1025)])
+@pytest.mark.parametrize("scale", [1.0, 1e-35, 1e33])
+def test_row_filter_tiles_and_scales(oracle, views, bins, scale):
+    """Both orders of the pre-weight on rows at the edges of the kernel's tiles, scaled to the ends of the normal
+    float range (the kernel scales each row to 1)."""
+    import torch
+    from ctgb.device import FanPlan
+    from ctgb.geometry import FanGeometry
+    rng = np.random.default_rng(views + bins)
+    P = np.linspace(-40.0, 40.0, bins)
+    beta = np.arange(1, views + 1) * (2 * np.pi / views)
+    R = (rng.random((views, bins)) * scale).astype(np.float32)
+    p32, b32 = P.astype(np.float32), beta.astype(np.float32)
+    plan = FanPlan(FanGeometry(8, 8, (8.0, 8.0), beta, P, 100.0))
+    for mode in (0, 1):
+        filt = oracle.fbpfan_filter(R, p32, 100.0, mode=mode)
+        ref = oracle.fbpfan_bp(filt, b32, p32, (8.0, 8.0), (8, 8), 100.0)
+        got = plan.fbp(torch.from_numpy(R).cuda(), filter_mode=mode).cpu().numpy()
+        assert rel_l2(got, ref) <= TOL
+
+
+def test_row_filter_infinities_stay_in_their_row():
+    """An infinity or NaN spoils its own row's outputs only."""
+    import torch
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry, centred_domain, view_angles
+    plan = ConePlan(ConeGeometry(4, 4, 4, (4.0, 4.0, 4.0), view_angles(3), centred_domain(300, 0.1),
+                                 centred_domain(5, 0.1), 50.0), fdk_filter=0)
+    R = torch.rand((3, 5, 300), device="cuda")
+    good = plan.fdk_filter(R)
+    bad = R.clone()
+    bad[1, 2, 7] = float("inf")
+    bad[2, 0, 299] = float("nan")
+    out = plan.fdk_filter(bad)
+    assert not torch.isfinite(out[1, 2]).any() and not torch.isfinite(out[2, 0]).any()
+    out[1, 2], out[2, 0] = good[1, 2], good[2, 0]
+    assert torch.equal(out, good)
