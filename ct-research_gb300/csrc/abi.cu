@@ -212,7 +212,7 @@ using namespace ct;
 struct ct_cone_plan {
     ConeGeom g{};
     DevBuf trig, vsrc, P, xi, xtab, vorder, trigf, vsrcf, Pd, xid;
-    DevBuf quads, rcov, G, wtab, norms, volT, volS, cols, pwt, win, scan, bpsum;
+    DevBuf pairs, bptab, rcov, G, wtab, norms, volT, volS, cols, pwt, win, scan, bpsum;
     double cols_res[3] = {0, 0, 0};   // voxel pitch the column table was built for
     GrazeBuf graze;
     int bp_chunk = 0;   // views per backprojection chunk; 0: automatic (cone_bp_chunk_views)
@@ -226,7 +226,7 @@ struct ct_cone_plan {
     ~ct_cone_plan() {
         trig.release(); vsrc.release(); P.release(); xi.release(); xtab.release(); vorder.release();
         trigf.release(); vsrcf.release(); Pd.release(); xid.release();
-        quads.release(); rcov.release(); G.release(); wtab.release(); norms.release(); graze.release();
+        pairs.release(); bptab.release(); rcov.release(); G.release(); wtab.release(); norms.release(); graze.release();
         volT.release(); volS.release(); cols.release(); pwt.release(); win.release(); scan.release(); bpsum.release();
     }
 };
@@ -424,21 +424,19 @@ int ct_cone_plan_set_short_scan(ct_cone_plan *plan, int enable) {
 
 size_t ct_cone_plan_workspace_bytes(const ct_cone_plan *plan) {
     if (!plan) return 0;
-    return plan->quads.bytes + plan->rcov.bytes + plan->G.bytes + plan->wtab.bytes + plan->norms.bytes +
+    return plan->pairs.bytes + plan->bptab.bytes + plan->rcov.bytes + plan->G.bytes + plan->wtab.bytes + plan->norms.bytes +
            plan->graze.buf.bytes + plan->volT.bytes + plan->volS.bytes + plan->cols.bytes + plan->bpsum.bytes;
 }
 
 // Views per backprojection chunk: the caller's setting, else chunks of about
-// kBpChunkBytes of packed quads, evened out over the scan.  Shorter launches
-// keep the views the resident blocks are working on close together, so their
-// quads stay in L2: at 512^3 / 360 views / 768x512 the backprojection took
-// 71.8 ms in one pass, 64.4 / 62.8 / 62.2 / 63.5 ms in chunks of
-// 60 / 90 / 120 / 180 views.
+// kBpChunkBytes at 16 bytes per detector sample, evened out over the scan.
+// Shorter launches keep the views the resident blocks are working on close
+// together, so their samples stay in L2.
 constexpr size_t kBpChunkBytes = size_t(768) << 20;
 static int cone_bp_chunk_views(const ct_cone_plan *plan) {
     const ConeGeom &g = plan->g;
     if (plan->bp_chunk > 0) return std::min(plan->bp_chunk, g.nb);
-    const size_t per_view = cone_quads_bytes(g, 1);
+    const size_t per_view = 16 * (size_t)g.nx * g.np;
     const int target = (int)std::max<size_t>(1, std::min<size_t>(g.nb, kBpChunkBytes / std::max<size_t>(per_view, 1)));
     const int nch = (g.nb + target - 1) / target;
     return (g.nb + nch - 1) / nch;
@@ -507,18 +505,27 @@ int ct_cone_fp_residual(ct_cone_plan *plan, const float *d_vol, const float *d_b
                           1, gl, as_stream(stream));
 }
 
-// Backprojection in chunks of cone_bp_chunk_views views:
-// every chunk is packed into quads and backprojected, its sums added to the
-// volume (or, for the fused SIRT update, to a partial-sum volume that the last
-// chunk folds into the update).
+// Views whose column-view records are held at a time: at most kBpTableBytes of
+// them (360 x 8 MiB at 512^2 columns).
+constexpr size_t kBpTableBytes = size_t(2) << 30;
+static int cone_bp_table_views(const ct_cone_plan *plan, int chunk) {
+    const size_t per_view = cone_bp_table_bytes(plan->g, 1);
+    return (int)std::max<size_t>(1, std::min<size_t>(chunk, kBpTableBytes / per_view));
+}
+
+// Backprojection in chunks of cone_bp_chunk_views views (fewer where their
+// records would not fit): every chunk is packed into pairs and backprojected,
+// its sums added to the volume (or, for the fused SIRT update, to a partial-sum
+// volume that the last chunk folds into the update).
 static int cone_bp_common(ct_cone_plan *plan, const float *d_proj, float *d_vol, int weighting,
                           const float *colsum, float eps, float lambda, float lo, float hi, bool update,
                           cudaStream_t st) {
     const ConeGeom &g = plan->g;
-    const int chunk = cone_bp_chunk_views(plan);
+    const int chunk = cone_bp_table_views(plan, cone_bp_chunk_views(plan));
     const int nchunks = (g.nb + chunk - 1) / chunk;
-    int s = plan->quads.ensure(cone_quads_bytes(g, chunk));
-    if (s) return s;
+    int s;
+    if ((s = plan->pairs.ensure(cone_bp_pairs_bytes(g, chunk))) || (s = plan->bptab.ensure(cone_bp_table_bytes(g, chunk))))
+        return s;
     float *part = nullptr;
     if (update && nchunks > 1) {
         if ((s = plan->bpsum.ensure(sizeof(float) * (size_t)g.nt * g.ns * g.nz))) return s;
@@ -527,11 +534,11 @@ static int cone_bp_common(ct_cone_plan *plan, const float *d_proj, float *d_vol,
     for (int c = 0; c < nchunks; ++c) {
         const int v0 = c * chunk, nv = std::min(chunk, g.nb - v0);
         const bool last = c == nchunks - 1;
-        if ((s = cone_pack_quads(g, d_proj, plan->quads.as<float4>(), v0, nv, st))) return s;
+        if ((s = cone_bp_pack(g, d_proj, plan->pairs.as<float2>(), v0, nv, st))) return s;
         const float *prev = c == 0 ? nullptr : (update ? part : d_vol);
         float *out = (update && !last) ? part : d_vol;
-        if ((s = cone_bp_launch(g, plan->quads.as<float4>(), v0, nv, prev, out, weighting, colsum, eps, lambda, lo,
-                                hi, update && last, st)))
+        if ((s = cone_bp_launch(g, plan->pairs.as<float2>(), plan->bptab.ptr, false, v0, nv, prev, out, weighting, colsum,
+                                eps, lambda, lo, hi, update && last, st)))
             return s;
     }
     return CT_OK;
@@ -1048,15 +1055,16 @@ static int cone_bp_dropin(float *Display, const float *R, const float *xi, const
     DropinState &st = dropin();
     const size_t nv = (size_t)nt * ns * nz, npj = (size_t)nb * np * nx;
     if ((s = st.vol.ensure(nv * sizeof(float))) || (s = st.proj.ensure(npj * sizeof(float)))) return s;
-    const int bchunk = std::min(cone_bp_chunk_views(pl), kDropinChunk * 2);
+    const int bchunk = cone_bp_table_views(pl, std::min(cone_bp_chunk_views(pl), kDropinChunk * 2));
     if (!fdk && nb > bchunk && np >= 2 && nx >= 2 && host_pinned(R) && host_pinned(Display)) {
         // pinned buffers: copy view chunks (the backprojector's own chunks) in,
         // each backprojected (and added to the volume) while the next one arrives;
         // the last chunk runs in z slabs, each copied out while the next is summed
         const int nchunks = (nb + bchunk - 1) / bchunk;
-        const int ztile = cone_bp_ztile(), ntiles = (nz + ztile - 1) / ztile;
+        const int ztile = cone_bp_ztile(pl->g), ntiles = (nz + ztile - 1) / ztile;
         const int nslab = std::min(kDropinSlabs, ntiles);
-        if ((s = dropin_streams(st, nchunks + nslab)) || (s = pl->quads.ensure(cone_quads_bytes(pl->g, bchunk))))
+        if ((s = dropin_streams(st, nchunks + nslab)) || (s = pl->pairs.ensure(cone_bp_pairs_bytes(pl->g, bchunk))) ||
+            (s = pl->bptab.ensure(cone_bp_table_bytes(pl->g, bchunk))))
             return s;
         const size_t per_view = (size_t)np * nx;
         for (int c = 0; c < nchunks; ++c) {
@@ -1070,12 +1078,12 @@ static int cone_bp_dropin(float *Display, const float *R, const float *xi, const
             const int v0 = c * bchunk, n = std::min(bchunk, nb - v0);
             const bool last = c == nchunks - 1;
             CT_CUDA(cudaStreamWaitEvent(st.cs, st.ev[c], 0), "event wait");
-            if ((s = cone_pack_quads(pl->g, st.proj.as<float>(), pl->quads.as<float4>(), v0, n, st.cs))) return s;
+            if ((s = cone_bp_pack(pl->g, st.proj.as<float>(), pl->pairs.as<float2>(), v0, n, st.cs))) return s;
             for (int k = 0; k < (last ? nslab : 1); ++k) {
                 const int t0 = last ? k * ntiles / nslab : 0, t1 = last ? (k + 1) * ntiles / nslab : ntiles;
-                if ((s = cone_bp_launch(pl->g, pl->quads.as<float4>(), v0, n, c == 0 ? nullptr : st.vol.as<float>(),
-                                        st.vol.as<float>(), 0, nullptr, 0.f, 0.f, 0.f, 0.f, false, st.cs, t0,
-                                        t1 - t0)))
+                if ((s = cone_bp_launch(pl->g, pl->pairs.as<float2>(), pl->bptab.ptr, k > 0, v0, n,
+                                        c == 0 ? nullptr : st.vol.as<float>(), st.vol.as<float>(), 0, nullptr, 0.f, 0.f,
+                                        0.f, 0.f, false, st.cs, t0, t1 - t0)))
                     return s;
                 if (last) {
                     // slices [t0, t1) * ztile are final: copy them out behind the next slab

@@ -11,11 +11,9 @@
 //      the detector re-adds the last in-range value of its column, as the
 //      reference does because it never resets Display_pBeta (:73, :100-123).
 //
-// Layout: each view's projection is first repacked into 2x2 quads,
-//   Q[v][x][p] = (R[x][p], R[x][p+1], R[x+1][p], R[x+1][p+1]),
-// so the four bilinear taps of a voxel-view are one aligned 16-byte load.
-// This trades HBM capacity (4x the sinogram, 2.3 GB at 360x512x768) for a
-// quarter of the load instructions on a load-issue-bound kernel.
+// Layout: each view's projection is first repacked into pairs,
+//   Q[v][x][p] = (R[x][p], R[x][p+1]),
+// so that one aligned 8-byte load gives a detector row's two taps.
 //
 // Interpolation follows the reference's discontinuous index rule exactly:
 // column floor(|P - P0| / PInt) and row floor(|xi - xi0| / XigamaInt), with
@@ -27,12 +25,15 @@
 // float-float (ffloat.cuh), and the row quotient, affine in z, is stepped in
 // 64-bit fixed point with a per-row table of the samples' own quotients.
 //
-// Threads own one (t, s) column and ZC consecutive z; the view loop runs
-// inside the thread with the ZC sums in registers, and each voxel is written
-// once at the end (no atomics, deterministic).  The fused SIRT variant writes
-// clamp(x + lambda * bp / (colsum + eps), lo, hi) instead of bp.
-#include <type_traits>
-
+// Two kernels.  What depends on the (t, s) column and the view alone (detector
+// column and weights, row quotient and its step per z, the z range on the
+// detector, the chord factor and its ties) is a 32-byte record that
+// cone_bp_setup_kernel writes once per column-view; it used to be recomputed by
+// each of the column's nz / 32 threads, 250 of 1030 instructions per thread and
+// view.  cone_bp_kernel's threads own one column and ZC consecutive z; the view
+// loop runs inside the thread with the ZC sums in registers, and each voxel is
+// written once at the end (no atomics, deterministic).  The fused SIRT variant
+// writes clamp(x + lambda * bp / (colsum + eps), lo, hi) instead of bp.
 #include "cone_geom.cuh"
 #include "ffloat.cuh"
 
@@ -40,49 +41,36 @@ namespace ct {
 
 namespace {
 
-#ifndef CT_BP_ZC
-#define CT_BP_ZC 32
-#endif
-// Blocks per SM the register allocation aims at.  Chord weighting: 4 (128
-// registers, a few bytes spilled on the out-of-line tie paths) measured 71.8 ms
-// at 512^3 / 360 views against 73.0 ms at 3 (168 registers) and 85.7 ms at 2.
-// FDK weighting at 256^3 / 360 views: 8.08 ms at 3, 8.20 at 4, 12.5 at 5.
-#ifndef CT_BP_MINB
-#define CT_BP_MINB 4
-#endif
-#ifndef CT_BP_MINB_FDK
-#define CT_BP_MINB_FDK 3
-#endif
-constexpr int BP_BX = 32;          // t per block
-// s rows per block (warps of 32 t).  Chord weighting at 512^3 / 360 views,
-// 128 registers: 4 rows 54.6 ms, 2 rows 55.1, 1 row 56.6, 8 rows 57.4.
-#ifndef CT_BP_BY
-#define CT_BP_BY 4
-#endif
-constexpr int BP_BY = CT_BP_BY;    // s per block
-constexpr int BP_ZC = CT_BP_ZC;    // z per thread (register accumulators)
-static_assert(BP_ZC >= 1 && BP_ZC <= 64, "cone_bp: 1 to 64 z per thread");
-// bit k: z0 + k of the thread takes the view
-using zmask_t = std::conditional_t<(BP_ZC > 32), unsigned long long, unsigned>;
-constexpr zmask_t kZAll = BP_ZC >= 8 * (int)sizeof(zmask_t) ? ~zmask_t(0) : ((zmask_t(1) << BP_ZC) - 1);
+constexpr int BP_BX = 32;          // t per block (one warp)
+constexpr int BP_BY = 4;           // s per block
+// z per thread (register accumulators) and the blocks per SM its registers aim at.
+// 32 z share a column-view's record best: 45.2 ms at 512^3 / 360 views and 4 blocks
+// (57 at 5, 50 at 6), 47.7 with 16 z and 8 blocks; where 32 z leave the GPU with
+// few waves of blocks 16 z fill it (SIRT3D of 151 x 133 x 97: 5.2 -> 3.8 ms).
+constexpr int kZLong = 32, kZShort = 16;
+constexpr int bp_min_blocks(int zc) { return zc == kZLong ? 4 : 8; }
 
-// Quads of nb views; R points at the first of them.
+int bp_zc(const ConeGeom &g) {
+    const long long blocks = (long long)((g.nt + BP_BX - 1) / BP_BX) * ((g.ns + BP_BY - 1) / BP_BY) *
+                             ((g.nz + kZLong - 1) / kZLong);
+    return blocks < 3LL * bp_min_blocks(kZLong) * sm_count() ? kZShort : kZLong;
+}
+
+// Pairs of n consecutive samples; the last sample of a row pairs with 0.
 __global__ void __launch_bounds__(256)
-pack_quads_kernel(const float *__restrict__ R, float4 *__restrict__ Q, int nb, int nx, int np) {
-    const long long n = (long long)nb * nx * np;
+pack_pairs_kernel(const float *__restrict__ R, float2 *__restrict__ Q, long long n, int np) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int p = (int)(i % np);
-        const long long rv = i / np;
-        const int x = (int)(rv % nx);
-        const bool pr = p + 1 < np, xr = x + 1 < nx;
-        float4 q;
-        q.x = R[i];
-        q.y = pr ? R[i + 1] : 0.0f;
-        q.z = xr ? R[i + np] : 0.0f;
-        q.w = (pr && xr) ? R[i + np + 1] : 0.0f;
-        Q[i] = q;
-    }
+         i += (long long)gridDim.x * blockDim.x)
+        Q[i] = make_float2(R[i], (int)(i % np) + 1 < np ? R[i + 1] : 0.0f);
+}
+
+// The sum of detector row x's two taps, q0 + x * stride bytes their pair (one
+// multiply-add for the address).
+__device__ __forceinline__ float row_sum(const float2 *q0, unsigned x, unsigned stride, float wa, float wb) {
+    unsigned long long a;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(x), "r"(stride), "l"(q0));
+    const float2 q = __ldg(reinterpret_cast<const float2 *>(a));
+    return fmaf(wa, q.x, wb * q.y);
 }
 
 enum { W_CHORD = 0, W_FDK_ZERO = 1, W_FDK_STICKY = 2 };
@@ -197,55 +185,70 @@ __device__ __noinline__ int chord_end_z(const ConeGeom &g, int ti, int si, doubl
     return min(zhi, zab - 1);
 }
 
-// Views [v0, v0 + nv) of the scan, whose quads Q holds (Q[0] = view v0).
-// Each voxel's sum b = (sum over these views) + prev (when prev is given) is
-// written to out, or with UPDATE folded into out = vol as
-// clamp(vol + lambda * b / (colsum + eps), lo, hi).
-template <int WMODE, bool UPDATE>
-__global__ void __launch_bounds__(BP_BX * BP_BY, WMODE == W_CHORD ? CT_BP_MINB : CT_BP_MINB_FDK)
-cone_bp_kernel(const ConeGeom g, const float4 *__restrict__ Q, int v0, int nv, const float *prev, float *out,
-               const float *__restrict__ colsum, float eps, float lambda, float lo, float hi, int zt0) {
-    // the row table (x - q(xi[x]), q(xi[x+1]) - x) of ConeGeom::xtab
-    extern __shared__ float2 xtab[];
-    const int tid = threadIdx.x + BP_BX * threadIdx.y;
-    for (int x = tid; x < g.nx - 1; x += BP_BX * BP_BY) xtab[x] = g.xtab[x];
-    __syncthreads();
+// The record of a column-view, in two arrays [view][s][t]:
+//  a = (wa, wb, p1, zr): the weights of detector columns p1 and p1 + 1 times the
+//    chord factor 2 mts or the FDK weight; p1 < 0: nothing from this view; zr =
+//    zlo | (zend + 1) << 16, the z that take the view relative to the set-up's
+//    first slice, clamped to [0, 65535] (FDK sticky: zend the last z on the
+//    detector, whose row all z above keep);
+//  b = (r, dq): the row quotient at the set-up's first slice and its step per z,
+//    fixed point with kRowFrac fraction bits.
+constexpr int kRowFrac = 36;
+constexpr int kZSlab = 65504;      // slices a set-up covers (a multiple of the z tiles)
+struct __align__(16) ColView {
+    float wa, wb;
+    int p1;
+    unsigned zr;
+};
 
-    const int ti = blockIdx.x * BP_BX + threadIdx.x;
-    const int si = blockIdx.y * BP_BY + threadIdx.y;
-    const int z0 = (zt0 + (int)blockIdx.z) * BP_ZC;
+__device__ __forceinline__ long long ff_fixed(ff a) {
+    constexpr float one = (float)(1LL << kRowFrac);
+    return __float2ll_rn(__fmul_rn(a.hi, one)) + __float2ll_rn(__fmul_rn(a.lo, one));
+}
+
+// Chord face parameters of a column-view, h / |d| along t and s: approximate
+// reciprocals (a few ulp); the chord factor needs ~1e-7, and the tie tests have
+// margins of 1e-5.
+__device__ __forceinline__ void chord_faces(const ConeGeom &g, float it, float is, float sb, float cb, float &dt,
+                                            float &ds, float &mt, float &ms) {
+    dt = it + g.bp_Df * sb;
+    ds = is - g.bp_Df * cb;
+    mt = __fdividef(g.bp_ht, fabsf(dt));
+    ms = __fdividef(g.bp_hs, fabsf(ds));
+}
+
+// Records of views [v0, v0 + nv) for slices zbase .. zbase + kZSlab - 1.  A thread
+// takes one column and `per` views.
+template <int WMODE>
+__global__ void __launch_bounds__(128)
+cone_bp_setup_kernel(const ConeGeom g, ColView *__restrict__ ta, longlong2 *__restrict__ tb, int v0, int nv, int per,
+                     int zbase) {
+    const int ti = blockIdx.x * 32 + threadIdx.x;
+    const int si = blockIdx.y * 4 + threadIdx.y;
     if (ti >= g.nt || si >= g.ns) return;
-
     // voxel-centre coordinates relative to the rotation centre, exact to ~2^-48
     const ff it2 = ff_from((ti + 0.5) * g.res[0] - 0.5 * g.size[0]);
     const ff is2 = ff_from((si + 0.5) * g.res[1] - 0.5 * g.size[1]);
-    const ff iz02 = ff_from((z0 + 0.5) * g.res[2] - 0.5 * g.size[2]);
+    const ff izb2 = ff_from((zbase + 0.5) * g.res[2] - 0.5 * g.size[2]);
     const ff D2 = {g.bp_D.x, g.bp_D.y};
     const ff ipint2 = {g.bp_ipint.x, g.bp_ipint.y};
     const ff xq2 = {g.bp_xq.x, g.bp_xq.y};   // row quotient per mm of xi
     const ff p02 = {g.p0, 0.0f};
     // the view-independent factors of the row quotient: (iz lr - xi0) xq = lr (iz xq) - xi0 xq
-    const ff rzxq2 = {g.bp_rzxq.x, g.bp_rzxq.y}, iz0xq2 = ff_mul(iz02, xq2), x0xq2 = {g.bp_x0xq.x, g.bp_x0xq.y};
-
-    const float rz = g.bp_rz;
+    const ff rzxq2 = {g.bp_rzxq.x, g.bp_rzxq.y}, izbxq2 = ff_mul(izb2, xq2), x0xq2 = {g.bp_x0xq.x, g.bp_x0xq.y};
     const float it = it2.hi, is = is2.hi;
     const float D = g.bp_Df;
     const float ipint = g.bp_ipintf;
-    const float ht = g.bp_ht, hs = g.bp_hs, hz = g.bp_hz;
+    const float hz = g.bp_hz;
     const float czf = g.bp_czf;
-    const float x_base = g.bp_xbase;   // iz at z = 0
-    const float iz0 = iz02.hi;         // iz of this thread's first z
-    // largest |iz| of the thread's z range: decides whether z faces can limit the chord
-    const float izmax = fmaxf(fabsf(iz0), fabsf(fmaf((float)(BP_ZC - 1), rz, iz0)));
+    const float x_base = g.bp_xbase;      // iz at z = 0
     const float iz_vol = fabsf(x_base);   // largest |iz| of the volume
     const float irz = g.bp_irz, iD = g.bp_iD;
-    const long long vstride = (long long)g.nx * g.np;
-
-    float acc[BP_ZC];
-#pragma unroll
-    for (int k = 0; k < BP_ZC; ++k) acc[k] = 0.0f;
-
-    for (int v = v0; v < v0 + nv; ++v) {
+    const long long ncol = (long long)g.nt * g.ns;
+    const int k0 = blockIdx.z * per, k1 = min(k0 + per, nv);
+    long long o = k0 * ncol + (long long)si * g.nt + ti;
+    for (int k = k0; k < k1; ++k, o += ncol) {
+        const int v = v0 + k;
         const float2 tr = g.trigf[v];   // float (sin, cos): no FP64 conversion in the loop
         const float sb = tr.x, cb = tr.y;
         // detector coordinates of the column in float-float: the reference's
@@ -268,32 +271,29 @@ cone_bp_kernel(const ConeGeom g, const float4 *__restrict__ Q, int v0, int nv, c
         const bool near_edge = fabsf(zlo_f - rintf(zlo_f)) < 2.5e-4f || fabsf(zhi_f - rintf(zhi_f)) < 2.5e-4f ||
                                fabsf(P - g.minp) < 2e-4f || fabsf(P - g.maxp) < 2e-4f;
         if (near_edge) range_fp64(g, ti, si, g.trig[v].x, g.trig[v].y, pin, zlo, zhi);
-        if (!pin) continue;   // whole column off the detector for this view
-        if (WMODE == W_FDK_STICKY && zhi < zlo) continue;
+        ColView c{0.0f, 0.0f, -1, 0u};
+        if (!pin || (WMODE == W_FDK_STICKY && zhi < zlo)) {   // off the detector for this view
+            ta[o] = c;
+            tb[o] = make_longlong2(0, 0);
+            continue;
+        }
         // detector column floor(|P - P0| / PInt) and weights |P - P[p1]| / PInt,
         // |P[p1+1] - P| / PInt from the domain values (Backprojection3D.cu:73-83)
         const int p1 = min(max(ff_floor(ff_mul(ff_abs(ff_sub(P2, p02)), ipint2)), 0), g.np - 2);
         const float pa = __ldg(g.P + p1), pb = __ldg(g.P + p1 + 1);
         const float wq1 = fabsf(__fadd_rn(__fsub_rn(P2.hi, pa), P2.lo)) * ipint;   // weight of column p1+1
         const float wq0 = fabsf(__fsub_rn(__fsub_rn(pb, P2.hi), P2.lo)) * ipint;   // weight of column p1
-        const float4 *Qv = Q + (long long)(v - v0) * vstride + p1;
-        // row quotient q(z) = |xi(z) - xi[0]| / XigamaInt, affine in z, as 64-bit
-        // fixed point (32 fraction bits): floor and weights follow the
-        // reference's FP64 values except within ~1e-8 of a row boundary
-        const long long dqf = ff_fixed32(ff_mul(rzxq2, lr2));
-        long long r = ff_fixed32(ff_sub(ff_mul(iz0xq2, lr2), x0xq2));
+        // row quotient q(z) = |xi(z) - xi[0]| / XigamaInt, affine in z: floor and weights
+        // follow the reference's FP64 values except within ~1e-8 of a row boundary
+        long long dq = ff_fixed(ff_mul(rzxq2, lr2));
+        long long r = ff_fixed(ff_sub(ff_mul(izbxq2, lr2), x0xq2));
 
-        float wv = 1.0f, mts = 0.0f, qq = 0.0f;
         int zend = zhi;           // last z that receives this view's value
-        bool zlimit = false;      // some z face limits a chord in this thread's range
+        float c0 = lr * lr * g.bint;
         if (WMODE == W_CHORD) {
-            const float dt = it + D * sb, ds = is - D * cb;
-            // approximate reciprocals (a few ulp): the chord factor needs ~1e-7, and the
-            // tie tests below have margins of 1e-5
-            const float mt = __fdividef(ht, fabsf(dt)), ms = __fdividef(hs, fabsf(ds));
-            mts = fminf(mt, ms);
-            qq = fmaf(dt, dt, ds * ds);
-            zlimit = izmax * mts > hz;
+            float dt, ds, mt, ms;
+            chord_faces(g, it, is, sb, cb, dt, ds, mt, ms);
+            const float mts = fminf(mt, ms);
             // The source->centre line passes near a voxel edge when two faces'
             // parameters tie; only then can the reference's FP64 face tests all
             // fail and end the column.  Ties are found in FP32 with a wide margin
@@ -312,83 +312,187 @@ cone_bp_kernel(const ConeGeom g, const float4 *__restrict__ Q, int v0, int nv, c
             if (tie_ts || tz1 || tz2)
                 zend = chord_end_z(g, ti, si, g.trig[v].x, g.trig[v].y, zlo, zhi, tie_ts, hz / mts, fmaxf(mt, ms), tz1, zc1, tz2,
                                    zc2);
-        } else {
-            wv = lr * lr * g.bint;
+            c0 = 2.0f * mts;
         }
-        // the chord factor 2 * mts (or the FDK weight) folds into the detector-column
-        // weights; where a z face can limit the chord the factor becomes
-        // min(1, hz / (|iz| mts))
-        const float c0 = (WMODE == W_CHORD) ? 2.0f * mts : wv;
-        const float wa = wq0 * c0, wb = wq1 * c0;
+        c.wa = wq0 * c0;
+        c.wb = wq1 * c0;
+        c.p1 = p1;
+        if (WMODE == W_FDK_STICKY && zhi < zbase) {   // the whole slab keeps the row of zhi
+            r += (long long)(zhi - zbase) * dq;
+            dq = 0;
+            zend = 0x7ffffff0;
+        }
+        const int a = min(max(zlo - zbase, 0), 65535), e = min(max(zend - zbase + 1, 0), 65535);
+        c.zr = (unsigned)a | ((unsigned)e << 16);
+        ta[o] = c;
+        tb[o] = make_longlong2(r, dq);
+    }
+}
+
+// Views [v0, v0 + nv) of the scan, whose pairs Q and records (ta, tb) hold
+// (index 0 = view v0).  Each voxel's sum b = (sum over these views) + prev
+// (when prev is given) is written to out, or with UPDATE folded into out = vol
+// as clamp(vol + lambda * b / (colsum + eps), lo, hi).
+//
+// Per voxel-view of the fast path: the fixed-point step, one row-table load, one
+// pair load (two where z advances a row or more), the row sum, the blend, the
+// chord polynomial and the sum.
+template <int WMODE, bool UPDATE, int BP_ZC>
+__global__ void __launch_bounds__(BP_BX * BP_BY, bp_min_blocks(BP_ZC))
+cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__restrict__ ta,
+               const longlong2 *__restrict__ tb, int v0, int nv, const float *prev, float *out,
+               const float *__restrict__ colsum, float eps, float lambda, float lo, float hi, int zt0, int zbase) {
+    // the row table (x - q(xi[x]), q(xi[x+1]) - x) of ConeGeom::xtab
+    extern __shared__ float2 xtab[];
+    const int tid = threadIdx.x + BP_BX * threadIdx.y;
+    for (int x = tid; x < g.nx - 1; x += BP_BX * BP_BY) xtab[x] = g.xtab[x];
+    __syncthreads();
+
+    const int ti = blockIdx.x * BP_BX + threadIdx.x;
+    const int si = blockIdx.y * BP_BY + threadIdx.y;
+    const int z0 = (zt0 + (int)blockIdx.z) * BP_ZC;
+    if (ti >= g.nt || si >= g.ns) return;
+    const int zr0 = z0 - zbase;        // relative to the set-up
+
+    const float it = ff_from((ti + 0.5) * g.res[0] - 0.5 * g.size[0]).hi;
+    const float is = ff_from((si + 0.5) * g.res[1] - 0.5 * g.size[1]).hi;
+    const float rz = g.bp_rz, hz = g.bp_hz;
+    const float iz0 = ff_from((z0 + 0.5) * g.res[2] - 0.5 * g.size[2]).hi;   // iz of this thread's first z
+    // largest |iz| of the thread's z range: decides whether z faces can limit the chord
+    const float izmax = fmaxf(fabsf(iz0), fabsf(fmaf((float)(BP_ZC - 1), rz, iz0)));
+    const long long vstride = (long long)g.nx * g.np;
+    const long long ncol = (long long)g.nt * g.ns;
+    const unsigned last = (unsigned)(g.nx - 2);
+    constexpr unsigned all = 0xffffffffu >> (32 - BP_ZC);
+    const float kc = 0.5f * (BP_ZC - 1);
+    const float izc = fmaf(kc, rz, iz0);
+    const float hspan = kc * rz;
+
+    float acc[BP_ZC];
+#pragma unroll
+    for (int k = 0; k < BP_ZC; ++k) acc[k] = 0.0f;
+
+    ta += (long long)si * g.nt + ti;
+    tb += (long long)si * g.nt + ti;
+    const float2 *Qview = Q;
+    const unsigned row_bytes = 8u * (unsigned)g.np;
+    // the records stream from DRAM once per z tile: the next view's are fetched
+    // before this one's work
+    float4 cn = __ldcs(reinterpret_cast<const float4 *>(ta));
+    longlong2 rn = __ldcs(tb);
+    for (int v = 0; v < nv; ++v, Qview += vstride) {
+        const float4 c = cn;
+        const longlong2 rb = rn;
+        if (v + 1 < nv) {
+            ta += ncol;
+            tb += ncol;
+            cn = __ldcs(reinterpret_cast<const float4 *>(ta));
+            rn = __ldcs(tb);
+        }
+        const int p1 = __float_as_int(c.z);
+        if (p1 < 0) continue;   // whole column off the detector for this view
+        const float wa = c.x, wb = c.y;
+        const unsigned zr = __float_as_uint(c.w);
+        const int zlo = (int)(zr & 0xffffu), zend = (int)(zr >> 16) - 1;
+        long long dqf = rb.y >> (kRowFrac - 32);
+        long long r = (rb.x + zr0 * rb.y) >> (kRowFrac - 32);     // 32 fraction bits from here
+        const float2 *Qv = Qview + p1, *Qn = Qv + g.np;     // rows x and x + 1
         // sticky FDK: z above zhi re-add the value at zhi (the row quotient stops there)
-        const int kz = zhi - z0;
+        const int kz = zend - zr0;
         if (WMODE == W_FDK_STICKY && kz < 0) r += (long long)kz * dqf;
         // z of this thread that take this view, as a bit mask over k
-        const int klo = max(zlo - z0, 0), khi = min(((WMODE == W_FDK_STICKY) ? 0x7fff : zend) - z0, BP_ZC - 1);
-        const zmask_t inmask = (klo > khi) ? zmask_t(0)
-                               : ((khi >= BP_ZC - 1 ? kZAll : ((zmask_t(2) << khi) - 1)) & ~((zmask_t(1) << klo) - 1));
-        // Fast path: every z of the thread takes the view, no z face limits the
-        // chord, and the chord length |d| = sqrt(qq + iz^2) is the quadratic in k
-        // about the thread's middle z (relative error below 1e-7, bounded by the
-        // third-order term |iz| h^3 / (2 |d|^4), h the half span of the 32 z).
-        const float kc = 0.5f * (BP_ZC - 1);
-        const float izc = fmaf(kc, rz, iz0);
-        const float lc2 = fmaf(izc, izc, qq);
-        const float ilc = rsqrtf(lc2), lc = lc2 * ilc;
-        const float l1 = izc * rz * ilc, l2 = 0.5f * qq * rz * rz * ilc * ilc * ilc;
-        const float hspan = kc * rz;
-        // more than 32 z: a cubic term, whose error (fourth order) is below
-        // h^4 / (2 |d|^4)
-        const float l3 = (BP_ZC > 32) ? -0.5f * qq * izc * rz * rz * rz * ilc * ilc * ilc * ilc * ilc : 0.0f;
-        const float hl = hspan * ilc;
-        const bool quad_ok = WMODE != W_CHORD ||
-                             ((BP_ZC > 32) ? 0.5f * hl * hl * hl * hl < 2e-7f
-                                           : fabsf(izc) * hspan * hspan * hspan * ilc * ilc * ilc * ilc < 2e-7f);
-        const bool fast = inmask == kZAll && !zlimit && quad_ok &&
-                          !(WMODE == W_FDK_STICKY && kz < BP_ZC - 1);
-        auto body = [&](auto fastpath) {
-            constexpr bool FAST = decltype(fastpath)::value;
+        const int klo = max(zlo - zr0, 0), khi = min(((WMODE == W_FDK_STICKY) ? 0x7fff : kz), BP_ZC - 1);
+        const unsigned inmask = (klo > khi) ? 0u
+                               : ((khi >= BP_ZC - 1 ? all : ((2u << khi) - 1)) & ~((1u << klo) - 1));
+        // Fast path: every z of the thread takes the view from rows [0, nx - 2] (the ends of
+        // the affine quotient decide), no z face limits the chord, and the chord length
+        // |d| = sqrt(qq + iz^2) is the quadratic in k about the thread's middle z
+        // (relative error below 1e-7, bounded by the third-order term
+        // |iz| h^3 / (2 |d|^4), h the half span of the z).
+        bool fast = inmask == all && (unsigned)(int)(r >> 32) <= last &&
+                    (unsigned)(int)((r + (BP_ZC - 1) * dqf) >> 32) <= last &&
+                    !(WMODE == W_FDK_STICKY && kz < BP_ZC - 1);
+        float dt = 0.0f, ds = 0.0f, qq = 0.0f, lc = 0.0f, l1 = 0.0f, l2 = 0.0f;
+        if (WMODE == W_CHORD) {
+            const float2 tr = g.trigf[v0 + v];
+            dt = it + g.bp_Df * tr.x;
+            ds = is - g.bp_Df * tr.y;
+            qq = fmaf(dt, dt, ds * ds);
+            const float lc2 = fmaf(izc, izc, qq);
+            const float ilc = rsqrtf(lc2);
+            lc = lc2 * ilc;
+            l1 = izc * rz * ilc;
+            l2 = 0.5f * qq * rz * rz * ilc * ilc * ilc;
+            const float hl = hspan * ilc;
+            // the weights sum to 2 mts to the samples' drift: 10% of margin
+            fast = fast && 0.55f * izmax * (wa + wb) < hz && fabsf(izc) * ilc * hl * hl * hl < 2e-7f;
+        }
+        if (fast) {
+            auto add = [&](int k, unsigned x, unsigned f, float top, float bot) {
+                const float fr = __uint2float_rn(f);                          // fraction * 2^32
+                const float2 xt = xtab[x];
+                const float w1 = fmaf(fr, 2.3283064365386963e-10f, xt.x);    // |w1|: weight of row x+1
+                const float w0 = fmaf(fr, -2.3283064365386963e-10f, xt.y);   // |w0|: weight of row x
+                const float val = fmaf(fabsf(w0), top, fabsf(w1) * bot);
+                if (WMODE == W_CHORD) {
+                    // chord 2 * min(h_a / |d_a|) * |d|, d = (dt, ds, iz)
+                    const float dk = (float)k - kc;
+                    acc[k] = fmaf(val, fmaf(dk, fmaf(dk, l2, l1), lc), acc[k]);
+                } else {
+                    acc[k] += val;
+                }
+            };
+            unsigned x = (unsigned)(r >> 32), f = (unsigned)r;
+            if ((dqf >> 32) == 0) {
+                // less than a row per z: the upper row is the upper or the lower row of the z before
+                const unsigned df = (unsigned)dqf;
+                float top = row_sum(Qv, x, row_bytes, wa, wb), bot = row_sum(Qn, x, row_bytes, wa, wb);
+#pragma unroll
+                for (int k = 0; k < BP_ZC; ++k) {
+                    if (k > 0) {
+                        const unsigned xo = x;
+                        asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(f), "+r"(x) : "r"(df));
+                        top = x != xo ? bot : top;
+                        bot = row_sum(Qn, x, row_bytes, wa, wb);
+                    }
+                    add(k, x, f, top, bot);
+                }
+            } else {
+                long long rk = r;
+#pragma unroll
+                for (int k = 0; k < BP_ZC; ++k) {
+                    if (k > 0) rk += dqf;
+                    const unsigned xk = (unsigned)(rk >> 32);
+                    add(k, xk, (unsigned)rk, row_sum(Qv, xk, row_bytes, wa, wb), row_sum(Qn, xk, row_bytes, wa, wb));
+                }
+            }
+        } else {
+            float mts = 0.0f;
+            if (WMODE == W_CHORD) mts = fminf(__fdividef(g.bp_ht, fabsf(dt)), __fdividef(g.bp_hs, fabsf(ds)));
             long long rk = r;
 #pragma unroll
             for (int k = 0; k < BP_ZC; ++k) {
-                if (k > 0) rk += (!FAST && WMODE == W_FDK_STICKY && k > kz) ? 0LL : dqf;
+                if (k > 0) rk += (WMODE == W_FDK_STICKY && k > kz) ? 0LL : dqf;
                 // an index outside [0, nx-2] (z off the detector, or a negative
                 // quotient wrapped by the unsigned compare) is clamped for the read only
-                const unsigned x1 = min((unsigned)(int)(rk >> 32), (unsigned)(g.nx - 2));
-                const float fr = __uint2float_rn((unsigned)rk);          // fraction * 2^32
+                const int x1 = (int)min((unsigned)(int)(rk >> 32), last);
+                const float fr = __uint2float_rn((unsigned)rk);
                 const float2 xt = xtab[x1];
-                const float w1 = fmaf(fr, 2.3283064365386963e-10f, xt.x);    // |w1|: weight of row x1+1
-                const float w0 = fmaf(fr, -2.3283064365386963e-10f, xt.y);   // |w0|: weight of row x1
-                const float4 q = __ldg(Qv + (int)x1 * g.np);
-                const float top = fmaf(wa, q.x, wb * q.y);
-                const float bot = fmaf(wa, q.z, wb * q.w);
-                const float val = fmaf(fabsf(w0), top, fabsf(w1) * bot);
-                float w;
+                const float w1 = fmaf(fr, 2.3283064365386963e-10f, xt.x);
+                const float w0 = fmaf(fr, -2.3283064365386963e-10f, xt.y);
+                const float val = fmaf(fabsf(w0), row_sum(Qv, x1, row_bytes, wa, wb),
+                                       fabsf(w1) * row_sum(Qn, x1, row_bytes, wa, wb));
+                float w = 1.0f;
                 if (WMODE == W_CHORD) {
-                    // chord 2 * min(h_a / |d_a|) * |d|, d = (dt, ds, iz); the factor
-                    // min(1, hz / (|iz| mts)) is 1 where no z face limits the chord
-                    if (FAST) {
-                        const float dk = (float)k - kc;
-                        if constexpr (BP_ZC > 32) w = fmaf(dk, fmaf(dk, fmaf(dk, l3, l2), l1), lc);
-                        else w = fmaf(dk, fmaf(dk, l2, l1), lc);
-                    } else {
-                        const float iz = fmaf((float)k, rz, iz0);
-                        const float d2 = fmaf(iz, iz, qq);
-                        w = fminf(1.0f, hz / (fabsf(iz) * mts)) * (d2 * rsqrtf(d2));
-                    }
-                } else {
-                    w = 1.0f;
+                    // a z face limits the chord by min(1, hz / (|iz| mts))
+                    const float iz = fmaf((float)k, rz, iz0);
+                    const float d2 = fmaf(iz, iz, qq);
+                    w = fminf(1.0f, hz / (fabsf(iz) * mts)) * (d2 * rsqrtf(d2));
                 }
-                if (FAST) {
-                    acc[k] = fmaf(val, w, acc[k]);
-                } else {
-                    const bool in = (inmask >> k) & 1;
-                    acc[k] = in ? fmaf(val, w, acc[k]) : acc[k];
-                }
+                const bool in = (inmask >> k) & 1;
+                acc[k] = in ? fmaf(val, w, acc[k]) : acc[k];
             }
-        };
-        if (fast) body(std::true_type{});
-        else body(std::false_type{});
+        }
     }
 #pragma unroll
     for (int k = 0; k < BP_ZC; ++k) {
@@ -408,46 +512,89 @@ cone_bp_kernel(const ConeGeom g, const float4 *__restrict__ Q, int v0, int nv, c
 
 }  // namespace
 
-size_t cone_quads_bytes(const ConeGeom &g, int nviews) { return sizeof(float4) * (size_t)nviews * g.nx * g.np; }
+size_t cone_bp_pairs_bytes(const ConeGeom &g, int nviews) { return sizeof(float2) * (size_t)nviews * g.nx * g.np; }
 
-int cone_pack_quads(const ConeGeom &g, const float *R, float4 *Q, int v0, int nv, cudaStream_t st) {
+size_t cone_bp_table_bytes(const ConeGeom &g, int nviews) {
+    return (sizeof(ColView) + sizeof(longlong2)) * (size_t)nviews * g.nt * g.ns;
+}
+
+int cone_bp_pack(const ConeGeom &g, const float *R, float2 *Q, int v0, int nv, cudaStream_t st) {
     const long long n = (long long)nv * g.nx * g.np;
     int blocks = (int)std::min<long long>((n + 255) / 256, (long long)sm_count() * 16);
-    pack_quads_kernel<<<blocks, 256, 0, st>>>(R + (long long)v0 * g.nx * g.np, Q, nv, g.nx, g.np);
-    CT_LAUNCH_CHECK("pack_quads_kernel");
+    pack_pairs_kernel<<<blocks, 256, 0, st>>>(R + (long long)v0 * g.nx * g.np, Q, n, g.np);
+    CT_LAUNCH_CHECK("pack_pairs_kernel");
     return CT_OK;
 }
 
-int cone_bp_ztile() { return BP_ZC; }
+int cone_bp_ztile(const ConeGeom &g) { return bp_zc(g); }
+
+namespace {
+
+// The records of views [v0, v0 + nv) from slice zbase into tab.
+int setup_launch(const ConeGeom &gk, void *tab, int v0, int nv, int weighting, int zbase, cudaStream_t st) {
+    const long long ncol = (long long)gk.nt * gk.ns;
+    ColView *ta = static_cast<ColView *>(tab);
+    longlong2 *tb = reinterpret_cast<longlong2 *>(ta + nv * ncol);
+    // 8 views per thread, fewer where the columns alone leave the GPU idle
+    int per = 8;
+    while (per > 1 && ncol * ((nv + per - 1) / per) < 1024LL * sm_count()) per /= 2;
+    const int nz = (nv + per - 1) / per;
+    CT_REQUIRE(nz <= 65535, "cone_bp: too many views per chunk");
+    const dim3 grid((gk.nt + 31) / 32, (gk.ns + 3) / 4, nz), block(32, 4);
+    if (weighting == W_CHORD) cone_bp_setup_kernel<W_CHORD><<<grid, block, 0, st>>>(gk, ta, tb, v0, nv, per, zbase);
+    else if (weighting == W_FDK_ZERO)
+        cone_bp_setup_kernel<W_FDK_ZERO><<<grid, block, 0, st>>>(gk, ta, tb, v0, nv, per, zbase);
+    else cone_bp_setup_kernel<W_FDK_STICKY><<<grid, block, 0, st>>>(gk, ta, tb, v0, nv, per, zbase);
+    CT_LAUNCH_CHECK("cone_bp_setup_kernel");
+    return CT_OK;
+}
+
+}  // namespace
 
 // weighting: 0 chord, 1 FDK (off-detector adds 0), 2 FDK sticky
-int cone_bp_launch(const ConeGeom &g, const float4 *Q, int v0, int nv, const float *prev, float *out, int weighting,
-                   const float *colsum, float eps, float lambda, float lo, float hi, bool update, cudaStream_t st,
-                   int zt0, int nzt) {
+int cone_bp_launch(const ConeGeom &g, const float2 *Q, void *tab, bool tab_ready, int v0, int nv, const float *prev,
+                   float *out, int weighting, const float *colsum, float eps, float lambda, float lo, float hi,
+                   bool update, cudaStream_t st, int zt0, int nzt) {
     CT_REQUIRE(g.np >= 2 && g.nx >= 2, "cone_bp: detector needs at least 2x2 samples");
     CT_REQUIRE(v0 >= 0 && nv > 0 && v0 + nv <= g.nb, "cone_bp: view range out of bounds");
-    const int ntiles = (g.nz + BP_ZC - 1) / BP_ZC;
+    const int zc = bp_zc(g);
+    const int ntiles = (g.nz + zc - 1) / zc;
     if (nzt <= 0) nzt = ntiles - zt0;
     CT_REQUIRE(zt0 >= 0 && nzt > 0 && zt0 + nzt <= ntiles, "cone_bp: z tile range out of bounds");
     ConeGeom gk = g;   // with the set-up's constants
     cone_bp_consts(gk);
     dim3 block(BP_BX, BP_BY);
-    dim3 grid((g.nt + BP_BX - 1) / BP_BX, (g.ns + BP_BY - 1) / BP_BY, nzt);
     const size_t smem = sizeof(float2) * (size_t)g.nx;
     CT_REQUIRE(smem <= 48 * 1024, "cone_bp: at most 6144 detector rows");
-#define CT_BP_CASE(W, U)                                                                     \
-    cone_bp_kernel<W, U><<<grid, block, smem, st>>>(gk, Q, v0, nv, prev, out, colsum, eps, lambda, lo, hi, zt0)
-    if (update) {
-        if (weighting == W_CHORD) CT_BP_CASE(W_CHORD, true);
-        else if (weighting == W_FDK_ZERO) CT_BP_CASE(W_FDK_ZERO, true);
-        else CT_BP_CASE(W_FDK_STICKY, true);
-    } else {
-        if (weighting == W_CHORD) CT_BP_CASE(W_CHORD, false);
-        else if (weighting == W_FDK_ZERO) CT_BP_CASE(W_FDK_ZERO, false);
-        else CT_BP_CASE(W_FDK_STICKY, false);
-    }
+    const ColView *ta = static_cast<const ColView *>(tab);
+    const longlong2 *tb = reinterpret_cast<const longlong2 *>(ta + nv * (long long)g.nt * g.ns);
+    // slabs of at most kZSlab slices, each with its own records (one slab below 65505 slices)
+    const int slab = kZSlab / zc;
+    for (int t = zt0; t < zt0 + nzt;) {
+        const int zb = t / slab * slab, n = std::min(zt0 + nzt, zb + slab) - t, zbase = zb * zc;
+        if (!tab_ready || ntiles > slab)
+            if (int s = setup_launch(gk, tab, v0, nv, weighting, zbase, st)) return s;
+        const dim3 grid((g.nt + BP_BX - 1) / BP_BX, (g.ns + BP_BY - 1) / BP_BY, n);
+#define CT_BP_RUN(W, U, Z)                                                                                        \
+    cone_bp_kernel<W, U, Z><<<grid, block, smem, st>>>(gk, Q, ta, tb, v0, nv, prev, out, colsum, eps, lambda, lo, \
+                                                       hi, t, zbase)
+#define CT_BP_CASE(W, U)                     \
+    if (zc == kZLong) CT_BP_RUN(W, U, kZLong); \
+    else CT_BP_RUN(W, U, kZShort)
+        if (update) {
+            if (weighting == W_CHORD) { CT_BP_CASE(W_CHORD, true); }
+            else if (weighting == W_FDK_ZERO) { CT_BP_CASE(W_FDK_ZERO, true); }
+            else { CT_BP_CASE(W_FDK_STICKY, true); }
+        } else {
+            if (weighting == W_CHORD) { CT_BP_CASE(W_CHORD, false); }
+            else if (weighting == W_FDK_ZERO) { CT_BP_CASE(W_FDK_ZERO, false); }
+            else { CT_BP_CASE(W_FDK_STICKY, false); }
+        }
+#undef CT_BP_RUN
 #undef CT_BP_CASE
-    CT_LAUNCH_CHECK("cone_bp_kernel");
+        CT_LAUNCH_CHECK("cone_bp_kernel");
+        t += n;
+    }
     return CT_OK;
 }
 

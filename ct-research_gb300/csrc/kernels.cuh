@@ -160,17 +160,21 @@ int cone_fixup_launch(const ConeGeom &g, const float *vol, float *out, const flo
                       float eps, double *norms, int mode, const GrazeList &gl, cudaStream_t st);
 int fan_fixup_launch(const FanGeom &g, const float *img, void *out, bool out_double, const float *b,
                      const float *rowsum, float eps, double *norms, int mode, const GrazeList &gl, cudaStream_t st);
-// Backprojection in view chunks: the quads of views [v0, v0 + nv) of the full
+// Backprojection in view chunks: the pairs of views [v0, v0 + nv) of the full
 // sinogram R are packed into Q, then backprojected; each voxel's chunk sum plus
 // prev (optional) goes to out, or, with update, into out = vol as
-// clamp(vol + lambda * sum / (colsum + eps), lo, hi).
-size_t cone_quads_bytes(const ConeGeom &g, int nviews);
-int cone_pack_quads(const ConeGeom &g, const float *R, float4 *Q, int v0, int nv, cudaStream_t st);
-// zt0, nzt: a range of z tiles of cone_bp_ztile() slices (nzt = 0: from zt0 to the top).
-int cone_bp_launch(const ConeGeom &g, const float4 *Q, int v0, int nv, const float *prev, float *out, int weighting,
-                   const float *colsum, float eps, float lambda, float lo, float hi, bool update, cudaStream_t st,
-                   int zt0 = 0, int nzt = 0);
-int cone_bp_ztile();
+// clamp(vol + lambda * sum / (colsum + eps), lo, hi).  tab holds the chunk's
+// column-view records (cone_bp_table_bytes), written by the launch unless
+// tab_ready: then they are those of the last launch with the same views and
+// weighting.
+size_t cone_bp_pairs_bytes(const ConeGeom &g, int nviews);
+size_t cone_bp_table_bytes(const ConeGeom &g, int nviews);
+int cone_bp_pack(const ConeGeom &g, const float *R, float2 *Q, int v0, int nv, cudaStream_t st);
+// zt0, nzt: a range of z tiles of cone_bp_ztile(g) slices (nzt = 0: from zt0 to the top).
+int cone_bp_launch(const ConeGeom &g, const float2 *Q, void *tab, bool tab_ready, int v0, int nv, const float *prev,
+                   float *out, int weighting, const float *colsum, float eps, float lambda, float lo, float hi,
+                   bool update, cudaStream_t st, int zt0 = 0, int nzt = 0);
+int cone_bp_ztile(const ConeGeom &g);
 int row_filter_launch(const RowFilter &f, const float *R, float *out, cudaStream_t st);
 // The set-up table of every ray of g (nb * np records), for g.ray_tab.
 int fan_ray_table_launch(const FanGeom &g, FanRay *tab, cudaStream_t st);

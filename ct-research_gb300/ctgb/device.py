@@ -130,9 +130,10 @@ class ConePlan:
 
     def launches_per_pair(self) -> int:
         """Kernels of one fp + bp: layout transpose, walk, grazing re-walk, and
-        per backprojection chunk the quad packing and the backprojection."""
+        per backprojection chunk the pair packing, the set-up and the
+        backprojection."""
         nb = len(self.geom.beta)
-        return 3 + 2 * -(-nb // self.bp_chunk_views())
+        return 3 + 3 * -(-nb // self.bp_chunk_views())
 
     def set_filter(self, kind="shepp-logan", window: int = 0, short_scan: bool = False):
         """FDK filter stage: ramp taps, Hamming smoothing window length (0 =

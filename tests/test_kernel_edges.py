@@ -87,3 +87,36 @@ def test_row_filter_infinities_stay_in_their_row():
     assert not torch.isfinite(out[1, 2]).any() and not torch.isfinite(out[2, 0]).any()
     out[1, 2], out[2, 0] = good[1, 2], good[2, 0]
     assert torch.equal(out, good)
+
+
+# (nt, ns, nz), views, (cols, rows), detector rows per voxel in z (below and above one), descending rows, source distance
+CONE_BP = [
+    ((33, 5, 16), 3, (40, 24), 0.7, False, 5.0),        # one z tile of 16, a second t tile of one column
+    ((31, 4, 17), 4, (40, 30), 1.3, False, 5.0),        # the last tile holds one slice
+    ((20, 18, 40), 9, (30, 20), 0.6, True, 5.0),        # rows descending: the quotient falls with z
+    ((24, 24, 64), 8, (40, 30), 0.9, False, 2.0),       # the cone leaves the detector in z, diagonal views
+    ((300, 260, 33), 2, (200, 60), 0.8, False, 4.0),    # wide enough for 32 z per thread
+    ((300, 260, 70), 2, (200, 90), 2.2, False, 4.0),
+]
+
+
+@pytest.mark.parametrize("shape,views,det,rows,down,dist", CONE_BP)
+def test_cone_backprojection_tiles_and_row_steps(oracle, shape, views, det, rows, down, dist):
+    import torch
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry
+    nt, ns, nz = shape
+    rng = np.random.default_rng(nt + nz)
+    cols, nx = det
+    P = (np.arange(cols) - (cols - 1) / 2) * (1.5 * max(nt, ns) / cols)
+    xi = (np.arange(nx) - (nx - 1) / 2) / rows
+    xi = xi[::-1].copy() if down else xi
+    beta = np.arange(1, views + 1) * (2 * np.pi / views)
+    size, D = (float(nt), float(ns), float(nz)), dist * max(nt, ns)
+    g = ConeGeometry(nt, ns, nz, size, beta, P, xi, D)
+    R = rng.random(g.sino_shape).astype(np.float32)
+    d = torch.from_numpy(R).cuda()
+    assert rel_l2(ConePlan(g).bp(d).cpu().numpy(), oracle.cone_bp(R, g.beta, g.P, g.xi, size, D, (nz, ns, nt))) <= TOL
+    for sticky in (0, 1):
+        ref = oracle.fdk_bp(R, g.beta, g.P, g.xi, size, D, (nz, ns, nt), sticky=sticky)
+        assert rel_l2(ConePlan(g, fdk_bp=sticky).fdk_bp(d).cpu().numpy(), ref) <= TOL
