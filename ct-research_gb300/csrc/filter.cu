@@ -123,6 +123,7 @@ row_filter_kernel(const RowFilter f, const float *__restrict__ R, float *__restr
                     l[i] = 0.0f;
                 }
                 float4 hi = *reinterpret_cast<const float4 *>(gp - q0);
+#pragma unroll 2
                 for (int q = q0; q < q1; q += 4) {
                     const float4 lo = *reinterpret_cast<const float4 *>(gp - q - 4);
                     const float4 m4 = *reinterpret_cast<const float4 *>(mix + q);
