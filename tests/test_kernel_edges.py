@@ -120,3 +120,40 @@ def test_cone_backprojection_tiles_and_row_steps(oracle, shape, views, det, rows
     for sticky in (0, 1):
         ref = oracle.fdk_bp(R, g.beta, g.P, g.xi, size, D, (nz, ns, nt), sticky=sticky)
         assert rel_l2(ConePlan(g, fdk_bp=sticky).fdk_bp(d).cpu().numpy(), ref) <= TOL
+
+
+def _curved(lg, lx, views):
+    """Equiangular detector of lg gammas and lx rows around a 90 mm display at distance 300."""
+    gama = -(np.arange(lg) - (lg - 1) / 2) * (0.4 / lg)
+    xi = (np.arange(lx) - (lx - 1) / 2) * (60.0 / lx)
+    beta = 0.03 + np.arange(views) * (4.2 / views)
+    return gama, xi, beta, 0.03, 1.001 * abs(gama[-1] - gama[0]), 300.0, 560.0
+
+
+@pytest.mark.parametrize("lg", [2, 3, 5, 64, 66, 127, 1030])
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 1e30])
+def test_curved_filter_row_lengths(oracle, lg, scale):
+    """Rows around the 4-output groups, the 64-sample sums and the block's 1024 outputs: the filter rounds a ~2^-40
+    sum to a float, so it agrees with the FP64 sum to a float's rounding (6e-8 rms of each value)."""
+    import torch
+    from ctgb.device import fdkui_filter
+    gama, xi, beta, b0, fan, D, ds = _curved(lg, 3, 4)
+    R = (1.0 + np.random.default_rng(lg).random((4, 3, lg))) * scale
+    ref = oracle.fdkui_filter(R, xi, gama, beta, b0, fan, D, ds)
+    got = fdkui_filter(torch.from_numpy(R).cuda(), xi, gama, beta, b0, fan, D, ds).cpu().numpy()
+    assert rel_l2(got, ref) <= 2e-7
+
+
+def test_curved_backprojection_in_view_chunks(oracle):
+    """More views than the records of one launch hold (170 at 512 x 512 columns), one and 17 slices."""
+    import torch
+    from ctgb.device import fdkui_bp
+    for n, nz, views in ((512, 1, 172), (40, 17, 9)):
+        gama, xi, beta, _, _, D, ds = _curved(60, 8, views)
+        D, ds = D * n / 90, ds * n / 90
+        xi = xi * (n / 90)
+        size = np.array([n, n, 2 if nz == 1 else n // 4], np.int32)
+        rc = np.random.default_rng(n).random((views, 8, 60)).astype(np.float32)
+        ref = oracle.fdkui_bp(rc, size, nz, beta, D, ds, gama, xi)
+        got = fdkui_bp(torch.from_numpy(rc).cuda(), xi, gama, beta, D, ds, size, nz).cpu().numpy()
+        assert rel_l2(got, ref) <= TOL
