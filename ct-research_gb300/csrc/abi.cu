@@ -734,9 +734,13 @@ static int fan_ray_table(ct_fan_plan *pl) {
     const FanGeom &g = pl->g;
     const size_t bytes = sizeof(FanRay) * (size_t)g.nb * g.np;
     if (bytes > kFanRayTableMax) return CT_OK;
-    int s = pl->rays.ensure(bytes);
-    if (s || (s = fan_ray_table_launch(g, pl->rays.as<FanRay>(), nullptr))) return s;
-    CT_CUDA(cudaStreamSynchronize(nullptr), "ray set-up table");
+    // the grazing count behind the table
+    int s = pl->rays.ensure(bytes + sizeof(unsigned long long));
+    if (s) return s;
+    unsigned long long *d_n = reinterpret_cast<unsigned long long *>(pl->rays.as<char>() + bytes), n = 0;
+    if ((s = fan_ray_table_launch(g, pl->rays.as<FanRay>(), d_n, nullptr))) return s;
+    CT_CUDA(cudaMemcpy(&n, d_n, sizeof(n), cudaMemcpyDeviceToHost), "ray set-up table");
+    pl->g.grazing = (long long)n;
     pl->g.ray_tab = pl->rays.as<FanRay>();
     return CT_OK;
 }
@@ -1251,6 +1255,13 @@ struct ct_fan_batch {
     }
 };
 
+// No slice has a grazing ray (by the set-up tables): nothing to list or re-walk.
+static bool batch_no_grazing(const ct_fan_batch *b) {
+    for (const BatchSlice &s : b->h)
+        if (!s.g.ray_tab || s.g.grazing) return false;
+    return true;
+}
+
 // Offsets of every slice in the packed buffers and its first block in each grid.
 static int batch_layout(ct_fan_batch *b) {
     long long io = 0, so = 0, fb = 0, bb = 0;
@@ -1265,7 +1276,7 @@ static int batch_layout(ct_fan_batch *b) {
         const long long nr = (long long)s.g.nb * s.g.np, npx = (long long)s.g.nt * s.g.ns;
         io += npx;
         so += nr;
-        fb += (nr + b->fp_block - 1) / b->fp_block;
+        fb += (nr * fan_fp_lanes(s.g) + b->fp_block - 1) / b->fp_block;
         const int per = fan_batch_bp_pixels(b->bp_block);
         bb += (npx + per - 1) / per;
     }
@@ -1360,7 +1371,7 @@ int ct_fan_batch_fp(ct_fan_batch *b, const float *d_img, float *d_proj, void *st
     int s = graze_list(b->graze, gl, b->sino_total, as_stream(stream));
     if (s) return s;
     return fan_batch_fp_launch(b->desc.as<BatchSlice>(), (int)b->h.size(), b->fp_blocks, b->fp_block, d_img, d_proj,
-                               nullptr, nullptr, 0.f, nullptr, 0, gl, as_stream(stream));
+                               nullptr, nullptr, 0.f, nullptr, 0, gl, batch_no_grazing(b), as_stream(stream));
 }
 
 int ct_fan_batch_fp_residual(ct_fan_batch *b, const float *d_img, const float *d_b, const float *d_rowsum, float eps,
@@ -1370,7 +1381,7 @@ int ct_fan_batch_fp_residual(ct_fan_batch *b, const float *d_img, const float *d
     int s = graze_list(b->graze, gl, b->sino_total, as_stream(stream));
     if (s) return s;
     return fan_batch_fp_launch(b->desc.as<BatchSlice>(), (int)b->h.size(), b->fp_blocks, b->fp_block, d_img, d_out,
-                               d_b, d_rowsum, eps, d_norms, 1, gl, as_stream(stream));
+                               d_b, d_rowsum, eps, d_norms, 1, gl, batch_no_grazing(b), as_stream(stream));
 }
 
 int ct_fan_batch_bp(ct_fan_batch *b, const float *d_proj, float *d_img, void *stream) {

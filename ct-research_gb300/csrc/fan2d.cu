@@ -15,12 +15,13 @@ __global__ void __launch_bounds__(F2_BLOCK)
 fan_fp_kernel(const FanGeom g, const float *__restrict__ img, OutT *__restrict__ out,
               const float *__restrict__ b, const float *__restrict__ rowsum, float eps,
               double *__restrict__ norms, const GrazeList gl) {
-    const long long r = (long long)blockIdx.x * F2_BLOCK + threadIdx.x;
+    const int lanes = fan_ray_lanes(g);
+    const long long r = ((long long)blockIdx.x * F2_BLOCK + threadIdx.x) / lanes;
+    bool grazing;
     const bool active = r < (long long)g.nb * g.np;
+    const float val = fan_ray_value(g, img, r, lanes, active, grazing);
     float r2 = 0.0f, b2 = 0.0f;
-    if (active) {
-        bool grazing;
-        const float val = fan_ray_value(g, img, r, grazing);
+    if (active && threadIdx.x % lanes == 0) {
         if (grazing) graze_push(gl, (unsigned long long)r, (unsigned long long)r);
         if (MODE == 0) {
             out[r] = (OutT)val;
@@ -34,8 +35,7 @@ fan_fp_kernel(const FanGeom g, const float *__restrict__ img, OutT *__restrict__
         }
     }
     if (MODE == 1) {
-        block_sum_atomic_f<F2_BLOCK / 32>(r2, norms);
-        block_sum_atomic_f<F2_BLOCK / 32>(b2, norms + 1);
+        block_sum_pair(r2, b2, norms);
     }
 }
 
@@ -57,12 +57,14 @@ fan_bp_kernel(const FanGeom g, const float *__restrict__ R, float *__restrict__ 
 
 }  // namespace
 
-// The set-up table: ray r's walk set-up as fan_ray_setup_compute makes it.
+// The set-up table: ray r's walk set-up as fan_ray_setup_compute makes it, and the
+// number of grazing rays.
 __global__ void __launch_bounds__(256)
-fan_ray_table_kernel(const FanGeom g, FanRay *__restrict__ tab) {
+fan_ray_table_kernel(const FanGeom g, FanRay *__restrict__ tab, unsigned long long *__restrict__ grazing) {
     const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (r >= (long long)g.nb * g.np) return;
     RayWalk w;
+    w.grazing = false;
     const bool hit = fan_ray_setup_compute(g, r, w);
     FanRay t;
     t.a0t = w.a0; t.a0s = w.a1; t.dat = w.d0; t.das = w.d1;
@@ -72,14 +74,16 @@ fan_ray_table_kernel(const FanGeom g, FanRay *__restrict__ tab) {
     t.flags = (hit ? 1 : 0) | (w.grazing ? 2 : 0);
     t.pad_ = 0;
     tab[r] = t;
+    if (hit && w.grazing) atomicAdd(grazing, 1ULL);
 }
 
-int fan_ray_table_launch(const FanGeom &g0, FanRay *tab, cudaStream_t st) {
+int fan_ray_table_launch(const FanGeom &g0, FanRay *tab, unsigned long long *grazing, cudaStream_t st) {
     FanGeom g = g0;
     fan_geom_derive(g);
     g.ray_tab = nullptr;
     const long long n = (long long)g.nb * g.np;
-    fan_ray_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, tab);
+    CT_CUDA(cudaMemsetAsync(grazing, 0, sizeof(*grazing), st), "grazing count");
+    fan_ray_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, tab, grazing);
     CT_LAUNCH_CHECK("fan_ray_table_kernel");
     return CT_OK;
 }
@@ -89,9 +93,11 @@ int fan_fp_launch(const FanGeom &g0, const float *img, void *out, const float *b
                   float eps, double *norms, int mode, const GrazeList &gl, cudaStream_t st) {
     FanGeom g = g0;
     fan_geom_derive(g);
-    const long long nray = (long long)g.nb * g.np;
+    const long long nray = (long long)g.nb * g.np * fan_ray_lanes(g);
     const unsigned blocks = (unsigned)((nray + F2_BLOCK - 1) / F2_BLOCK);
-    CT_CUDA(cudaMemsetAsync(gl.count, 0, sizeof(*gl.count), st), "graze list reset");
+    // a plan whose set-up table has no grazing ray lists none: no reset and no re-walk
+    const bool none = g.ray_tab && g.grazing == 0;
+    if (!none) CT_CUDA(cudaMemsetAsync(gl.count, 0, sizeof(*gl.count), st), "graze list reset");
     if (mode == 0)
         fan_fp_kernel<float, 0><<<blocks, F2_BLOCK, 0, st>>>(g, img, (float *)out, nullptr, nullptr, 0.f, nullptr, gl);
     else if (mode == 1)
@@ -99,6 +105,7 @@ int fan_fp_launch(const FanGeom &g0, const float *img, void *out, const float *b
     else
         fan_fp_kernel<double, 0><<<blocks, F2_BLOCK, 0, st>>>(g, img, (double *)out, nullptr, nullptr, 0.f, nullptr, gl);
     CT_LAUNCH_CHECK("fan_fp_kernel");
+    if (none) return CT_OK;
     return fan_fixup_launch(g, img, out, mode == 3, b, rowsum, eps, norms, mode == 1 ? 1 : 0, gl, st);
 }
 

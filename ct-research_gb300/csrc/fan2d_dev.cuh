@@ -82,15 +82,33 @@ __device__ __forceinline__ bool fan_ray_setup(const FanGeom &g, long long r, Ray
     return (flags & 1) != 0;
 }
 
-// Line integral of ray r = view * np + bin; sets `grazing` for rays the FP64
-// re-walk must redo (ref_walk.cu).
-__device__ __forceinline__ float fan_ray_value(const FanGeom &g, const float *__restrict__ img, long long r,
-                                               bool &grazing) {
+// Lanes per ray of the forward projection: rays of a small sinogram are walked
+// by kRayParts lanes each (a walk is one chain of ~1.5 n steps; at 90 x 256 rays
+// the GPU holds 7 times as many threads), decided by the sinogram alone.
+// 128^2, 90 views of 256 bins: 18.3 -> 12 us for the projection with the residual.
+constexpr long long kSplitRays = 65536;
+__host__ __device__ inline int fan_ray_lanes(const FanGeom &g) {
+    return (long long)g.nb * g.np <= kSplitRays ? kRayParts : 1;
+}
+
+// Line integral of ray r = view * np + bin, by `lanes` consecutive lanes (each gets
+// it; all lanes of the warp take part when lanes > 1); sets `grazing` for rays
+// the FP64 re-walk must redo (ref_walk.cu).
+__device__ __forceinline__ float fan_ray_value(const FanGeom &g, const float *__restrict__ img, long long r, int lanes,
+                                               bool active, bool &grazing) {
     RayWalk w;
+    float v = 0.0f;
     grazing = false;
-    if (!fan_ray_setup(g, r, w)) return 0.0f;
-    grazing = w.grazing;
-    return ray_integral(w, img, g.nt * g.ns - 1);
+    const unsigned nmax = (unsigned)(g.nt * g.ns - 1);
+    if (active && fan_ray_setup(g, r, w)) {
+        grazing = w.grazing;
+        v = lanes > 1 ? ray_part_2d(w, img, nmax, threadIdx.x % kRayParts) : ray_integral_2d(w, img, nmax);
+    }
+    if (lanes > 1) {
+#pragma unroll
+        for (int d = 1; d < kRayParts; d <<= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, d));
+    }
+    return v;
 }
 
 // The reference's weight 2 |T1S1 - End| of one pixel-view in FP64
@@ -471,35 +489,25 @@ __device__ __forceinline__ void fan_bp_block(const FanGeom &g, const float *__re
     }
 }
 
-// Block-level sum of a double into *out with one atomic per block, for any
-// blockDim.x that is a multiple of 32 and at most 1024.
-__device__ __forceinline__ void block_sum_any(double v, double *out) {
-    __shared__ double part[32];
-    v = warp_sum(v);
+// Sums of two per-thread FP32 terms over the block into out[0], out[1], for any
+// blockDim.x that is a multiple of 32 and at most 1024: FP32 warp sums, FP64
+// partials, one barrier and two atomics per block.
+__device__ __forceinline__ void block_sum_pair(float a, float b, double *out) {
+    __shared__ double part[2][32];
+    a = warp_sum(a);
+    b = warp_sum(b);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0) part[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        double w = lane < nw ? part[lane] : 0.0;
-        w = warp_sum(w);
-        if (lane == 0) atomicAdd(out, w);
+    if (lane == 0) {
+        part[0][wid] = (double)a;
+        part[1][wid] = (double)b;
     }
     __syncthreads();
-}
-
-// block_sum_any for per-thread FP32 terms (FP32 warp sums, FP64 partials).
-__device__ __forceinline__ void block_sum_any_f(float v, double *out) {
-    __shared__ double part[32];
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0) part[wid] = (double)v;
-    __syncthreads();
-    if (wid == 0) {
-        double w = lane < nw ? part[lane] : 0.0;
-        w = warp_sum(w);
-        if (lane == 0) atomicAdd(out, w);
+    if (wid < 2 && wid < nw) {
+        for (int j = wid; j < 2; j += nw) {
+            const double w = warp_sum(lane < nw ? part[j][lane] : 0.0);
+            if (lane == 0) atomicAdd(out + j, w);
+        }
     }
-    __syncthreads();
 }
 
 }  // namespace ct

@@ -44,13 +44,14 @@ fan_batch_fp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__r
                     float *__restrict__ out, const float *__restrict__ b, const float *__restrict__ rowsum,
                     float eps, double *__restrict__ norms, const GrazeList gl) {
     const int k = find_slice(sl, nsl, false);
-    const FanGeom g = sl[k].g;
-    const long long r = (long long)(blockIdx.x - sl[k].ray_blk0) * blockDim.x + threadIdx.x;
+    const FanGeom &g = sl[k].g;
+    const int lanes = fan_ray_lanes(g);
+    const long long r = ((long long)(blockIdx.x - sl[k].ray_blk0) * blockDim.x + threadIdx.x) / lanes;
+    bool grazing;
     const bool active = r < (long long)g.nb * g.np;
+    const float val = fan_ray_value(g, img + sl[k].img_off, r, lanes, active, grazing);
     float r2 = 0.0f, b2 = 0.0f;
-    if (active) {
-        bool grazing;
-        const float val = fan_ray_value(g, img + sl[k].img_off, r, grazing);
+    if (active && threadIdx.x % lanes == 0) {
         const long long o = sl[k].sino_off + r;
         if (grazing) graze_push(gl, ((unsigned long long)k << 40) | (unsigned long long)r, (unsigned long long)o);
         if (MODE == 0) {
@@ -65,8 +66,7 @@ fan_batch_fp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__r
         }
     }
     if (MODE == 1) {
-        block_sum_any_f(r2, norms + 2 * k);
-        block_sum_any_f(b2, norms + 2 * k + 1);
+        block_sum_pair(r2, b2, norms + 2 * k);
     }
 }
 
@@ -96,16 +96,19 @@ fan_batch_bp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__r
 
 int fan_batch_fp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block, const float *img, float *out,
                         const float *b, const float *rowsum, float eps, double *norms, int mode, const GrazeList &gl,
-                        cudaStream_t st) {
+                        bool no_grazing, cudaStream_t st) {
     CT_REQUIRE(block >= 32 && block <= 512 && block % 32 == 0, "batch: block size must be a multiple of 32 <= 512");
-    CT_CUDA(cudaMemsetAsync(gl.count, 0, sizeof(*gl.count), st), "graze list reset");
+    if (!no_grazing) CT_CUDA(cudaMemsetAsync(gl.count, 0, sizeof(*gl.count), st), "graze list reset");
     if (mode == 0)
         fan_batch_fp_kernel<0><<<nblocks, block, 0, st>>>(d_sl, nsl, img, out, nullptr, nullptr, 0.f, nullptr, gl);
     else
         fan_batch_fp_kernel<1><<<nblocks, block, 0, st>>>(d_sl, nsl, img, out, b, rowsum, eps, norms, gl);
     CT_LAUNCH_CHECK("fan_batch_fp_kernel");
+    if (no_grazing) return CT_OK;
     return fan_batch_fixup_launch(d_sl, nsl, img, out, b, rowsum, eps, norms, mode, gl, st);
 }
+
+int fan_fp_lanes(const FanGeom &g) { return fan_ray_lanes(g); }
 
 int fan_batch_bp_pixels(int block) { return fan_bp_pixels(block); }
 

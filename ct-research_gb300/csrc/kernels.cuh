@@ -30,6 +30,7 @@ struct FanGeom {
     float near_q;
     // the walk set-up of every ray (fan_ray_table_launch), or null: computed per ray
     const struct FanRay *ray_tab;
+    long long grazing;       // grazing rays of ray_tab
 };
 
 // The forward walk's set-up of one 2D ray, as the FP64 slab test makes it
@@ -177,7 +178,8 @@ int cone_bp_launch(const ConeGeom &g, const float2 *Q, void *tab, bool tab_ready
 int cone_bp_ztile(const ConeGeom &g);
 int row_filter_launch(const RowFilter &f, const float *R, float *out, cudaStream_t st);
 // The set-up table of every ray of g (nb * np records), for g.ray_tab.
-int fan_ray_table_launch(const FanGeom &g, FanRay *tab, cudaStream_t st);
+// *grazing (device) becomes the number of grazing rays.
+int fan_ray_table_launch(const FanGeom &g, FanRay *tab, unsigned long long *grazing, cudaStream_t st);
 int fan_fp_launch(const FanGeom &g, const float *img, void *out, const float *b, const float *rowsum,
                   float eps, double *norms, int mode, const GrazeList &gl, cudaStream_t st);
 int fan_bp_launch(const FanGeom &g, const float *R, float *img, int wmode, const float *colsum, float eps,
@@ -214,7 +216,9 @@ struct BatchSlice {
 
 int fan_batch_fp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block, const float *img, float *out,
                         const float *b, const float *rowsum, float eps, double *norms, int mode, const GrazeList &gl,
-                        cudaStream_t st);
+                        bool no_grazing, cudaStream_t st);
+// lanes that walk one ray of g
+int fan_fp_lanes(const FanGeom &g);
 // pixels a block of `block` threads of the batched backprojection covers
 int fan_batch_bp_pixels(int block);
 int fan_batch_bp_launch(const BatchSlice *d_sl, int nsl, int nblocks, int block, const float *R, float *img, int wmode,

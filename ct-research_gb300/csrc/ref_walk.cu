@@ -117,9 +117,17 @@ __device__ float cone_ray_ref(const ConeGeom &g, const float *__restrict__ vol, 
     return (float)ray;
 }
 
-// ProjectionFan (ProjectionFan_2D.cu:19-216): double angle and bin.
-template <class Visit>
-__device__ void fan_walk_ref(const FanGeom &g, double sb, double cb, double P, Visit &&visit) {
+// A 2D reference walk in progress: the line (a source point and both slopes) and
+// the current point in voxel units.
+struct Walk2 {
+    double r1, r2, src_t, src_s, t2s, s2t;
+    int sig_t, sig_s, up_t, up_s;
+    double tc, sc;
+};
+
+// ProjectionFan (ProjectionFan_2D.cu:19-216): double angle and bin.  The walk's
+// start; false for rays that miss.
+__device__ bool fan_ref_start(const FanGeom &g, double sb, double cb, double P, Walk2 &k) {
     const double r1 = g.res[0], r2 = g.res[1], D = g.D;
     const int nt = g.nt, ns = g.ns;
     const double ct = g.size[0] / 2, cs = g.size[1] / 2;
@@ -140,44 +148,20 @@ __device__ void fan_walk_ref(const FanGeom &g, double sb, double cb, double P, V
                         ft[3] >= 0 && ft[3] <= thi};
     int first = -1, second = -1;
     for (int f = 0; f < 4; ++f) if (ok[f]) { first = f; break; }
-    if (first < 0 || first == 3) return;
+    if (first < 0 || first == 3) return false;
     for (int f = first + 1; f < 4; ++f) if (ok[f]) { second = f; break; }
     const double T1 = ft[first], S1 = fs[first];
     double T2 = 0, S2 = 0;
     if (second >= 0) { T2 = ft[second]; S2 = fs[second]; }
     double Ts, Ss;
     if (d2(T1, S1, src_t, src_s) >= d2(T2, S2, src_t, src_s)) { Ts = T2; Ss = S2; } else { Ts = T1; Ss = S1; }
-    double tc = Ts / r1, sc = Ss / r2;
-    const int up_t = (1 + sig_t) / 2, up_s = (1 + sig_s) / 2;
-    for (int i = 0; i < nt + ns - 1; ++i) {
-        short gt, gs;
-        if (fabs(tc - round(tc)) < EPS15) gt = (short)(round(tc) + sig_t); else gt = (short)(floor(tc) + up_t);
-        const double gt_s = (src_s + (gt * r1 - src_t) * t2s) / r2;
-        if (fabs(sc - round(sc)) < EPS15) gs = (short)(round(sc) + sig_s); else gs = (short)(floor(sc) + up_s);
-        const double gs_t = (src_t + (gs * r2 - src_s) * s2t) / r1;
-        double w, nt_, ns_;
-        if (d2(gt, gt_s, tc, sc) <= d2(gs_t, gs, tc, sc)) {
-            w = sqrt(d2(gt * r1, gt_s * r2, tc * r1, sc * r2)); nt_ = gt; ns_ = gt_s;
-        } else {
-            w = sqrt(d2(gs_t * r1, gs * r2, tc * r1, sc * r2)); nt_ = gs_t; ns_ = gs;
-        }
-        const int it = (int)floor((nt_ + tc) / 2), is = (int)floor((ns_ + sc) / 2);
-        tc = nt_; sc = ns_;
-        if (it >= 0 && it < nt && is >= 0 && is < ns) visit((long long)is * nt + it, w);
-        else break;
-    }
-}
-
-__device__ double fan_ray_ref(const FanGeom &g, const float *__restrict__ pic, double sb, double cb, double P) {
-    double ray = 0;
-    fan_walk_ref(g, sb, cb, P, [&](long long i, double w) { ray += w * pic[i]; });
-    return ray;
+    k = Walk2{r1, r2, src_t, src_s, t2s, s2t, sig_t, sig_s, (1 + sig_t) / 2, (1 + sig_s) / 2, Ts / r1, Ss / r2};
+    return true;
 }
 
 // ProjectionParallel (ProjectionParallel_2D.cu:23-243); x = t axis (width),
 // y = s axis (height) of the FanGeom.
-template <class Visit>
-__device__ void par_walk_ref(const FanGeom &g, double sb, double cb, double t, Visit &&visit) {
+__device__ bool par_ref_start(const FanGeom &g, double sb, double cb, double t, Walk2 &k) {
     const double rx = g.res[0], ry = g.res[1], smax = g.smax;
     const int wd = g.nt, h = g.ns;
     const double cx = g.size[0] / 2, cy = g.size[1] / 2;
@@ -194,11 +178,11 @@ __device__ void par_walk_ref(const FanGeom &g, double sb, double cb, double t, V
                         fy[3] >= 0 && fy[3] <= yhi};
     int first = -1;
     for (int f = 0; f < 4; ++f) if (ok[f]) { first = f; break; }
-    if (first < 0 || first == 3) return;
+    if (first < 0 || first == 3) return false;
     const int order[3][3] = {{2, 3, 1}, {2, 3, -1}, {3, -1, -1}};
     int second = -1;
-    for (int k = 0; k < 3; ++k) {
-        const int f = order[first][k];
+    for (int i = 0; i < 3; ++i) {
+        const int f = order[first][i];
         if (f >= 0 && ok[f]) { second = f; break; }
     }
     const double X1 = fx[first], Y1 = fy[first];
@@ -206,31 +190,105 @@ __device__ void par_walk_ref(const FanGeom &g, double sb, double cb, double t, V
     if (second >= 0) { X2 = fx[second]; Y2 = fy[second]; }
     double Xs, Ys;
     if (d2(X1, Y1, xs, ys) >= d2(X2, Y2, xs, ys)) { Xs = X2; Ys = Y2; } else { Xs = X1; Ys = Y1; }
-    double xc = Xs / rx, yc = Ys / ry;
-    const int up_x = (1 + sig_x) / 2, up_y = (1 + sig_y) / 2;
-    for (int i = 0; i < h + wd - 1; ++i) {
-        short gx, gy;
-        if (fabs(xc - round(xc)) < ERR5) gx = (short)(round(xc) + sig_x); else gx = (short)(floor(xc) + up_x);
-        const double gx_y = (ys + (gx * rx - xs) * x2y) / ry;
-        if (fabs(yc - round(yc)) < ERR5) gy = (short)(round(yc) + sig_y); else gy = (short)(floor(yc) + up_y);
-        const double gy_x = (xs + (gy * ry - ys) * y2x) / rx;
-        double w, nx_, ny_;
-        if (d2(gx, gx_y, xc, yc) >= d2(gy_x, gy, xc, yc)) {
-            w = sqrt(d2(gy_x * rx, gy * ry, xc * rx, yc * ry)); nx_ = gy_x; ny_ = gy;
-        } else {
-            w = sqrt(d2(gx * rx, gx_y * ry, xc * rx, yc * ry)); nx_ = gx; ny_ = gx_y;
-        }
-        const int ix = (int)floor((nx_ + xc) / 2), iy = (int)floor((ny_ + yc) / 2);
-        xc = nx_; yc = ny_;
-        if (ix >= 0 && ix < wd && iy >= 0 && iy < h) visit((long long)iy * wd + ix, w);
+    k = Walk2{rx, ry, xs, ys, x2y, y2x, sig_x, sig_y, (1 + sig_x) / 2, (1 + sig_y) / 2, Xs / rx, Ys / ry};
+    return true;
+}
+
+// The next grid planes of a point (gt, gs), each with the line's other coordinate there.
+template <bool PAR>
+__device__ __forceinline__ void ref_planes(const Walk2 &k, double tc, double sc, short &gt, short &gs, double &gt_s,
+                                           double &gs_t) {
+    const double eps = PAR ? ERR5 : EPS15;
+    if (fabs(tc - round(tc)) < eps) gt = (short)(round(tc) + k.sig_t); else gt = (short)(floor(tc) + k.up_t);
+    gt_s = (k.src_s + (gt * k.r1 - k.src_t) * k.t2s) / k.r2;
+    if (fabs(sc - round(sc)) < eps) gs = (short)(round(sc) + k.sig_s); else gs = (short)(floor(sc) + k.up_s);
+    gs_t = (k.src_t + (gs * k.r2 - k.src_s) * k.s2t) / k.r1;
+}
+
+// One step of the reference's walk from (tc, sc): the nearer of the next planes,
+// the segment's length w and its midpoint's voxel (it, is).
+template <bool PAR>
+__device__ __forceinline__ void ref_step(const Walk2 &k, double tc, double sc, double &tn, double &sn, double &w,
+                                         int &it, int &is) {
+    short gt, gs;
+    double gt_s, gs_t;
+    ref_planes<PAR>(k, tc, sc, gt, gs, gt_s, gs_t);
+    const double dT = d2(gt, gt_s, tc, sc), dS = d2(gs_t, gs, tc, sc);
+    // a tie goes to t in the fan walk and to s in the parallel one
+    if (PAR ? dT < dS : dT <= dS) {
+        w = sqrt(d2(gt * k.r1, gt_s * k.r2, tc * k.r1, sc * k.r2)); tn = gt; sn = gt_s;
+    } else {
+        w = sqrt(d2(gs_t * k.r1, gs * k.r2, tc * k.r1, sc * k.r2)); tn = gs_t; sn = gs;
+    }
+    it = (int)floor((tn + tc) / 2);
+    is = (int)floor((sn + sc) / 2);
+}
+
+// The walk, one step after the other; visit(pixel, length) in walk order.
+template <bool PAR, class Visit>
+__device__ void walk2_ref(const FanGeom &g, double sb, double cb, double P, Visit &&visit) {
+    Walk2 k;
+    if (!(PAR ? par_ref_start(g, sb, cb, P, k) : fan_ref_start(g, sb, cb, P, k))) return;
+    double tc = k.tc, sc = k.sc;
+    for (int i = 0; i < g.nt + g.ns - 1; ++i) {
+        double tn, sn, w;
+        int it, is;
+        ref_step<PAR>(k, tc, sc, tn, sn, w, it, is);
+        tc = tn; sc = sn;
+        if (it >= 0 && it < g.nt && is >= 0 && is < g.ns) visit((long long)is * g.nt + it, w);
         else break;
     }
 }
 
-__device__ double par_ray_ref(const FanGeom &g, const float *__restrict__ pic, double sb, double cb, double t) {
-    double ray = 0;
-    par_walk_ref(g, sb, cb, t, [&](long long i, double w) { ray += w * pic[i]; });
-    return ray;
+// The line integral of a grazing ray by a whole warp (every lane gets it).  Such a
+// ray runs along a grid line, so nearly all its steps cross the planes of one
+// axis: lane j takes its step from the point that j such crossings lead to
+// (a point on a plane depends on the plane alone), and the steps are the walk's as
+// far as each lane's point is, bit for bit, where the step before it ended.
+// ~1000 FP64 steps of a 512^2 slice in a chain took 1.57 ms, whatever the number
+// of rays; 32 at a time, with the two-axis walk, the projection of 64 slices with its
+// re-walk took 3.5 ms instead of 5.7.
+template <bool PAR>
+__device__ double warp_ray_ref(const FanGeom &g, const float *__restrict__ pic, double sb, double cb, double P) {
+    Walk2 k;
+    if (!(PAR ? par_ref_start(g, sb, cb, P, k) : fan_ref_start(g, sb, cb, P, k))) return 0.0;
+    const int lane = threadIdx.x & 31;
+    const bool along_s = fabs(k.s2t) < fabs(k.t2s);      // crosses the s planes
+    double tc = k.tc, sc = k.sc, ray = 0.0;
+    int left = g.nt + g.ns - 1;
+    while (left > 0) {
+        short gt, gs;
+        double gt_s, gs_t, pt = tc, ps = sc;
+        ref_planes<PAR>(k, tc, sc, gt, gs, gt_s, gs_t);
+        if (lane > 0) {
+            if (along_s) {
+                const short q = (short)(gs + (lane - 1) * k.sig_s);
+                pt = (k.src_t + (q * k.r2 - k.src_s) * k.s2t) / k.r1;
+                ps = q;
+            } else {
+                const short q = (short)(gt + (lane - 1) * k.sig_t);
+                pt = q;
+                ps = (k.src_s + (q * k.r1 - k.src_t) * k.t2s) / k.r2;
+            }
+        }
+        double tn, sn, w;
+        int it, is;
+        ref_step<PAR>(k, pt, ps, tn, sn, w, it, is);
+        const double tb = __shfl_up_sync(0xffffffffu, tn, 1), sb_ = __shfl_up_sync(0xffffffffu, sn, 1);
+        const bool same = lane == 0 || (__double_as_longlong(tb) == __double_as_longlong(pt) &&
+                                        __double_as_longlong(sb_) == __double_as_longlong(ps));
+        const unsigned bad = __ballot_sync(0xffffffffu, !same);
+        const int n = min(bad ? __ffs(bad) - 1 : 32, left);            // steps of the walk
+        const bool in = it >= 0 && it < g.nt && is >= 0 && is < g.ns;
+        const unsigned out = __ballot_sync(0xffffffffu, !in) & (n == 32 ? 0xffffffffu : (1u << n) - 1u);
+        const int m = out ? __ffs(out) - 1 : n;                         // steps before it leaves the image
+        if (lane < m) ray += w * pic[(long long)is * g.nt + it];
+        if (out) break;
+        tc = __shfl_sync(0xffffffffu, tn, n - 1);
+        sc = __shfl_sync(0xffffffffu, sn, n - 1);
+        left -= n;
+    }
+    return warp_sum(ray);
 }
 
 // Visit every grazing ray the fast kernel recorded: the listed entries, and,
@@ -263,6 +321,30 @@ __device__ __forceinline__ void graze_drain(const GrazeList &gl, OnEntry on_entr
     }
 }
 
+// graze_drain for warps: each entry or bit by a whole warp.
+template <class OnEntry, class OnBit>
+__device__ __forceinline__ void graze_drain_warps(const GrazeList &gl, OnEntry on_entry, OnBit on_bit) {
+    const unsigned long long cnt = *gl.count;
+    const long long n = (long long)min(cnt, (unsigned long long)gl.cap);
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    const long long warp = (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = (long long)gridDim.x * wpb;
+    for (long long i = warp; i < n; i += nwarps) on_entry(gl.rays[i]);
+    if (cnt > (unsigned long long)gl.cap && gl.bits) {
+        const long long nw = (gl.nbits + 31) >> 5;
+        for (long long w = warp; w < nw; w += nwarps) {
+            unsigned m = gl.bits[w];
+            __syncwarp();
+            if (!m) continue;
+            if (lane == 0) gl.bits[w] = 0u;
+            while (m) {
+                const int bit = __ffs(m) - 1;
+                m &= m - 1;
+                on_bit((unsigned long long)w * 32 + bit);
+            }
+        }
+    }
+}
+
 // Re-walk the recorded rays.  mode 0: out = A x;  mode 1: out = (b - A x) * scale
 // with norms[0] corrected by the change of the squared residual.
 __global__ void __launch_bounds__(64)
@@ -285,15 +367,21 @@ cone_fixup_kernel(const ConeGeom g, const float *__restrict__ vol, float *__rest
     graze_drain(gl, fix, fix);
 }
 
+// The value of a ray of the 2D geometry by a whole warp.
+__device__ __forceinline__ double warp_fan_value(const FanGeom &g, const float *__restrict__ img, unsigned long long r) {
+    const int p = (int)(r % g.np), v = (int)(r / g.np);
+    const double2 tr = g.trig_d[v];
+    return g.parallel ? warp_ray_ref<true>(g, img, tr.x, tr.y, g.Pd[p]) : warp_ray_ref<false>(g, img, tr.x, tr.y, g.Pd[p]);
+}
+
 template <typename OutT>
 __global__ void __launch_bounds__(64)
 fan_fixup_kernel(const FanGeom g, const float *__restrict__ img, OutT *__restrict__ out,
                  const float *__restrict__ b, const float *__restrict__ rowsum, float eps, double *norms, int mode,
                  const GrazeList gl) {
     auto fix = [&](unsigned long long r) {
-        const int p = (int)(r % g.np), v = (int)(r / g.np);
-        const double2 tr = g.trig_d[v];
-        const double val = g.parallel ? par_ray_ref(g, img, tr.x, tr.y, g.Pd[p]) : fan_ray_ref(g, img, tr.x, tr.y, g.Pd[p]);
+        const double val = warp_fan_value(g, img, r);
+        if ((threadIdx.x & 31) != 0) return;
         if (mode == 0) {
             out[r] = (OutT)val;
         } else {
@@ -303,7 +391,7 @@ fan_fixup_kernel(const FanGeom g, const float *__restrict__ img, OutT *__restric
             atomicAdd(norms, (double)rr * rr);   // the fast kernel left this ray out of the norm
         }
     };
-    graze_drain(gl, fix, fix);
+    graze_drain_warps(gl, fix, fix);
 }
 
 // Batched slices: list entries are (slice << 40) | ray; bitmap bits are the
@@ -313,11 +401,8 @@ fan_batch_fixup_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *
                        float *__restrict__ out, const float *__restrict__ b, const float *__restrict__ rowsum,
                        float eps, double *norms, int mode, const GrazeList gl) {
     auto fix = [&](int k, unsigned long long r) {
-        const FanGeom g = sl[k].g;
-        const int p = (int)(r % g.np), v = (int)(r / g.np);
-        const double2 tr = g.trig_d[v];
-        const float *im = img + sl[k].img_off;
-        const double val = g.parallel ? par_ray_ref(g, im, tr.x, tr.y, g.Pd[p]) : fan_ray_ref(g, im, tr.x, tr.y, g.Pd[p]);
+        const double val = warp_fan_value(sl[k].g, img + sl[k].img_off, r);
+        if ((threadIdx.x & 31) != 0) return;
         const long long o = sl[k].sino_off + (long long)r;
         if (mode == 0) {
             out[o] = (float)val;
@@ -337,7 +422,7 @@ fan_batch_fixup_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *
         }
         fix(lo, o - (unsigned long long)sl[lo].sino_off);
     };
-    graze_drain(gl, on_entry, on_bit);
+    graze_drain_warps(gl, on_entry, on_bit);
 }
 
 // One CSR row from a reference walk: pieces of zero length are dropped and
@@ -387,8 +472,8 @@ fan_sysmat_ref_kernel(const FanGeom g, long long *__restrict__ row_ptr, int *__r
         const int p = (int)(r % g.np), v = (int)(r / g.np);
         const double2 tr = g.trig_d[v];
         CsrRow e{fill, col, val, fill ? row_ptr[r] : 0, 0, -1};
-        if (g.parallel) par_walk_ref(g, tr.x, tr.y, g.Pd[p], e);
-        else fan_walk_ref(g, tr.x, tr.y, g.Pd[p], e);
+        if (g.parallel) walk2_ref<true>(g, tr.x, tr.y, g.Pd[p], e);
+        else walk2_ref<false>(g, tr.x, tr.y, g.Pd[p], e);
         if (!fill) row_ptr[r + 1] = e.n;
     };
     graze_drain(gl, row_of, row_of);

@@ -171,4 +171,75 @@ __device__ __forceinline__ float ray_integral(RayWalk &w, const float *__restric
     return acc * w.scale;
 }
 
+// Steps `first` .. `last` of a ray on one slice (no z crossings), from parameter
+// acur with k0, k1 crossings of the two axes behind it, and the rest of the
+// segment after them up to `end`; without the factor |d|.  An index that rounding
+// moves off the image is read as the last pixel (its segment is a rounding error
+// long).  Every rounding is written out, so that the single-slice and the
+// batched builds give identical results.
+__device__ __forceinline__ float walk_2d(const RayWalk &w, const float *__restrict__ img, unsigned nmax, int steps,
+                                         float acur, float k0, float k1, unsigned idx, float end) {
+    float acc = 0.0f;
+    float n0 = __fmaf_rn(k0, w.d0, w.a0), n1 = __fmaf_rn(k1, w.d1, w.a1);
+    auto step = [&](float &len, unsigned &vox) {
+        const float m = fminf(n0, n1);
+        const bool b0 = n0 <= n1;
+        len = __fsub_rn(m, acur);
+        acur = m;
+        vox = min(idx, nmax);
+        if (b0) k0 += 1.0f;
+        else k1 += 1.0f;
+        n0 = __fmaf_rn(k0, w.d0, w.a0);
+        n1 = __fmaf_rn(k1, w.d1, w.a1);
+        idx += (unsigned)(b0 ? w.s0 : w.s1);
+    };
+    int it = 0;
+    for (; it + 4 <= steps; it += 4) {
+        float l[4];
+        unsigned i[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) step(l[j], i[j]);
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = __ldg(img + i[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc = __fmaf_rn(l[j], v[j], acc);
+    }
+    for (; it < steps; ++it) {
+        float l;
+        unsigned i;
+        step(l, i);
+        acc = __fmaf_rn(l, __ldg(img + i), acc);
+    }
+    return __fmaf_rn(__fsub_rn(end, acur), __ldg(img + min(idx, nmax)), acc);
+}
+
+// Line integral of a ray on one slice.
+__device__ __forceinline__ float ray_integral_2d(const RayWalk &w, const float *__restrict__ img, unsigned nmax) {
+    return __fmul_rn(walk_2d(w, img, nmax, w.nseg - 1, 0.0f, 0.0f, 0.0f, (unsigned)w.idx, w.L), w.scale);
+}
+
+// Part `part` of kRayParts of a ray, cut at equal parameters: the crossings before
+// a cut follow from its parameter (the first k with a0 + k d0 >= cut).  Short
+// rays stay whole, in part 0.
+constexpr int kRayParts = 4, kRayPartMin = 16;
+__device__ __forceinline__ float ray_part_2d(const RayWalk &w, const float *__restrict__ img, unsigned nmax, int part) {
+    const int ninner = w.nseg - 1;
+    if (ninner < kRayPartMin) return part == 0 ? ray_integral_2d(w, img, nmax) : 0.0f;
+    auto crossings = [](float cut, float a, float d) {
+        if (!(d > 0.0f)) return 0.0f;
+        float k = fmaxf(ceilf(__fdividef(__fsub_rn(cut, a), d)), 0.0f);
+        if (k > 0.0f && __fmaf_rn(k - 1.0f, d, a) >= cut) k -= 1.0f;
+        if (__fmaf_rn(k, d, a) < cut) k += 1.0f;
+        return k;
+    };
+    const float c0 = __fmul_rn(w.L, (float)part / kRayParts), c1 = __fmul_rn(w.L, (float)(part + 1) / kRayParts);
+    const float k0 = part ? crossings(c0, w.a0, w.d0) : 0.0f, k1 = part ? crossings(c0, w.a1, w.d1) : 0.0f;
+    const int before = (int)k0 + (int)k1;
+    const bool last = part == kRayParts - 1;
+    const int upto = last ? ninner : (int)crossings(c1, w.a0, w.d0) + (int)crossings(c1, w.a1, w.d1);
+    const unsigned idx = (unsigned)(w.idx + (int)k0 * w.s0 + (int)k1 * w.s1);
+    return __fmul_rn(walk_2d(w, img, nmax, max(min(upto, ninner) - before, 0), c0, k0, k1, idx, last ? w.L : c1), w.scale);
+}
+
 }  // namespace ct

@@ -157,3 +157,29 @@ def test_curved_backprojection_in_view_chunks(oracle):
         ref = oracle.fdkui_bp(rc, size, nz, beta, D, ds, gama, xi)
         got = fdkui_bp(torch.from_numpy(rc).cuda(), xi, gama, beta, D, ds, size, nz).cpu().numpy()
         assert rel_l2(got, ref) <= TOL
+
+
+@pytest.mark.parametrize("n,views,bins", [(5, 4, 3), (64, 4, 41), (97, 8, 33), (300, 4, 601)])
+@pytest.mark.parametrize("parallel", [False, True])
+def test_grazing_rays_by_warps_and_split_rays(oracle, n, views, bins, parallel):
+    """Rays on grid lines (odd bins, views on the axes) around 32 steps and more, short rays that are not split, and a
+    sinogram above the size that is."""
+    import torch
+    from ctgb.device import FanPlan, ParPlan
+    from ctgb.geometry import FanGeometry
+    if parallel and n % 2:
+        pytest.skip("no parallel ray on a grid line")
+    views = 256 if bins == 601 and not parallel else views     # parallel: every ray runs along a grid line
+    rng = np.random.default_rng(n)
+    img = rng.random((n, n)).astype(np.float32)
+    ang = np.arange(1, views + 1) * (2 * np.pi / views)
+    P = (np.arange(bins) - (bins - 1) // 2) * 1.0
+    if parallel:
+        plan = ParPlan(n, n, (1.0, 1.0), ang, P)
+        ref = oracle.par_fp(img, ang, P, (float(n), float(n)))
+    else:
+        plan = FanPlan(FanGeometry(n, n, (float(n), float(n)), ang, P, 3.0 * n))
+        ref = oracle.fan_fp(img, ang, P, (float(n), float(n)), 3.0 * n)
+    got = plan.fp(torch.from_numpy(img).cuda()).cpu().numpy()
+    assert plan.grazing_rays() > 0 or n % 2
+    assert rel_l2(got, ref) <= TOL
