@@ -183,3 +183,22 @@ def test_grazing_rays_by_warps_and_split_rays(oracle, n, views, bins, parallel):
     got = plan.fp(torch.from_numpy(img).cuda()).cpu().numpy()
     assert plan.grazing_rays() > 0 or n % 2
     assert rel_l2(got, ref) <= TOL
+
+
+# (nz, ny, nx) around the gradient's warps (30 columns, 4 rows, 16 rows per block) and runs of planes
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 5, 7), (2, 4, 30), (3, 17, 31), (40, 16, 61), (33, 33, 90), (70, 3, 121)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_tv_gradient_tiles_and_alignment(shape, offset):
+    """One sub-step, its move 0.05 rms on values of ~0.5: FP32 rounding leaves ~1e-6 of the move.  offset: x starts 4
+    bytes off a 16-byte boundary."""
+    import torch
+    from ctgb.device import tv_flow
+    from oracle.oracle import tv_flow as tv_ref
+    n = int(np.prod(shape))
+    x = (0.5 + 0.2 * np.random.default_rng(n).normal(size=shape)).astype(np.float32)
+    buf = torch.zeros(n + 4, device="cuda")
+    t = buf[offset:offset + n].view(shape)
+    t.copy_(torch.from_numpy(x))
+    got = tv_flow(t, 1, 0.05, 1e-8, -1e9).cpu().numpy().astype(np.float64) - x
+    ref = tv_ref(x, 1, 0.05, 1e-8, -1e9) - x.astype(np.float64)
+    assert rel_l2(got, ref) <= TOL
