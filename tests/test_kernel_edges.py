@@ -202,3 +202,32 @@ def test_tv_gradient_tiles_and_alignment(shape, offset):
     got = tv_flow(t, 1, 0.05, 1e-8, -1e9).cpu().numpy().astype(np.float64) - x
     ref = tv_ref(x, 1, 0.05, 1e-8, -1e9) - x.astype(np.float64)
     assert rel_l2(got, ref) <= TOL
+
+
+def test_dropin_2d_plans_kept_between_calls(oracle):
+    """More geometries than plans are kept, of equal sizes but other contents, from several threads, twice, and after a
+    release."""
+    from concurrent.futures import ThreadPoolExecutor
+    from ctgb import _lib, ops
+    rng = np.random.default_rng(11)
+    size, n, nb, bins = np.array([24.0, 24.0]), 24, 20, 31
+    cases = []
+    for k in range(6):
+        beta = (np.arange(1, nb + 1) * (2 * np.pi / nb) + 0.01 * k).astype(np.float32)
+        P = (np.linspace(-30, 30, bins) * (1 + 0.01 * k)).astype(np.float32)
+        R = rng.random((nb, bins)).astype(np.float32)
+        D = 70.0 + (k == 5)
+        filt = oracle.fbpfan_filter(R, P, D, mode=1)
+        cases.append((R, beta, P, D, oracle.fbpfan_bp(filt, beta, P, size, (n, n), D),
+                      oracle.fan_bp(R, beta, P, size, (n, n), D)))
+
+    def check(k):
+        R, beta, P, D, fbp, bp = cases[k]
+        return (rel_l2(ops.FBPfan(R.ravel(), beta, P, size, n, n, D), fbp.ravel()),
+                rel_l2(ops.BackprojectionFan2D(R.ravel(), beta, P, size, n, n, D), bp.ravel()))
+
+    for rounds in range(2):
+        with ThreadPoolExecutor(4) as ex:
+            for errs in ex.map(check, [0, 0, 1, 2, 3, 4, 5, 0, 3]):
+                assert max(errs) <= TOL
+        _lib.call("ct_dropin_release")
