@@ -231,3 +231,37 @@ def test_dropin_2d_plans_kept_between_calls(oracle):
             for errs in ex.map(check, [0, 0, 1, 2, 3, 4, 5, 0, 3]):
                 assert max(errs) <= TOL
         _lib.call("ct_dropin_release")
+
+
+# channel-major x-shifted copies: whole 16-byte groups, channel tiles that end inside 32, 64-voxel blocks that end
+# inside a volume, an x of one group, and sizes and views that take the element-wise kernel.  The copies are exact.
+@pytest.mark.gpu
+@pytest.mark.parametrize("c,nb,nz,ny,nx,off", [(32, 2, 3, 5, 8, 0), (40, 1, 2, 3, 24, 8), (8, 1, 1, 1, 8, 0),
+                                               (64, 2, 4, 4, 64, 32), (32, 1, 2, 3, 12, 0), (12, 2, 2, 2, 16, 4),
+                                               (32, 1, 3, 3, 72, 1)])
+def test_shift_copies_groups_and_remainders(c, nb, nz, ny, nx, off):
+    import torch
+    from ctgb import _lib
+    from ctgb.unet import _tptr, _stream
+    g = torch.Generator(device="cuda").manual_seed(c + nx)
+    x = torch.randn((nb, nz, ny, nx, c), device="cuda", generator=g).to(torch.bfloat16)
+    ctot = c + off + 3
+    outs = [torch.full((nb, ctot, nz, ny, nx), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    for skip in (None, 0, 2):
+        ptr = [None if skip == k else _tptr(o) for k, o in enumerate(outs)]
+        for o in outs:
+            o.fill_(7.0)
+        _lib.call("ct_unet_shift_t", _tptr(x), c, nb, nz, ny, nx, *ptr, ctot, off, _stream())
+        t = x.permute(0, 4, 1, 2, 3)
+        for k, o in enumerate(outs):
+            ref = torch.full_like(o, 7.0)
+            if k != skip:
+                want = torch.zeros_like(t)
+                if k == 0:
+                    want[..., 1:] = t[..., :-1]
+                elif k == 1:
+                    want[...] = t
+                else:
+                    want[..., :-1] = t[..., 1:]
+                ref[:, off:off + c] = want
+            assert torch.equal(o, ref), (k, skip)
