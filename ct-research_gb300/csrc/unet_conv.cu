@@ -14,6 +14,8 @@
 //   concatenated along K (the skip connection) without a copy.  The epilogue
 //   adds the bias, applies ReLU or the ReLU-derivative mask of a saved
 //   activation, rounds to bf16 and splits the channels over one or two outputs.
+//   conv_march_kernel is the same convolution for few channels: it keeps the
+//   filters in shared memory and reads each input slice once.
 // * conv_wgrad_kernel (weight gradient): rows = (tap, input channel), columns
 //   = output channels, K = voxels in 64-voxel slices (128-byte rows, 128-byte
 //   swizzle).  Activations and output gradients are read channel-major
@@ -30,6 +32,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
+
+#include <algorithm>
 
 #include "ct_common.cuh"
 
@@ -294,6 +298,59 @@ struct FwdArgs {
     const __nv_bfloat16 *mask1, *mask2;   // ReLU-derivative masks (same layout as out1 / out2) or null
 };
 
+// ReLU-derivative mask values of columns c0 .. c0 + 15 of a voxel.
+struct Mask16 {
+    uint4 q0, q1;
+};
+
+__device__ __forceinline__ Mask16 load_mask(const FwdArgs &a, long long vox, int c0) {
+    const bool first = c0 < a.co1;
+    const __nv_bfloat16 *m = first ? a.mask1 : a.mask2;
+    Mask16 r{};
+    if (m) {
+        const uint4 *mp = reinterpret_cast<const uint4 *>(m + vox * (first ? a.co1 : a.co2) + (first ? c0 : c0 - a.co1));
+        r.q0 = __ldg(mp);
+        r.q1 = __ldg(mp + 1);
+    }
+    return r;
+}
+
+// Bias, ReLU, mask, rounding and the store of columns c0 .. c0 + 15 of a voxel.
+__device__ __forceinline__ void store16(const FwdArgs &a, long long vox, int c0, float (&v)[16], const Mask16 &mask) {
+    const bool first = c0 < a.co1;
+    __nv_bfloat16 *o = first ? a.out1 : a.out2;
+    const int cc = first ? c0 : c0 - a.co1, stride = first ? a.co1 : a.co2;
+    if (a.bias) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += __ldg(a.bias + c0 + j);
+    }
+    if (a.relu) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
+    }
+    if (first ? a.mask1 : a.mask2) {
+        const __nv_bfloat16 *mb0 = reinterpret_cast<const __nv_bfloat16 *>(&mask.q0);
+        const __nv_bfloat16 *mb1 = reinterpret_cast<const __nv_bfloat16 *>(&mask.q1);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (!(__bfloat162float(mb0[j]) > 0.0f)) v[j] = 0.0f;
+            if (!(__bfloat162float(mb1[j]) > 0.0f)) v[8 + j] = 0.0f;
+        }
+    }
+    uint4 w0, w1;
+    uint32_t *p0 = reinterpret_cast<uint32_t *>(&w0), *p1 = reinterpret_cast<uint32_t *>(&w1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        const __nv_bfloat162 h1 = __floats2bfloat162_rn(v[8 + 2 * j], v[8 + 2 * j + 1]);
+        p0[j] = *reinterpret_cast<const uint32_t *>(&h0);
+        p1[j] = *reinterpret_cast<const uint32_t *>(&h1);
+    }
+    uint4 *op = reinterpret_cast<uint4 *>(o + vox * stride + cc);
+    op[0] = w0;
+    op[1] = w1;
+}
+
 template <int N, bool YR>
 __global__ void __launch_bounds__(128, 1)
 conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mx2,
@@ -387,45 +444,289 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
         float v[16];
         tmem_ld16(trow + c0, v);
         if (!ok) continue;
-        const bool first = c0 < a.co1;
-        __nv_bfloat16 *o = first ? a.out1 : a.out2;
-        const __nv_bfloat16 *m = first ? a.mask1 : a.mask2;
-        const int cc = first ? c0 : c0 - a.co1, stride = first ? a.co1 : a.co2;
-        if (a.bias) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] += __ldg(a.bias + c0 + j);
-        }
-        if (a.relu) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
-        }
-        if (m) {
-            const uint4 *mp = reinterpret_cast<const uint4 *>(m + vox * stride + cc);
-            const uint4 q0 = __ldg(mp), q1 = __ldg(mp + 1);
-            const __nv_bfloat16 *mb0 = reinterpret_cast<const __nv_bfloat16 *>(&q0);
-            const __nv_bfloat16 *mb1 = reinterpret_cast<const __nv_bfloat16 *>(&q1);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (!(__bfloat162float(mb0[j]) > 0.0f)) v[j] = 0.0f;
-                if (!(__bfloat162float(mb1[j]) > 0.0f)) v[8 + j] = 0.0f;
-            }
-        }
-        uint4 w0, w1;
-        uint32_t *p0 = reinterpret_cast<uint32_t *>(&w0), *p1 = reinterpret_cast<uint32_t *>(&w1);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-            const __nv_bfloat162 h1 = __floats2bfloat162_rn(v[8 + 2 * j], v[8 + 2 * j + 1]);
-            p0[j] = *reinterpret_cast<const uint32_t *>(&h0);
-            p1[j] = *reinterpret_cast<const uint32_t *>(&h1);
-        }
-        uint4 *op = reinterpret_cast<uint4 *>(o + vox * stride + cc);
-        op[0] = w0;
-        op[1] = w1;
+        const Mask16 m = load_mask(a, vox, c0);
+        store16(a, vox, c0, v, m);
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 2) tmem_dealloc(tmem, N);
+}
+
+// ---------------------------------------------------------------------------
+// z-marching mode of the 3x3x3 convolution, for filters that fit in shared
+// memory (32 outputs from 32 or 64 channels, 64 outputs from 32).
+//
+// conv_fwd_kernel reads 9 boxes of each 32-channel chunk and all 27 filter
+// slices for every 128-voxel tile (138 KB of L2 reads for 32 -> 32 channels:
+// the L2's rate sets its time), in 54 instructions of N = 32 that the
+// reading of A from shared memory holds to a quarter of the tensor cores' rate.
+// Here a CTA keeps all filter slices and walks 8 x 16 voxel columns along z: each
+// input slice is fetched once (three boxes, one per dx) and multiplied by the
+// filters of the three dz at once, one 128 x 3N x 16 instruction per (dx, dy,
+// 16 channels): the accumulators of the outputs z - 1, z, z + 1 are neighbours
+// in a ring of tensor-memory columns, and the filter rows are stored in the order
+// dz = +1, 0, -1.  An output still sums its taps in conv_fwd_kernel's order
+// (dz, dx, chunk, dy), so the results are the same bits.
+//
+// An instruction takes 56 cycles at 3N = 96 (7 KB of operands from shared memory
+// at 128 B/clock; 48 at the tensor cores' rate) and 96 at 3N = 192; issuing, waiting
+// and committing cost the issuing thread about as long again per slice, so a
+// CTA holds two groups of warps that share the filters, each with its own
+// columns, load ring and half of the tensor memory, and one's waits pass under the
+// other's instructions.  Per group: four warps store finished slices, one issues
+// the loads, one the instructions.  Persistent, one CTA per SM: a group takes
+// items = (sample, z chunk, tile) in turn.
+//
+// GB300, 256^3: 32 -> 32 channels 1542 -> 662 us (1.4 PFLOP/s), 64 -> 32 2518 ->
+// 1314; 128^3: 32 -> 64 324 -> 181, 64 -> 64 489 -> 363.  One group per CTA: 1125 us for
+// 32 -> 32; with one thread of an undivided warp issuing (operands moved to
+// uniform registers for each instruction) 2386 us.
+// ---------------------------------------------------------------------------
+constexpr int kMGroups = 2;
+constexpr int kMBoxes = 6;                    // boxes (8 x 18 voxels, 32 channels) in a group's load ring
+constexpr int kMCols = 256;                   // tensor-memory columns of a group's accumulator ring
+
+struct MarchGroup {
+    uint64_t full[kMBoxes / 2];
+    uint64_t empty[kMBoxes / 2];
+    uint64_t accfull[kMCols / 32];
+    uint64_t accempty[kMCols / 32];
+    uint64_t done;
+};
+
+struct MarchCtrl {
+    MarchGroup g[kMGroups];
+    uint64_t wfull;
+    uint32_t tmem;
+};
+
+struct MarchArgs {
+    FwdArgs f;
+    int tx, ty;              // tiles along x and y
+    int zc, nzc;             // output slices per item, items along z
+    int parts;               // CTAs b, b + parts, ... compute outputs (b % parts) * N .. + N - 1
+    long long items;
+};
+
+struct MarchItem {
+    int x0, y0, z0, z1, n;   // outputs z0 .. z1 - 1 of the tile at (x0, y0)
+};
+
+__device__ __forceinline__ MarchItem march_item(const MarchArgs &a, long long i) {
+    MarchItem it;
+    it.x0 = static_cast<int>(i % a.tx) * kYBx;
+    i /= a.tx;
+    it.y0 = static_cast<int>(i % a.ty) * kYBy;
+    i /= a.ty;
+    it.z0 = static_cast<int>(i % a.nzc) * a.zc;
+    it.z1 = min(it.z0 + a.zc, a.f.nz);
+    it.n = static_cast<int>(i / a.nzc);
+    return it;
+}
+
+// One lane of a converged warp; the compiler then keeps the operands of the
+// instructions in uniform registers instead of selecting them lane by lane.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+template <int N, int NCH>                                  // outputs, 32-channel chunks of the input
+__global__ void __launch_bounds__(192 * kMGroups, 1)
+conv_march_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mx2,
+                  const __grid_constant__ CUtensorMap mw, const MarchArgs a) {
+    constexpr int R = kMCols / N;                          // accumulators in a group's ring
+    // a stage: all boxes of a slice (one chunk), or those of one dx (two chunks)
+    constexpr int DXS = NCH == 1 ? 3 : 1, S = kMBoxes / (DXS * NCH);
+    constexpr uint32_t stage = DXS * NCH * kYABytes;
+    constexpr uint32_t wblock = N * kRowBytes;             // filter rows of one tap and chunk
+    constexpr uint32_t wbytes = 27 * NCH * wblock;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *wsm = align1024(smem_raw);                    // [dx][chunk][dy][dz = +1, 0, -1][N] filter rows
+    uint8_t *rings = wsm + wbytes;
+    MarchCtrl *ctrl = reinterpret_cast<MarchCtrl *>(rings + kMGroups * S * stage);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    // warps 0 .. 4 G - 1: stores, four per group; then the groups' loading warps, then their multiplying warps
+    const int role = warp < 4 * kMGroups ? 0 : (warp < 5 * kMGroups ? 1 : 2);
+    const int grp = role == 0 ? warp / 4 : warp % kMGroups;
+    MarchGroup *c = ctrl->g + grp;
+    uint8_t *ring = rings + grp * S * stage;
+    const int n0 = blockIdx.x % a.parts * N;               // first output channel
+    const long long item0 = blockIdx.x / a.parts * kMGroups + grp;
+    const long long istep = static_cast<long long>(gridDim.x / a.parts) * kMGroups;
+    const int nz = a.f.nz;
+
+    if (threadIdx.x < kMGroups) {
+        MarchGroup *q = ctrl->g + threadIdx.x;
+        for (int s = 0; s < S; ++s) {
+            mbar_init(&q->full[s], 1);
+            mbar_init(&q->empty[s], 1);
+        }
+        for (int s = 0; s < R; ++s) {
+            mbar_init(&q->accfull[s], 1);
+            mbar_init(&q->accempty[s], 4);
+        }
+        mbar_init(&q->done, 1);
+        if (threadIdx.x == 0) mbar_init(&ctrl->wfull, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 6 * kMGroups - 1) tmem_alloc(&ctrl->tmem, kMGroups * kMCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = ctrl->tmem + grp * kMCols;
+
+    if (role == 1) {
+        if (grp == 0 && lane == 0) {
+            mbar_expect_tx(&ctrl->wfull, wbytes);
+            for (int b = 0; b < 27 * NCH; ++b) {           // b = ((dx * NCH + chunk) * 3 + dy) * 3 + j, dz = 1 - j
+                const int tap = (2 - b % 3) * 9 + (b / 3 % 3) * 3 + b / (9 * NCH);
+                tma_load3(wsm + b * wblock, &mw, &ctrl->wfull, b / 9 % NCH * 32, tap, n0);
+            }
+        }
+        __syncwarp();
+        int s = 0, used = 0;                               // stage, stages filled so far (up to S)
+        uint32_t ph = 0;
+        bool ok = true;
+        for (long long i = item0; ok && i < a.items; i += istep) {
+            const MarchItem it = march_item(a, i);
+            const int ze = min(it.z1, nz - 1);
+            for (int z = max(it.z0 - 1, 0); ok && z <= ze; ++z) {
+#pragma unroll
+                for (int g = 0; g < 3 / DXS; ++g) {
+                    if (used == S) ok = __all_sync(0xffffffffu, mbar_wait(&c->empty[s], ph ^ 1));
+                    if (!ok) break;
+                    if (elect_one()) {
+                        mbar_expect_tx(&c->full[s], stage);
+#pragma unroll
+                        for (int j = 0; j < DXS * NCH; ++j) {
+                            const int dx = g * DXS + j / NCH - 1, ch = j % NCH * 32;
+                            const bool second = ch >= a.f.c1;
+                            tma_load5(ring + s * stage + j * kYABytes, second ? &mx2 : &mx1, &c->full[s],
+                                      second ? ch - a.f.c1 : ch, it.x0 + dx, it.y0 - 1, z, it.n);
+                        }
+                    }
+                    __syncwarp();
+                    used = min(used + 1, S);
+                    if (++s == S) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(&g_unet_err, 1);
+        // every load has landed before the CTA may leave: the last use of stage j
+        mbar_wait(&ctrl->wfull, 0);
+        for (int j = 0; j < used; ++j) mbar_wait(&c->full[j], j < s ? ph : ph ^ 1);
+    } else if (role == 2) {
+        bool ok = __all_sync(0xffffffffu, mbar_wait(&ctrl->wfull, 0));
+        const uint64_t wdesc = sw64_desc(smem_u32(wsm)), adesc = sw64_desc(smem_u32(ring));
+        unsigned obase = 0;                                // outputs of earlier items
+        int s = 0;
+        uint32_t ph = 0;
+        for (long long i = item0; ok && i < a.items; i += istep) {
+            const MarchItem it = march_item(a, i);
+            const int ze = min(it.z1, nz - 1);
+            for (int z = max(it.z0 - 1, 0); ok && z <= ze; ++z) {
+                const int lo = max(z - 1, it.z0), hi = min(z + 1, it.z1 - 1), cnt = hi - lo + 1;
+                const unsigned olo = obase + lo - it.z0, blo = olo % R;
+                // this slice is the first input of output z + 1 (and of output 0): it starts in a free accumulator
+                for (int zo = max(z ? z + 1 : 0, lo); zo <= hi; ++zo) {
+                    const unsigned o = olo + zo - lo;
+                    if (o >= R && !mbar_wait(&c->accempty[o % R], (o / R - 1) & 1)) ok = false;
+                }
+                const bool whole = cnt == 3 && blo + 3 <= R;   // and z > 0: outputs z - 1, z go on, z + 1 starts
+                const int la = min(cnt, static_cast<int>(R - blo)), lb = cnt - la;
+                const uint64_t b0 = wdesc + static_cast<uint64_t>(lo - z + 1) * (wblock / 16);
+                const uint32_t d0 = tmem + blo * N;
+#pragma unroll
+                for (int g = 0; g < 3 / DXS; ++g) {
+                    if (!mbar_wait(&c->full[s], ph)) ok = false;
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint64_t a0 = adesc + static_cast<uint64_t>(s) * (stage / 16);
+#pragma unroll
+                        for (int q = 0; q < DXS * NCH * 6; ++q) {   // q = ((dx * NCH + chunk) * 3 + dy) * 2 + half
+                            const uint64_t ad = a0 + (q / 6) * (kYABytes / 16) + (q / 2 % 3) * (kYBx * kRowBytes / 16) +
+                                                (q % 2) * 2;
+                            const uint64_t bd = b0 + (g * DXS * NCH * 3 + q / 2) * (3 * wblock / 16) + (q % 2) * 2;
+                            if (g == 0 && q == 0) {
+                                if (whole) {
+                                    umma_bf16(d0, ad, bd, idesc_bf16(kTileM, 2 * N), 1);
+                                    umma_bf16(d0 + 2 * N, ad, bd + 2 * wblock / 16, idesc_bf16(kTileM, N), 0);
+                                } else {
+                                    for (int j = 0; j < cnt; ++j)
+                                        umma_bf16(tmem + (blo + j) % R * N, ad, bd + j * (wblock / 16),
+                                                  idesc_bf16(kTileM, N), z != max(lo + j - 1, 0));
+                                }
+                            } else if (whole) {
+                                umma_bf16(d0, ad, bd, idesc_bf16(kTileM, 3 * N), 1);
+                            } else {
+                                umma_bf16(d0, ad, bd, idesc_bf16(kTileM, N * la), 1);
+                                if (lb)                    // the ring's end lies between the outputs
+                                    umma_bf16(tmem, ad, bd + la * (wblock / 16), idesc_bf16(kTileM, N * lb), 1);
+                            }
+                        }
+                        umma_commit(&c->empty[s]);
+                        if (g == 3 / DXS - 1) {            // outputs that this slice is the last input of
+                            if (lo < z) umma_commit(&c->accfull[blo]);
+                            if (z == nz - 1 && hi == z) umma_commit(&c->accfull[(blo + z - lo) % R]);
+                        }
+                    }
+                    __syncwarp();
+                    if (++s == S) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+            obase += it.z1 - it.z0;
+        }
+        if (!ok && lane == 0) atomicOr(&g_unet_err, 2);
+        if (elect_one()) umma_commit(&c->done);
+    } else {
+        const int r = (warp & 3) * 32 + lane;
+        const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        unsigned o = 0;
+        bool ok = true;
+        for (long long i = item0; ok && i < a.items; i += istep) {
+            const MarchItem it = march_item(a, i);
+            long long vox = ((static_cast<long long>(it.n) * nz + it.z0) * a.f.ny + it.y0 + r / kYBx) * a.f.nx + it.x0 +
+                            r % kYBx;
+            for (int z = it.z0; z < it.z1; ++z, ++o, vox += static_cast<long long>(a.f.ny) * a.f.nx) {
+                Mask16 m[N / 16];
+#pragma unroll
+                for (int j = 0; j < N / 16; ++j) m[j] = load_mask(a.f, vox, n0 + 16 * j);
+                ok = __all_sync(0xffffffffu, mbar_wait(&c->accfull[o % R], (o / R) & 1));
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int j = 0; j < N / 16; ++j) {
+                    float v[16];
+                    tmem_ld16(trow + o % R * N + 16 * j, v);
+                    if (j == N / 16 - 1) {                 // the accumulator is in registers: free it
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&c->accempty[o % R]))
+                                         : "memory");
+                    }
+                    store16(a.f, vox, n0 + 16 * j, v, m[j]);
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(&g_unet_err, 4);
+    }
+    __syncwarp();
+    if (!mbar_wait(&c->done, 0)) atomicOr(&g_unet_err, 4);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 6 * kMGroups - 1) tmem_dealloc(ctrl->tmem, kMGroups * kMCols);
 }
 
 struct WgradArgs {
@@ -619,6 +920,44 @@ int launch_fwd(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &
     return CT_OK;
 }
 
+template <int N, int NCH>
+constexpr size_t march_smem() {
+    return 1024 + 27 * NCH * N * kRowBytes + kMGroups * kMBoxes * kYABytes + sizeof(MarchCtrl);
+}
+
+// Slices per item: the groups of the persistent CTAs share ceil(items / groups) items each, and an item of zc outputs
+// reads zc + 2 slices; the zc with the fewest slices read by the busiest group, the longer one of equals.
+template <int N, int NCH>
+int launch_march(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &mw, const FwdArgs &f, int nb,
+                 cudaStream_t st) {
+    MarchArgs a{};
+    a.f = f;
+    a.tx = f.nx / kYBx;
+    a.ty = f.ny / kYBy;
+    a.parts = (f.co1 + f.co2) / N;
+    const long long cols = (long long)nb * a.tx * a.ty, groups = (long long)kMGroups * std::max(1, sm_count() / a.parts);
+    long long best = -1;
+    for (int chunks = 1; chunks <= f.nz; ++chunks) {
+        const int zc = (f.nz + chunks - 1) / chunks;
+        const long long items = cols * ((f.nz + zc - 1) / zc), cost = (items + groups - 1) / groups * (zc + 2);
+        if (best >= 0 && cost >= best) continue;
+        best = cost;
+        a.zc = zc;
+        a.items = items;
+    }
+    a.nzc = (f.nz + a.zc - 1) / a.zc;
+    constexpr size_t smem = march_smem<N, NCH>();
+    static bool attr = false;
+    if (!attr) {
+        CT_CUDA(cudaFuncSetAttribute(conv_march_kernel<N, NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "conv_march smem");
+        attr = true;
+    }
+    conv_march_kernel<N, NCH><<<(unsigned)((std::min(a.items, groups) + kMGroups - 1) / kMGroups * a.parts), 192 * kMGroups, smem, st>>>(m1, m2, mw, a);
+    CT_LAUNCH_CHECK("conv_march_kernel");
+    return CT_OK;
+}
+
 template <int N>
 int launch_wgrad(const CUtensorMap &mm, const CUtensorMap &m0, const CUtensorMap &mp, const CUtensorMap &md,
                  const WgradArgs &a, dim3 grid, cudaStream_t st) {
@@ -677,6 +1016,11 @@ int ct_unet_conv3d(const void *x1, int c1, const void *x2, int c2, int nb, int n
                "conv3d: pointers must be 16-byte aligned");
     const long long tiles = (long long)nb * (nz / bz) * (ny / by) * (nx / bx);
     CT_REQUIRE(tiles < (1ll << 31), "conv3d: too many tiles");
+    // Outputs per CTA of the z-marching kernel where its filters fit in shared memory (64 outputs of 64 channels in
+    // two halves), else 0.  It starts by loading the filters (about 8 us for 110 KB) and walks several slices per CTA:
+    // a volume that conv_fwd_kernel covers in about one wave of its four CTAs per SM is left to that.  32^3 (256 tiles):
+    // 12.5 us there, 16.0 here for 64 -> 32 channels, 8.8 / 8.6 for 32 -> 32; 48^3 (864 tiles): 25.1 / 21.9, 16.3 / 11.9.
+    const int march = !yr || n > 64 || tiles <= 4LL * sm_count() ? 0 : (c1 + c2 == 32 ? n : (c1 + c2 == 64 ? 32 : 0));
     CUtensorMap m1, m2, mw;
     int s;
     const int box_y = yr ? by + 2 : by;
@@ -686,7 +1030,7 @@ int ct_unet_conv3d(const void *x1, int c1, const void *x2, int c2, int nb, int n
         const int cin = c1 + c2;
         const uint64_t dims[3] = {(uint64_t)cin, (uint64_t)ntaps, (uint64_t)n};
         const uint64_t st[2] = {(uint64_t)cin * 2, (uint64_t)ntaps * cin * 2};
-        const uint32_t box[3] = {32, 1, (uint32_t)n};
+        const uint32_t box[3] = {32, 1, (uint32_t)(march ? march : n)};
         if ((s = make_map(&mw, w, 3, dims, st, box))) return s;
     }
     FwdArgs a{};
@@ -709,6 +1053,10 @@ int ct_unet_conv3d(const void *x1, int c1, const void *x2, int c2, int nb, int n
     a.mask1 = static_cast<const __nv_bfloat16 *>(mask1);
     a.mask2 = static_cast<const __nv_bfloat16 *>(mask2);
     cudaStream_t st = as_stream(stream);
+    if (march) {
+        if (c1 + c2 == 64) return launch_march<32, 2>(m1, m2, mw, a, nb, st);
+        return march == 32 ? launch_march<32, 1>(m1, m2, mw, a, nb, st) : launch_march<64, 1>(m1, m2, mw, a, nb, st);
+    }
     if (yr) {
         switch (n) {
             case 32: return launch_fwd<32, true>(m1, m2, mw, a, (int)tiles, st);

@@ -265,3 +265,46 @@ def test_shift_copies_groups_and_remainders(c, nb, nz, ny, nx, off):
                     want[..., :-1] = t[..., 1:]
                 ref[:, off:off + c] = want
             assert torch.equal(o, ref), (k, skip)
+
+
+# z-marching convolution: one slice, fewer slices than accumulators, chunks along z with several items per CTA, two
+# inputs, a split output with masks.  Products of bf16 numbers are exact in FP32, so only the order of the sums
+# differs from torch's FP32 result: 27 cin terms of size ~1 err by at most 27 cin 2^-24 of their absolute sum, far
+# below the bf16 step; outputs equal but for roundings at a tie (at least 99 in 100, 2e-3 of the norm).
+@pytest.mark.gpu
+@pytest.mark.parametrize("c1,c2,cout,nb,nz,ny,nx,split,masked", [
+    (32, 0, 32, 5, 1, 128, 128, None, False), (32, 0, 32, 3, 2, 128, 128, None, True),
+    (32, 32, 32, 2, 3, 128, 128, None, False), (32, 0, 64, 2, 5, 96, 128, 32, True), (32, 0, 64, 2, 70, 32, 64, 48, True),
+    (32, 32, 32, 2, 45, 64, 64, None, True), (32, 0, 32, 3, 33, 48, 72, 16, False), (64, 0, 64, 1, 29, 48, 64, 48, True)])
+def test_conv3d_marching_along_z(c1, c2, cout, nb, nz, ny, nx, split, masked):
+    import torch
+    import torch.nn.functional as F
+    from ctgb import unet
+    g = torch.Generator(device="cuda").manual_seed(c1 + c2 + cout + nz)
+    bf = torch.bfloat16
+
+    def rnd(*shape):
+        return torch.randn(shape, device="cuda", generator=g)
+
+    x1 = rnd(nb, nz, ny, nx, c1).to(bf)
+    x2 = rnd(nb, nz, ny, nx, c2).to(bf) if c2 else None
+    w = (rnd(cout, 27, c1 + c2) * 0.05).to(bf)
+    bias = rnd(cout)
+    co = [cout] if split is None else [split, cout - split]
+    masks = tuple(rnd(nb, nz, ny, nx, k).to(bf) for k in co) if masked else ()
+    masks = masks + (None,) * (2 - len(masks))
+    out = unet.conv3d(x1, w, bias, relu=not masked, x2=x2, split=split, masks=masks)
+    assert unet.status() == 0
+    x = x1 if x2 is None else torch.cat((x1, x2), -1)
+    ref = F.conv3d(x.float().permute(0, 4, 1, 2, 3), w.float().permute(0, 2, 1).reshape(cout, c1 + c2, 3, 3, 3), bias,
+                   padding=1).permute(0, 2, 3, 4, 1)
+    ref = ref if masked else ref.relu()
+    outs, at = ((out,) if split is None else out), 0
+    for k, o in enumerate(outs):
+        r = ref[..., at:at + co[k]]
+        at += co[k]
+        if masked:
+            r = r * (masks[k].float() > 0)
+        r = r.to(bf).float()
+        err = float((o.float() - r).norm() / r.norm())
+        assert err <= 2e-3 and float((o.float() == r).float().mean()) >= 0.99, err
