@@ -24,9 +24,9 @@
 //   the box.  Split-K over voxel ranges; partial sums are added to an FP32
 //   gradient with atomics.
 //
-// A warp-specialised pipeline per CTA: thread 0 issues TMA loads into a
-// 4-stage ring, thread 32 issues the MMAs, and after the last MMA all four
-// warps read the accumulator from TMEM (tcgen05.ld) for the epilogue.  Every
+// A warp-specialised pipeline per CTA: warp 0 issues TMA loads into a
+// 3- or 4-stage ring, warp 1 the MMAs (one elected lane of a converged warp each),
+// and after the last MMA all four warps read the accumulator from TMEM (tcgen05.ld) for the epilogue.  Every
 // mbarrier wait is bounded by a 2 s timer; a timeout sets a device error flag
 // (read by ct_unet_status), drains the loads in flight and frees TMEM.
 #include <cuda.h>
@@ -241,36 +241,52 @@ __device__ void drain_loads(Ctrl *c, int issued) {
     }
 }
 
-// The MMA side of one CTA over an S-stage ring of (A_BYTES of A, NG * N rows
-// of B) stages with ROWB-byte rows (64: 64-byte swizzle, 128: 128-byte
-// swizzle): per K step, NG groups of ROWB / 32 instructions of 128 x N x 16,
-// group g reading A from byte offset g * A_STEP and the g-th B tile.
+// One lane of a converged warp; the compiler then keeps the operands of the
+// instructions in uniform registers instead of selecting them lane by lane.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// The MMA side of one CTA, called by a whole warp, over an S-stage ring of
+// (A_BYTES of A, NG * N rows of B) stages with ROWB-byte rows (64: 64-byte
+// swizzle, 128: 128-byte swizzle): per K step, NG groups of ROWB / 32
+// instructions of 128 x N x 16, group g reading A from byte offset g * A_STEP
+// and the g-th B tile.
 template <int N, int S, uint32_t A_BYTES, int NG, uint32_t A_STEP, int ROWB = kRowBytes>
 __device__ __forceinline__ void mma_loop(Ctrl *c, uint8_t *ring, uint32_t tmem, int ksteps) {
     constexpr uint32_t stage = A_BYTES + NG * N * ROWB;
     constexpr uint32_t idesc = idesc_bf16(kTileM, N);
     constexpr int KK = ROWB / 32;
+    const uint32_t ra = smem_u32(ring);
+    const uint64_t ad0 = ROWB == 128 ? sw128_desc(ra) : sw64_desc(ra);
+    const uint64_t bd0 = ROWB == 128 ? sw128_desc(ra + A_BYTES) : sw64_desc(ra + A_BYTES);
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
     for (int k = 0; k < ksteps; ++k) {
-        const int s = k % S;
-        if (aborted(c)) break;
-        if (!mbar_wait(&c->full[s], static_cast<uint32_t>((k / S) & 1))) {
-            fail(c, 2);
-            break;
-        }
+        ok = __all_sync(0xffffffffu, mbar_wait(&c->full[s], ph));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t sa = smem_u32(ring + s * stage), sb = sa + A_BYTES;
+        if (elect_one()) {
+            const uint64_t so = static_cast<uint64_t>(s) * (stage / 16);
 #pragma unroll
-        for (int g = 0; g < NG; ++g)
+            for (int g = 0; g < NG; ++g)
 #pragma unroll
-            for (int kk = 0; kk < KK; ++kk) {
-                const uint32_t ao = sa + g * A_STEP + kk * 32, bo = sb + g * N * ROWB + kk * 32;
-                const uint64_t ad = ROWB == 128 ? sw128_desc(ao) : sw64_desc(ao);
-                const uint64_t bd = ROWB == 128 ? sw128_desc(bo) : sw64_desc(bo);
-                umma_bf16(tmem, ad, bd, idesc, k | g | kk);
-            }
-        umma_commit(&c->empty[s]);
+                for (int kk = 0; kk < KK; ++kk)
+                    umma_bf16(tmem, ad0 + so + (g * A_STEP + kk * 32) / 16, bd0 + so + (g * N * ROWB + kk * 32) / 16,
+                              idesc, k | g | kk);
+            umma_commit(&c->empty[s]);
+        }
+        __syncwarp();
+        if (++s == S) {
+            s = 0;
+            ph ^= 1;
+        }
     }
-    umma_commit(&c->done);
+    if (!ok) fail(c, 2);
+    if (elect_one()) umma_commit(&c->done);
 }
 
 // y-halo mode of the forward kernel: 8 x 16 voxel tiles of one slice; one box of
@@ -362,7 +378,7 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
     extern __shared__ uint8_t smem_raw[];
     uint8_t *ring = align1024(smem_raw);
     Ctrl *c = reinterpret_cast<Ctrl *>(ring + S * stage);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     int t = blockIdx.x;
     const int tx = a.nx / a.bx, ty = a.ny / a.by, tz = a.nz / a.bz;
@@ -387,18 +403,13 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem = c->tmem;
 
-    if (threadIdx.x == 0) {
-        const int nch = (a.c1 + a.c2) / 32;
-        int issued = 0;
-        for (int k = 0; k < a.ksteps; ++k) {
-            const int s = k % S;
-            if (aborted(c)) break;
-            if (k >= S && !mbar_wait(&c->empty[s], static_cast<uint32_t>((k / S - 1) & 1))) {
-                fail(c, 1);
-                break;
-            }
-            // K order: (tap or (dz, dx) group) major, 32-channel chunks inner
-            const int grp = k / nch, ch = (k % nch) * 32;
+    if (warp == 0) {
+        // K order: (tap or (dz, dx) group) major, 32-channel chunks inner
+        const int cin = a.c1 + a.c2, ngrp = YR ? 9 : a.ntaps;
+        int s = 0, issued = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int grp = 0; ok && grp < ngrp; ++grp) {
             int dz, dy, dx;
             if (YR) {
                 dz = grp / 3 - 1;
@@ -407,24 +418,36 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
             } else {
                 tap_offsets(grp, a.ntaps, dz, dy, dx);
             }
-            uint8_t *sa = ring + s * stage;
-            mbar_expect_tx(&c->full[s], stage);
-            if (ch < a.c1)
-                tma_load5(sa, &mx1, &c->full[s], ch, x0 + dx, y0 + dy, z0 + dz, n0);
-            else
-                tma_load5(sa, &mx2, &c->full[s], ch - a.c1, x0 + dx, y0 + dy, z0 + dz, n0);
-            if (YR) {
+            for (int ch = 0; ch < cin; ch += 32) {
+                if (issued >= S) ok = __all_sync(0xffffffffu, mbar_wait(&c->empty[s], ph ^ 1));
+                if (!ok) break;
+                if (elect_one()) {
+                    uint8_t *sa = ring + s * stage;
+                    mbar_expect_tx(&c->full[s], stage);
+                    if (ch < a.c1)
+                        tma_load5(sa, &mx1, &c->full[s], ch, x0 + dx, y0 + dy, z0 + dz, n0);
+                    else
+                        tma_load5(sa, &mx2, &c->full[s], ch - a.c1, x0 + dx, y0 + dy, z0 + dz, n0);
+                    if (YR) {
 #pragma unroll
-                for (int g = 0; g < 3; ++g)                 // dy = g - 1
-                    tma_load3(sa + a_bytes + g * N * kRowBytes, &mw, &c->full[s], ch, (dz + 1) * 9 + g * 3 + (dx + 1),
-                              0);
-            } else {
-                tma_load3(sa + a_bytes, &mw, &c->full[s], ch, grp, 0);
+                        for (int g = 0; g < 3; ++g)         // dy = g - 1
+                            tma_load3(sa + a_bytes + g * N * kRowBytes, &mw, &c->full[s], ch,
+                                      (dz + 1) * 9 + g * 3 + (dx + 1), 0);
+                    } else {
+                        tma_load3(sa + a_bytes, &mw, &c->full[s], ch, grp, 0);
+                    }
+                }
+                __syncwarp();
+                ++issued;
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
-            ++issued;
         }
+        if (!ok) fail(c, 1);
         if (aborted(c)) drain_loads<S>(c, issued);
-    } else if (threadIdx.x == 32) {
+    } else if (warp == 1) {
         mma_loop<N, S, a_bytes, ng, kYBx * kRowBytes>(c, ring, tmem, a.ksteps);
     }
     __syncwarp();
@@ -522,14 +545,6 @@ __device__ __forceinline__ MarchItem march_item(const MarchArgs &a, long long i)
     it.z1 = min(it.z0 + a.zc, a.f.nz);
     it.n = static_cast<int>(i / a.nzc);
     return it;
-}
-
-// One lane of a converged warp; the compiler then keeps the operands of the
-// instructions in uniform registers instead of selecting them lane by lane.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
 }
 
 template <int N, int NCH>                                  // outputs, 32-channel chunks of the input
@@ -749,7 +764,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap mxm, const __grid_constant
     extern __shared__ uint8_t smem_raw[];
     uint8_t *ring = align1024(smem_raw);
     Ctrl *c = reinterpret_cast<Ctrl *>(ring + kWStages * stage);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     const int tgroup = blockIdx.x / a.cblocks, cb = blockIdx.x % a.cblocks;
     const int tap0 = tgroup * a.taps_per_tile, ci0 = cb * a.rows_per_tap;
@@ -771,34 +786,46 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap mxm, const __grid_constant
     tc_fence_after();
     const uint32_t tmem = c->tmem;
 
-    if (threadIdx.x == 0) {
-        const int pchunks = a.pchunks;
-        int issued = 0;
-        for (int k = 0; k < ksteps; ++k) {
-            const int s = k % kWStages;
-            if (aborted(c)) break;
-            if (k >= kWStages && !mbar_wait(&c->empty[s], static_cast<uint32_t>((k / kWStages - 1) & 1))) {
-                fail(c, 1);
-                break;
+    if (warp == 0) {
+        // slice k0: voxels p .. p + 63 of the y*x plane z of sample n
+        int p = static_cast<int>(k0 % a.pchunks) * kWK;
+        int z = static_cast<int>(k0 / a.pchunks % a.nz), n = static_cast<int>(k0 / a.pchunks / a.nz);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        int k = 0;
+        for (; k < ksteps; ++k) {
+            if (k >= kWStages) ok = __all_sync(0xffffffffu, mbar_wait(&c->empty[s], ph ^ 1));
+            if (!ok) break;
+            if (elect_one()) {
+                uint8_t *sa = ring + s * stage;
+                mbar_expect_tx(&c->full[s], stage);
+                for (int j = 0; j < a.taps_per_tile; ++j) {
+                    const int tap = min(tap0 + j, a.ntaps - 1);
+                    int dz, dy, dx;
+                    tap_offsets(tap, a.ntaps, dz, dy, dx);
+                    const CUtensorMap *m = dx < 0 ? &mxm : (dx > 0 ? &mxp : &mx0);
+                    tma_load4(sa + j * a.rows_per_tap * kWRowBytes, m, &c->full[s], p + dy * a.nx, z + dz, ci0, n);
+                }
+                tma_load4(sa + a_bytes, &mdy, &c->full[s], p, z, 0, n);
             }
-            long long q = k0 + k;
-            const int p = static_cast<int>(q % pchunks) * kWK;
-            q /= pchunks;
-            const int z = static_cast<int>(q % a.nz), n = static_cast<int>(q / a.nz);
-            uint8_t *sa = ring + s * stage;
-            mbar_expect_tx(&c->full[s], stage);
-            for (int j = 0; j < a.taps_per_tile; ++j) {
-                const int tap = min(tap0 + j, a.ntaps - 1);
-                int dz, dy, dx;
-                tap_offsets(tap, a.ntaps, dz, dy, dx);
-                const CUtensorMap *m = dx < 0 ? &mxm : (dx > 0 ? &mxp : &mx0);
-                tma_load4(sa + j * a.rows_per_tap * kWRowBytes, m, &c->full[s], p + dy * a.nx, z + dz, ci0, n);
+            __syncwarp();
+            if (++s == kWStages) {
+                s = 0;
+                ph ^= 1;
             }
-            tma_load4(sa + a_bytes, &mdy, &c->full[s], p, z, 0, n);
-            ++issued;
+            p += kWK;
+            if (p >= a.pchunks * kWK) {
+                p = 0;
+                if (++z == a.nz) {
+                    z = 0;
+                    ++n;
+                }
+            }
         }
-        if (aborted(c)) drain_loads<kWStages>(c, issued);
-    } else if (threadIdx.x == 32) {
+        if (!ok) fail(c, 1);
+        if (aborted(c)) drain_loads<kWStages>(c, k);
+    } else if (warp == 1) {
         mma_loop<N, kWStages, a_bytes, 1, 0, kWRowBytes>(c, ring, tmem, ksteps);
     }
     __syncwarp();
