@@ -16,7 +16,8 @@
 //   activation, rounds to bf16 and splits the channels over one or two outputs.
 //   conv_march_kernel is the same convolution for few channels: it keeps the
 //   filters in shared memory and reads each input slice once.
-// * conv_wgrad_kernel (weight gradient): rows = (tap, input channel), columns
+// * conv_wgrad_cl_kernel (weight gradient): the channels-last tensors as they are,
+//   see below.  conv_wgrad_kernel, for volumes that its tiles do not fit: rows = (tap, input channel), columns
 //   = output channels, K = voxels in 64-voxel slices (128-byte rows, 128-byte
 //   swizzle).  Activations and output gradients are read channel-major
 //   [n][c][z][y*x]; x offsets come from three x-shifted copies (so the
@@ -154,12 +155,27 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
     return d;
 }
 
+// Descriptor of an MN-major operand in the 64-byte swizzle layout: atoms of 32
+// MN elements (64 bytes) x 8 k rows; mn_step bytes from one atom to the next
+// along MN (leading byte offset), 512 along k (stride byte offset).
+__device__ __forceinline__ uint64_t sw64_mn_desc(uint32_t saddr, uint32_t mn_step) {
+    uint64_t d = static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
+    d |= static_cast<uint64_t>(mn_step >> 4) << 16;
+    d |= static_cast<uint64_t>(512 >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(4) << 61;
+    return d;
+}
+
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
 // K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
            (static_cast<uint32_t>(m >> 4) << 24);
 }
+
+// The same with both operands MN-major.
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n) { return idesc_bf16(m, n) | (1u << 15) | (1u << 16); }
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int acc) {
     asm volatile(
@@ -854,6 +870,239 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap mxm, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------
+// Weight gradient straight from channels-last tensors, 32 input x 32 output
+// channels per CTA.
+//
+// conv_wgrad_kernel wants its K dimension (voxels) contiguous, so the tensors
+// are first copied channel-major, X three times; each of its boxes then
+// gathers 128-byte rows that lie a whole volume apart, and 4 taps x 32 channels against
+// 32 outputs need 7 passes over the volume.  Here the 8 x 16 voxel tiles of the
+// channels-last tensors are the operands as they are (MN-major: 32 channels of
+// a voxel contiguous, voxels along K).  M = 3 boxes of X, one per dx, of 32 channels each (a fourth
+// quarter of M reads what follows them and is dropped); N = the three
+// dy: three atoms that start one tile row (8 voxels, 512 bytes) apart in one
+// box of dY with a halo row on either side.  A CTA walks its columns along z and multiplies X of
+// slice z by dY of z + 1, z, z - 1 into three accumulators (dz = -1, 0, 1): each
+// slice of either tensor is fetched once per column, all 27 taps from 34 KB per 128 voxels
+// instead of 280.  X is zero outside the volume, so every tap's sum over
+// the tiles of X is complete.
+//
+// Partial sums are added to dw after every `flush` tiles, so an FP32 sum is as long
+// as with conv_wgrad_kernel's kper, and its error is the same (128^3: 1.88e-6
+// of the norm for both, 32^3: 2.1e-7 against 7.8e-7).
+//
+// GB300, with the copies that conv_wgrad_kernel needs (before / after): 128^3,
+// 32 x 32 channels 948 / 125 us, 64 x 32 1805 / 232, 64 x 64 2291 / 444; 64^3, 64 x 64 138 / 81,
+// 128 x 128 328 / 274, 256 x 128 595 / 566; 32^3, 256 x 256 164 / 157.  No channel count was found
+// at which the copies pay, so conv_wgrad_kernel only serves volumes whose y is
+// not a multiple of the tile's 16.  What remains is the issuing thread's
+// waits and commits (about as long as the 24 instructions of 56 cycles per
+// tile) and, at many channels, 3 of 4 useful rows.
+// ---------------------------------------------------------------------------
+constexpr int kClStages = 6;
+constexpr uint32_t kClBox = kYBx * kYBy * kRowBytes;       // 128 voxels x 32 channels
+
+struct ClCtrl {
+    uint64_t full[kClStages];
+    uint64_t empty[kClStages];
+    uint64_t accfull;
+    uint64_t accempty[3];
+    uint64_t done;
+    uint32_t tmem;
+};
+
+struct ClArgs {
+    int c1, cin, cout;
+    int nz, tx, ty;
+    int zc, nzc;             // slices per item, items along z
+    int flush;               // tiles per partial sum
+    long long items;
+    float *dw;               // [cout][taps][cin], FP32, accumulated
+};
+
+template <int TAPS>
+__host__ __device__ constexpr uint32_t cl_stage() {
+    return TAPS == 27 ? 3 * kClBox + kYABytes : 2 * kClBox;
+}
+
+template <int TAPS>
+constexpr size_t cl_smem() {
+    return 1024 + kClStages * cl_stage<TAPS>() + sizeof(ClCtrl);
+}
+
+// grid (CTAs, 32-channel chunks of X, 32-channel chunks of dY)
+template <int TAPS>
+__global__ void __launch_bounds__(192, 1)
+conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mx2,
+                     const __grid_constant__ CUtensorMap mdy, const ClArgs a) {
+    constexpr int S = kClStages, NZ = TAPS == 27 ? 3 : 1, NX = NZ;   // dz blocks, boxes of X
+    constexpr int N = 32 * NZ, H = TAPS == 27 ? 1 : 0;               // columns of a block, halo of dY
+    constexpr uint32_t stage = cl_stage<TAPS>(), xbytes = NX * kClBox, dbytes = stage - xbytes;
+    constexpr uint32_t cols = TAPS == 27 ? 512 : 32;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *ring = align1024(smem_raw);
+    ClCtrl *c = reinterpret_cast<ClCtrl *>(ring + S * stage);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int ci0 = blockIdx.y * 32, co0 = blockIdx.z * 32;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(&c->full[s], 1);
+            mbar_init(&c->empty[s], 1);
+        }
+        mbar_init(&c->accfull, 1);
+        for (int j = 0; j < 3; ++j) mbar_init(&c->accempty[j], NX);
+        mbar_init(&c->done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 5) tmem_alloc(&c->tmem, cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = c->tmem;
+
+    // item i: slices z0 .. z1 - 1 of a tile column
+    auto item = [&](long long i, int &x0, int &y0, int &z0, int &z1, int &n) {
+        x0 = static_cast<int>(i % a.tx) * kYBx;
+        i /= a.tx;
+        y0 = static_cast<int>(i % a.ty) * kYBy;
+        i /= a.ty;
+        z0 = static_cast<int>(i % a.nzc) * a.zc;
+        z1 = min(z0 + a.zc, a.nz);
+        n = static_cast<int>(i / a.nzc);
+    };
+    int x0, y0, z0, z1, n;
+
+    if (warp == 4) {
+        int s = 0, used = 0;                               // stage, stages filled so far (up to S)
+        uint32_t ph = 0;
+        bool ok = true;
+        for (long long i = blockIdx.x; ok && i < a.items; i += gridDim.x) {
+            item(i, x0, y0, z0, z1, n);
+            for (int z = z0 - H; z < z1 + H; ++z) {        // stage: dY of slice z, X of it where it is the item's
+                if (used == S) ok = __all_sync(0xffffffffu, mbar_wait(&c->empty[s], ph ^ 1));
+                if (!ok) break;
+                if (elect_one()) {
+                    const bool x = z >= z0 && z < z1;
+                    uint8_t *sa = ring + s * stage;
+                    mbar_expect_tx(&c->full[s], dbytes + (x ? xbytes : 0));
+                    tma_load5(sa + xbytes, &mdy, &c->full[s], co0, x0, y0 - H, z, n);
+                    if (x) {
+#pragma unroll
+                        for (int j = 0; j < NX; ++j)
+                            tma_load5(sa + j * kClBox, ci0 < a.c1 ? &mx1 : &mx2, &c->full[s],
+                                      ci0 < a.c1 ? ci0 : ci0 - a.c1, x0 + j - H, y0, z, n);
+                    }
+                }
+                __syncwarp();
+                used = min(used + 1, S);
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(&g_unet_err, 1);
+        // every load has landed before the CTA may leave: the last use of stage j
+        for (int j = 0; j < used; ++j) mbar_wait(&c->full[j], j < s ? ph : ph ^ 1);
+    } else if (warp == 5) {
+        const uint64_t xd = sw64_mn_desc(smem_u32(ring), TAPS == 27 ? kClBox : 512);
+        const uint64_t yd = sw64_mn_desc(smem_u32(ring) + xbytes, 512);
+        int s = 0, p1 = 0, p2 = 0;                         // stages of this slice and the two before it
+        int tiles = 0;                                     // since the last partial sum was handed over
+        uint32_t ph = 0, sums = 0;
+        bool ok = true;
+        for (long long i = blockIdx.x; ok && i < a.items; i += gridDim.x) {
+            item(i, x0, y0, z0, z1, n);
+            for (int z = z0 - H; z < z1 + H; ++z) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&c->full[s], ph));
+                if (!ok) break;
+                const int zx = z - H;                      // the slice of X that has all its dY now
+                if (zx >= z0) {
+                    tc_fence_after();
+#pragma unroll
+                    for (int j = 0; j < NZ; ++j) {         // dz = j - 1: dY of slice zx - dz
+                        if (tiles == 0 && sums) ok = __all_sync(0xffffffffu, mbar_wait(&c->accempty[j], (sums - 1) & 1));
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {
+                            const int sx = H ? p1 : s, sy = H ? (j == 0 ? s : (j == 1 ? p1 : p2)) : s;
+                            const uint64_t ad = xd + static_cast<uint64_t>(sx) * (stage / 16);
+                            const uint64_t bd = yd + static_cast<uint64_t>(sy) * (stage / 16);
+#pragma unroll
+                            for (int kk = 0; kk < kYBx * kYBy / 16; ++kk)
+                                umma_bf16(tmem + j * N, ad + kk * 64, bd + kk * 64, idesc_bf16_mn(kTileM, N),
+                                          tiles | kk);
+                        }
+                        __syncwarp();
+                    }
+                    if (!ok) break;
+                    const bool last = zx == z1 - 1, full = ++tiles == a.flush || (last && i + gridDim.x >= a.items);
+                    if (elect_one()) {
+                        if (H) {
+                            umma_commit(&c->empty[p2]);
+                            if (last) umma_commit(&c->empty[p1]);
+                        }
+                        if (!H || last) umma_commit(&c->empty[s]);
+                        if (full) umma_commit(&c->accfull);
+                    }
+                    __syncwarp();
+                    if (full) {
+                        tiles = 0;
+                        ++sums;
+                    }
+                }
+                p2 = p1;
+                p1 = s;
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicOr(&g_unet_err, 2);
+        if (elect_one()) umma_commit(&c->done);
+    } else if (warp < NX) {                                // warp = dx + 1, lane = input channel
+        long long tiles = 0;
+        for (long long i = blockIdx.x; i < a.items; i += gridDim.x) {
+            item(i, x0, y0, z0, z1, n);
+            tiles += z1 - z0;
+        }
+        const long long sums = (tiles + a.flush - 1) / a.flush, cstride = static_cast<long long>(TAPS) * a.cin;
+        const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+        bool ok = true;
+        for (long long q = 0; q < sums; ++q) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&c->accfull, static_cast<uint32_t>(q & 1)));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int j = 0; j < NZ; ++j) {
+#pragma unroll 1
+                for (int b = 0; b < 2 * NZ; ++b) {         // 16 output channels of dy = 1 - b / 2
+                    float v[16];
+                    tmem_ld16(trow + j * N + b * 16, v);
+                    const int tap = TAPS == 27 ? j * 9 + (2 - b / 2) * 3 + warp : 0;
+                    float *dst = a.dw + (co0 + b % 2 * 16) * cstride + static_cast<long long>(tap) * a.cin + ci0 + lane;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) atomicAdd(dst + e * cstride, v[e]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&c->accempty[j])) : "memory");
+            }
+        }
+        if (!ok && lane == 0) atomicOr(&g_unet_err, 4);
+    }
+    __syncwarp();
+    if (!mbar_wait(&c->done, 0)) atomicOr(&g_unet_err, 4);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 5) tmem_dealloc(tmem, cols);
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 
@@ -1000,6 +1249,21 @@ int launch_wgrad(const CUtensorMap &mm, const CUtensorMap &m0, const CUtensorMap
     return CT_OK;
 }
 
+template <int TAPS>
+int launch_wgrad_cl(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &md, const ClArgs &a, int chunks_x,
+                    int chunks_y, unsigned ctas, cudaStream_t st) {
+    constexpr size_t smem = cl_smem<TAPS>();
+    static bool attr = false;
+    if (!attr) {
+        CT_CUDA(cudaFuncSetAttribute(conv_wgrad_cl_kernel<TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "conv_wgrad_cl smem");
+        attr = true;
+    }
+    conv_wgrad_cl_kernel<TAPS><<<dim3(ctas, chunks_x, chunks_y), 192, smem, st>>>(m1, m2, md, a);
+    CT_LAUNCH_CHECK("conv_wgrad_cl_kernel");
+    return CT_OK;
+}
+
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 bool valid_n(int n) { return n == 32 || n == 64 || n == 128 || n == 256; }
@@ -1143,6 +1407,53 @@ int ct_unet_conv3d_wgrad(const void *xm, const void *x0, const void *xp, int cin
         case 128: return launch_wgrad<128>(mm, m0, mp, md, a, grid, st);
         default: return launch_wgrad<256>(mm, m0, mp, md, a, grid, st);
     }
+}
+
+int ct_unet_conv3d_wgrad_cl(const void *x1, int c1, const void *x2, int c2, const void *dy, int cout, int nb, int nz,
+                            int ny, int nx, int ntaps, int kper, float *dw, void *stream) {
+    CT_REQUIRE(x1 && dy && dw && (c2 == 0 || x2), "conv3d_wgrad_cl: null pointer");
+    CT_REQUIRE(ntaps == 1 || ntaps == 27, "conv3d_wgrad_cl: ntaps must be 1 or 27");
+    CT_REQUIRE(c1 > 0 && c1 % 32 == 0 && c2 >= 0 && c2 % 32 == 0 && cout > 0 && cout % 32 == 0 &&
+                   c1 <= 32 * 65535 - c2 && cout <= 32 * 65535,
+               "conv3d_wgrad_cl: channels must be positive multiples of 32");
+    CT_REQUIRE(nb > 0 && nz > 0 && ny > 0 && nx > 0 && nx % kYBx == 0 && ny % kYBy == 0 && (long long)nx * ny < (1ll << 30),
+               "conv3d_wgrad_cl: x must be a multiple of 8, y of 16");
+    CT_REQUIRE(kper > 0, "conv3d_wgrad_cl: kper must be positive");
+    CT_REQUIRE(aligned16(x1) && aligned16(dy) && (!x2 || aligned16(x2)),
+               "conv3d_wgrad_cl: pointers must be 16-byte aligned");
+    CT_REQUIRE(((long long)nb * nz * ((nx * ny + kWK - 1) / kWK) + kper - 1) / kper <= 65535,
+               "conv3d_wgrad_cl: too many K splits (raise kper)");
+    CUtensorMap m1, m2, md;
+    int s;
+    if ((s = map_ndhwc(&m1, x1, c1, nx, ny, nz, nb, kYBx, kYBy, 1))) return s;
+    if ((s = map_ndhwc(&m2, c2 ? x2 : x1, c2 ? c2 : c1, nx, ny, nz, nb, kYBx, kYBy, 1))) return s;
+    if ((s = map_ndhwc(&md, dy, cout, nx, ny, nz, nb, kYBx, ntaps == 27 ? kYBy + 2 : kYBy, 1))) return s;
+    ClArgs a{};
+    a.c1 = c1;
+    a.cin = c1 + c2;
+    a.cout = cout;
+    a.nz = nz;
+    a.tx = nx / kYBx;
+    a.ty = ny / kYBy;
+    a.flush = std::max(1, kper / 2);                       // tiles of 128 voxels, slices of 64
+    a.dw = dw;
+    // slices per item: the fewest steps of the busiest CTA, as the z-marching forward kernel chooses them
+    const int px = a.cin / 32, py = cout / 32;
+    const long long columns = (long long)nb * a.tx * a.ty, sms = std::max(1, sm_count() / (px * py));
+    long long best = -1;
+    for (int parts = 1; parts <= nz; ++parts) {
+        const int zc = (nz + parts - 1) / parts;
+        const long long items = columns * ((nz + zc - 1) / zc), cost = (items + sms - 1) / sms * (zc + 1);
+        if (best >= 0 && cost >= best) continue;
+        best = cost;
+        a.zc = zc;
+        a.items = items;
+    }
+    a.nzc = (nz + a.zc - 1) / a.zc;
+    const unsigned ctas = (unsigned)std::min(a.items, sms);
+    cudaStream_t st = as_stream(stream);
+    return ntaps == 27 ? launch_wgrad_cl<27>(m1, m2, md, a, px, py, ctas, st)
+                       : launch_wgrad_cl<1>(m1, m2, md, a, px, py, ctas, st);
 }
 
 int ct_unet_wait_selftest(long long limit_ns, void *stream) {

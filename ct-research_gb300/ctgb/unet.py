@@ -19,7 +19,7 @@ Architecture (4 levels, 32 base channels, 3x3x3 convolutions, ReLU):
     head: 1x1, 32 -> 1, added to the input
 
 Every convolution, forward and both gradients, runs in ``ct_unet_conv3d`` /
-``ct_unet_conv3d_wgrad`` (bf16 operands, FP32 accumulation in tensor memory);
+``ct_unet_conv3d_wgrad[_cl]`` (bf16 operands, FP32 accumulation in tensor memory);
 pooling, upsampling, the head and the bias gradients are small CUDA kernels of
 the same library.  PyTorch holds the tensors and runs Adam on the FP32 master
 weights.  Activations are bf16 channels-last [n][z][y][x][c].
@@ -100,16 +100,29 @@ def shift_copies(xs, ntaps=27):
     return xm, x0, xp
 
 
+def _wgrad_cl(cs, cout, y, x):
+    """Whether a weight gradient can read the channels-last tensors: whole 32-channel chunks and 8 x 16 voxel tiles
+    (faster than the channel-major copies at every channel count measured: 128^3, 32 x 32: 125 against 948 us,
+    32^3, 256 x 256: 157 against 164)."""
+    return len(cs) <= 2 and all(c % 32 == 0 for c in cs) and cout in (32, 64, 128, 256) and x % 8 == 0 and y % 16 == 0
+
+
 def conv3d_wgrad(xs, dy, ntaps=27, kper=None):
     """FP32 weight gradient [cout][taps][cin] of conv3d(concat(xs)) for output gradient dy."""
     n, z, y, x, cout = dy.shape
-    xm, x0, xp = shift_copies(xs, ntaps)
-    _, dyt, _ = shift_copies([dy], 1)
-    cin = x0.shape[1]
+    cs = [t.shape[-1] for t in xs]
+    cin = sum(cs)
     dw = torch.zeros((cout, ntaps, cin), dtype=torch.float32, device=dy.device)
     if kper is None:
         chunks = n * z * y * x // 64
         kper = max(16, -(-chunks // 1024))
+    if _wgrad_cl(cs, cout, y, x):
+        x2 = xs[1] if len(xs) > 1 else None
+        _lib.call("ct_unet_conv3d_wgrad_cl", _tptr(xs[0]), cs[0], _p(x2), cin - cs[0], _tptr(dy), cout, n, z, y, x,
+                  ntaps, int(kper), _tptr(dw), _stream())
+        return dw
+    xm, x0, xp = shift_copies(xs, ntaps)
+    _, dyt, _ = shift_copies([dy], 1)
     _lib.call("ct_unet_conv3d_wgrad", _p(xm), _tptr(x0), _p(xp), cin, _tptr(dyt), cout, n, z, y, x, ntaps, int(kper),
               _tptr(dw), _stream())
     return dw

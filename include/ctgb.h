@@ -393,6 +393,12 @@ int ct_unet_conv3d(const void *d_x1, int c1, const void *d_x2, int c2, int nb, i
  * planes. */
 int ct_unet_conv3d_wgrad(const void *d_xm, const void *d_x0, const void *d_xp, int cin, const void *d_dy, int cout,
                          int nb, int nz, int ny, int nx, int ntaps, int kper, float *d_dw, void *stream);
+/* The same gradient from the channels-last tensors themselves: X the concat of
+ * d_x1 [v][c1] and d_x2 [v][c2] (c2 may be 0), dY [v][cout].  Channels multiples
+ * of 32, x a multiple of 8, y of 16; partial sums of kper / 2 tiles of 128
+ * voxels. */
+int ct_unet_conv3d_wgrad_cl(const void *d_x1, int c1, const void *d_x2, int c2, const void *d_dy, int cout, int nb,
+                            int nz, int ny, int nx, int ntaps, int kper, float *d_dw, void *stream);
 /* Reads and clears the device flag of the convolutions' bounded waits:
  * CT_ERR_TIMEOUT (flags != 0) when a wait gave up since the last call.  Flag
  * bits: 1 a free ring stage, 2 a loaded stage, 4 the last MMA, 8 the self-test. */

@@ -308,3 +308,29 @@ def test_conv3d_marching_along_z(c1, c2, cout, nb, nz, ny, nx, split, masked):
         r = r.to(bf).float()
         err = float((o.float() - r).norm() / r.norm())
         assert err <= 2e-3 and float((o.float() == r).float().mean()) >= 0.99, err
+
+
+# weight gradient from channels-last tensors: one slice, partial sums of one tile and of a number that does not divide
+# the tiles, more items than CTAs, two inputs, three chunks, one tap, a y that the tiles do not fit.  Against FP64 sums
+# of the same bf16 values: FP32 sums of at most 2^14 products between two additions, so 2^14 2^-24 = 1e-3 of the
+# absolute sum at the very worst and, rounding at random, about 2^7 2^-24 = 8e-6 of the norm; 1e-4 leaves ten times that.
+@pytest.mark.gpu
+@pytest.mark.parametrize("cins,cout,taps,nb,nz,ny,nx,kper", [
+    ((32,), 32, 27, 1, 1, 16, 8, 1), ((32,), 64, 27, 2, 2, 16, 24, 6), ((64, 32), 32, 27, 1, 7, 32, 16, 10),
+    ((32,), 32, 27, 3, 21, 64, 72, None), ((32, 32), 64, 1, 2, 5, 48, 40, 14), ((128,), 128, 27, 1, 3, 16, 16, 4),
+    ((32,), 32, 27, 1, 3, 24, 16, 4)])
+def test_conv3d_wgrad_channels_last(cins, cout, taps, nb, nz, ny, nx, kper):
+    import torch
+    from ctgb import unet
+    g = torch.Generator(device="cuda").manual_seed(sum(cins) + cout + nz)
+    xs = [torch.randn((nb, nz, ny, nx, c), device="cuda", generator=g).to(torch.bfloat16) for c in cins]
+    dy = torch.randn((nb, nz, ny, nx, cout), device="cuda", generator=g).to(torch.bfloat16)
+    dw = unet.conv3d_wgrad(xs, dy, taps, kper=kper)
+    assert unet.status() == 0
+    r = 1 if taps == 27 else 0
+    x = torch.nn.functional.pad(torch.cat(xs, -1).double(), (0, 0) + (r,) * 6)
+    ref = torch.zeros_like(dw, dtype=torch.float64)
+    for t in range(taps):
+        a, b, e = (t // 9, t // 3 % 3, t % 3) if r else (0, 0, 0)
+        ref[:, t] = dy.double().reshape(-1, cout).t() @ x[:, a:a + nz, b:b + ny, e:e + nx].reshape(-1, sum(cins))
+    assert float((dw.double() - ref).norm() / ref.norm()) <= 1e-4
