@@ -313,6 +313,82 @@ colsum_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long l
     }
 }
 
+// The same where a voxel's channels come in whole 16-byte groups: 8 channels per
+// thread, lanes of a block summed in a tree, one atomic per block and channel
+// with a block's channels side by side (a thread adding its 8 itself makes eight
+// times the requests: 56 us instead of 15 for 64 channels).  128^3 x 32 channels
+// (134 MB): 35 us against 43 with 2-byte loads; 64^3 x 128: 5.7 against 9.3.
+__global__ void __launch_bounds__(256)
+colsum8_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long long nvox) {
+    const int c8 = c / 8, lanes = 256 / c8;
+    const int g = threadIdx.x % c8, l = threadIdx.x / c8;
+    float s[8] = {};
+    const uint4 *src = reinterpret_cast<const uint4 *>(dy) + g;
+    const long long step = static_cast<long long>(gridDim.x) * lanes;
+    long long v = blockIdx.x * static_cast<long long>(lanes) + l;
+    for (; v + 3 * step < nvox; v += 4 * step) {           // four loads in flight
+        uint4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = __ldg(src + (v + u * step) * c8);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            float f[8];
+            unpack8(q[u], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += f[j];
+        }
+    }
+    for (; v < nvox; v += step) {
+        float f[8];
+        unpack8(__ldg(src + v * c8), f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += f[j];
+    }
+    __shared__ float red[8][256];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[j][threadIdx.x] = s[j];
+    for (int h = lanes / 2; h > 0; h /= 2) {
+        __syncthreads();
+        if (l < h)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) red[j][threadIdx.x] += red[j][threadIdx.x + h * c8];
+    }
+    __syncthreads();
+    if (threadIdx.x < c) atomicAdd(db + threadIdx.x, red[threadIdx.x % 8][threadIdx.x / 8]);   // whole lines at once
+}
+
+// One Adam step of a parameter and its bf16 copy (null: none).  Twelve
+// element-wise passes of separate launches in one: bound by memory at the large
+// parameters, by the launch at the small ones.
+__global__ void __launch_bounds__(256)
+adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
+            bf16 *__restrict__ wb, long long n, float b1, float a1, float b2, float a2, float inv1, float inv2, float lr,
+            float eps) {
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (i >= n) return;
+    const float gi = g[i], mi = fmaf(a1, gi, m[i] * b1), vi = fmaf(a2 * gi, gi, v[i] * b2);
+    const float pi = fmaf(-lr, (mi * inv1) / (sqrtf(vi * inv2) + eps), p[i]);
+    m[i] = mi;
+    v[i] = vi;
+    p[i] = pi;
+    if (wb) wb[i] = __float2bfloat16(pi);
+}
+
+// Weights of the data gradient: [cout][taps][cin] -> [cin][taps reversed][cout],
+// 32 x 32 channel tiles of one tap through shared memory.
+__global__ void __launch_bounds__(256)
+flip_weights_kernel(const bf16 *__restrict__ w, bf16 *__restrict__ out, int cout, int taps, int cin) {
+    __shared__ bf16 tile[32][33];
+    const int t = blockIdx.z, ci0 = blockIdx.x * 32, co0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += 8)
+        if (co0 + r < cout && ci0 + threadIdx.x < cin)
+            tile[r][threadIdx.x] = w[((long long)(co0 + r) * taps + t) * cin + ci0 + threadIdx.x];
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += 8)
+        if (ci0 + r < cin && co0 + threadIdx.x < cout)
+            out[((long long)(ci0 + r) * taps + taps - 1 - t) * cout + co0 + threadIdx.x] = tile[threadIdx.x][r];
+}
+
 unsigned blocks_for(long long n, int threads) { return static_cast<unsigned>((n + threads - 1) / threads); }
 
 bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -434,10 +510,39 @@ int ct_unet_colsum(const void *dy, int c, long long nvox, float *db, void *strea
     CT_REQUIRE(dy && db, "colsum: null pointer");
     CT_REQUIRE(c > 0 && c <= 256 && 256 % c == 0, "colsum: channels must divide 256");
     CT_REQUIRE(nvox > 0, "colsum: bad voxel count");
+    if (c % 8 == 0 && al16(dy)) {
+        // about four voxels per lane and block at least: an atomic per block and channel
+        const unsigned blocks = static_cast<unsigned>(
+            std::min<long long>((nvox + 1024LL / (c / 8) - 1) / (1024 / (c / 8)), 8LL * sm_count()));
+        colsum8_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const bf16 *>(dy), db, c, nvox);
+        CT_LAUNCH_CHECK("colsum8_kernel");
+        return CT_OK;
+    }
     const long long lanes = 256 / c;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((nvox + lanes - 1) / lanes, 8LL * sm_count()));
     colsum_kernel<<<grid, 256, 0, as_stream(stream)>>>(static_cast<const bf16 *>(dy), db, c, nvox);
     CT_LAUNCH_CHECK("colsum_kernel");
+    return CT_OK;
+}
+
+int ct_unet_adam(float *p, const float *g, float *m, float *v, void *wb, long long n, double b1, double b2, double c1,
+                 double c2, double lr, double eps, void *stream) {
+    CT_REQUIRE(p && g && m && v, "adam: null pointer");
+    CT_REQUIRE(n > 0 && (n + 255) / 256 < (1ll << 31), "adam: bad element count");
+    adam_kernel<<<blocks_for(n, 256), 256, 0, as_stream(stream)>>>(
+        p, g, m, v, static_cast<bf16 *>(wb), n, (float)b1, (float)(1.0 - b1), (float)b2, (float)(1.0 - b2),
+        1.0f / (float)c1, 1.0f / (float)c2, (float)lr, (float)eps);
+    CT_LAUNCH_CHECK("adam_kernel");
+    return CT_OK;
+}
+
+int ct_unet_flip_weights(const void *w, void *out, int cout, int taps, int cin, void *stream) {
+    CT_REQUIRE(w && out && w != out, "flip_weights: null pointer, or in place");
+    CT_REQUIRE(cout > 0 && cin > 0 && taps > 0 && taps <= 65535 && (cout + 31) / 32 <= 65535,
+               "flip_weights: bad sizes");
+    flip_weights_kernel<<<dim3((cin + 31) / 32, (cout + 31) / 32, taps), dim3(32, 8), 0, as_stream(stream)>>>(
+        static_cast<const bf16 *>(w), static_cast<bf16 *>(out), cout, taps, cin);
+    CT_LAUNCH_CHECK("flip_weights_kernel");
     return CT_OK;
 }
 

@@ -107,12 +107,14 @@ def _wgrad_cl(cs, cout, y, x):
     return len(cs) <= 2 and all(c % 32 == 0 for c in cs) and cout in (32, 64, 128, 256) and x % 8 == 0 and y % 16 == 0
 
 
-def conv3d_wgrad(xs, dy, ntaps=27, kper=None):
-    """FP32 weight gradient [cout][taps][cin] of conv3d(concat(xs)) for output gradient dy."""
+def conv3d_wgrad(xs, dy, ntaps=27, kper=None, out=None):
+    """FP32 weight gradient [cout][taps][cin] of conv3d(concat(xs)) for output gradient dy; added to ``out`` if given."""
     n, z, y, x, cout = dy.shape
     cs = [t.shape[-1] for t in xs]
     cin = sum(cs)
-    dw = torch.zeros((cout, ntaps, cin), dtype=torch.float32, device=dy.device)
+    dw = torch.zeros((cout, ntaps, cin), dtype=torch.float32, device=dy.device) if out is None else out
+    if dw.shape != (cout, ntaps, cin) or dw.dtype != torch.float32:
+        raise ValueError("out must be float32 [cout][taps][cin]")
     if kper is None:
         chunks = n * z * y * x // 64
         kper = max(16, -(-chunks // 1024))
@@ -247,7 +249,12 @@ class UNet3D:
     def _wt(self, name):
         if name not in self.wt:
             w = self.wb[name]                            # [cout][taps][cin]
-            self.wt[name] = w.flip(1).transpose(0, 2).contiguous()   # [cin][taps][cout], taps reversed
+            if w.is_cuda:
+                cout, taps, cin = w.shape                # [cin][taps][cout], taps reversed
+                self.wt[name] = torch.empty((cin, taps, cout), dtype=BF16, device=w.device)
+                _lib.call("ct_unet_flip_weights", _tptr(w), _tptr(self.wt[name]), cout, taps, cin, _stream())
+            else:
+                self.wt[name] = w.flip(1).transpose(0, 2).contiguous()
         return self.wt[name]
 
     def state_dict(self):
@@ -309,10 +316,11 @@ class UNet3D:
         a = self.cache
         if a is None:
             raise RuntimeError("backward needs forward(..., keep=True)")
-        grads = {k: torch.zeros_like(v) for k, v in self.params.items()}
+        grads = {k: torch.empty_like(v) for k, v in self.params.items()}
+        torch._foreach_zero_(list(grads.values()))
 
         def wgrad(name, xs, dy, ntaps):
-            grads[name + ".w"] += conv3d_wgrad(xs, dy, ntaps)
+            conv3d_wgrad(xs, dy, ntaps, out=grads[name + ".w"])
             colsum(dy, grads[name + ".b"])
 
         dout = dout.reshape(a["x"].shape).contiguous()
@@ -368,17 +376,30 @@ class UNet3D:
     def adam_step(self, grads: dict, lr: float | None = None):
         s = self.adam
         s.t += 1
-        lr = s.lr if lr is None else lr
+        lr = float(s.lr if lr is None else lr)
         c1 = 1.0 - s.b1 ** s.t
         c2 = 1.0 - s.b2 ** s.t
+        wb = {}
         for k, p in self.params.items():
             g = grads[k]
-            m = s.m.setdefault(k, torch.zeros_like(p))
-            v = s.v.setdefault(k, torch.zeros_like(p))
-            m.mul_(s.b1).add_(g, alpha=1 - s.b1)
-            v.mul_(s.b2).addcmul_(g, g, value=1 - s.b2)
-            p.addcdiv_(m / c1, (v / c2).sqrt_().add_(s.eps), value=-lr)
-        self._refresh()
+            for st in (s.m, s.v):
+                if k not in st:
+                    st[k] = torch.zeros_like(p)
+            m, v = s.m[k], s.v[k]
+            w = k[:-2] if k.endswith(".w") and not k.startswith("head") else None
+            if all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.shape == p.shape
+                   and t.device == p.device for t in (p, g, m, v)):
+                if w:
+                    wb[w] = torch.empty(p.shape, dtype=BF16, device=p.device)
+                _lib.call("ct_unet_adam", _tptr(p), _tptr(g), _tptr(m), _tptr(v), _p(wb.get(w)), p.numel(), s.b1, s.b2,
+                          c1, c2, lr, s.eps, _stream())
+            else:
+                m.mul_(s.b1).add_(g, alpha=1 - s.b1)
+                v.mul_(s.b2).addcmul_(g, g, value=1 - s.b2)
+                p.addcdiv_(m / c1, (v / c2).sqrt_().add_(s.eps), value=-lr)
+                if w:
+                    wb[w] = p.to(BF16).contiguous()
+        self.wb, self.wt = wb, {}
 
 
 # -- FP32 reference of the same network (tests) ---------------------------------

@@ -399,6 +399,12 @@ int ct_unet_conv3d_wgrad(const void *d_xm, const void *d_x0, const void *d_xp, i
  * voxels. */
 int ct_unet_conv3d_wgrad_cl(const void *d_x1, int c1, const void *d_x2, int c2, const void *d_dy, int cout, int nb,
                             int nz, int ny, int nx, int ntaps, int kper, float *d_dw, void *stream);
+/* One Adam step of n FP32 parameters: m = b1 m + (1 - b1) g, v = b2 v + (1 - b2)
+ * g^2, p -= lr (m / c1) / (sqrt(v / c2) + eps); wb, if not null, gets p in bf16. */
+int ct_unet_adam(float *d_p, const float *d_g, float *d_m, float *d_v, void *d_wb, long long n, double b1, double b2,
+                 double c1, double c2, double lr, double eps, void *stream);
+/* bf16 weights [cout][taps][cin] to those of the data gradient, [cin][taps][cout] with the taps reversed. */
+int ct_unet_flip_weights(const void *d_w, void *d_out, int cout, int taps, int cin, void *stream);
 /* Reads and clears the device flag of the convolutions' bounded waits:
  * CT_ERR_TIMEOUT (flags != 0) when a wait gave up since the last call.  Flag
  * bits: 1 a free ring stage, 2 a loaded stage, 4 the last MMA, 8 the self-test. */

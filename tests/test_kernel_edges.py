@@ -334,3 +334,56 @@ def test_conv3d_wgrad_channels_last(cins, cout, taps, nb, nz, ny, nx, kper):
         a, b, e = (t // 9, t // 3 % 3, t % 3) if r else (0, 0, 0)
         ref[:, t] = dy.double().reshape(-1, cout).t() @ x[:, a:a + nz, b:b + ny, e:e + nx].reshape(-1, sum(cins))
     assert float((dw.double() - ref).norm() / ref.norm()) <= 1e-4
+
+
+# channel sums: 8 channels per thread at every channel count, lanes that the voxels do not fill, an unaligned tensor
+# (the 2-byte kernel).  FP32 sums of n values of size 1 against FP64: n 2^-24 of the absolute sum at the very worst.
+@pytest.mark.gpu
+@pytest.mark.parametrize("c,n,off", [(8, 1, 0), (8, 70001, 0), (32, 33, 0), (32, 500003, 0), (128, 4097, 0), (256, 7, 0),
+                                     (256, 100003, 0), (16, 1001, 2), (4, 999, 0)])
+def test_channel_sums(c, n, off):
+    import torch
+    from ctgb import _lib
+    from ctgb.unet import _tptr, _stream
+    g = torch.Generator(device="cuda").manual_seed(c + n)
+    x = torch.randn(n * c + off, device="cuda", generator=g).to(torch.bfloat16)[off:]
+    db = torch.ones(c, device="cuda")
+    _lib.call("ct_unet_colsum", _tptr(x), c, n, _tptr(db), _stream())
+    v = x.reshape(n, c).double()
+    assert bool(((db.double() - 1 - v.sum(0)).abs() <= (n + 8) * 2.0 ** -24 * (1 + v.abs().sum(0))).all())
+
+
+# one fused Adam pass against the same formula in FP64: a dozen FP32 roundings (2^-24 each) of m, v and the step; the
+# bf16 copy is the rounding of the new parameter.  The element-wise path of a non-contiguous gradient agrees with it.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 255, 70001])
+def test_adam_pass_and_flipped_weights(n):
+    import torch
+    from ctgb import unet
+    net = unet.UNet3D()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    net.params = {"a.w": torch.randn(n, device="cuda", generator=g), "head.b": torch.randn(1, device="cuda", generator=g)}
+    ref = {k: v.double() for k, v in net.params.items()}
+    other = {k: v.clone() for k, v in net.params.items()}
+    s = net.adam
+    m = {k: torch.zeros_like(v) for k, v in ref.items()}
+    v2 = {k: torch.zeros_like(v) for k, v in ref.items()}
+    twin = unet.UNet3D()
+    twin.params = other
+    for t in range(1, 4):
+        gr = {k: torch.randn(v.shape, device="cuda", generator=g) for k, v in net.params.items()}
+        net.adam_step(gr, lr=1e-2)
+        twin.adam_step({k: torch.stack((v, v), -1)[..., 0] for k, v in gr.items()}, lr=1e-2)
+        for k in ref:
+            gd = gr[k].double()
+            m[k] = s.b1 * m[k] + (1 - s.b1) * gd
+            v2[k] = s.b2 * v2[k] + (1 - s.b2) * gd * gd
+            ref[k] -= 1e-2 * (m[k] / (1 - s.b1 ** t)) / ((v2[k] / (1 - s.b2 ** t)).sqrt() + s.eps)
+            tol = 3 * 2.0 ** -24 * (ref[k].abs() + 1) * 4
+            assert bool(((net.params[k].double() - ref[k]).abs() <= tol).all())
+            assert bool(((twin.params[k].double() - ref[k]).abs() <= tol).all())
+    assert set(net.wb) == set(twin.wb) == {"a"} and torch.equal(net.wb["a"], net.params["a.w"].to(torch.bfloat16))
+    for shape in ((32, 27, 64), (64, 1, 32), (40, 27, 33)):
+        net.wb["w"] = torch.randn(shape, device="cuda", generator=g).to(torch.bfloat16)
+        net.wt.pop("w", None)
+        assert torch.equal(net._wt("w"), net.wb["w"].flip(1).transpose(0, 2).contiguous())
