@@ -138,6 +138,14 @@ def im2col27(vol):
     return out
 
 
+def conv_first(vol, w, bias=None, relu=False):
+    """conv3d(im2col27(vol), w, bias, relu, ntaps=1) without the gathered tensor: fp32 [n][z][y][x] -> bf16 [..][32]."""
+    n, z, y, x = vol.shape
+    out = torch.empty((n, z, y, x, 32), dtype=BF16, device=vol.device)
+    _lib.call("ct_unet_conv_first", _tptr(vol), n, z, y, x, _tptr(w), _p(bias), int(relu), _tptr(out), _stream())
+    return out
+
+
 def pool2(t):
     n, z, y, x, c = t.shape
     out = torch.empty((n, z // 2, y // 2, x // 2, c), dtype=BF16, device=t.device)
@@ -280,8 +288,11 @@ class UNet3D:
                              f"8-voxel tiles at the coarsest level); got {tuple(x.shape)}")
         x = x.contiguous()
         a = {"x": x}
-        a["g"] = im2col27(x)
-        a["e1a"] = self._conv("e1a", a["g"], ntaps=1)
+        if keep:
+            a["g"] = im2col27(x)                 # the weight gradient reads the gathered taps
+            a["e1a"] = self._conv("e1a", a["g"], ntaps=1)
+        else:
+            a["e1a"] = conv_first(x, self.wb["e1a"], self.params["e1a.b"], relu=_RELU["e1a"])
         a["e1"] = self._conv("e1b", a["e1a"], ntaps=27)
         a["p1"] = pool2(a["e1"])
         a["e2a"] = self._conv("e2a", a["p1"], ntaps=27)

@@ -417,6 +417,10 @@ int ct_unet_wait_selftest(long long limit_ns, void *stream);
 /* out[v][k] = vol[v + off(k)] (k < 27, zero outside), 0 for k = 27..31: the
  * one-channel input as 32 channels for a 1-tap convolution. */
 int ct_unet_im2col27(const float *d_vol, int nb, int nz, int ny, int nx, void *d_out, void *stream);
+/* That 1-tap convolution straight from the volume: 32 outputs, w bf16 [32][32]
+ * (out, tap), voxels a multiple of 128. */
+int ct_unet_conv_first(const float *d_vol, int nb, int nz, int ny, int nx, const void *d_w, const float *d_bias,
+                       int relu, void *d_out, void *stream);
 /* 2x2x2 max pooling and its gradient (to the first maximum of each window,
  * when that maximum is > 0: the pooled tensors are ReLU outputs);
  * nearest 2x upsampling and its gradient (sum of the 8 children).  Sizes are

@@ -387,3 +387,24 @@ def test_adam_pass_and_flipped_weights(n):
         net.wb["w"] = torch.randn(shape, device="cuda", generator=g).to(torch.bfloat16)
         net.wt.pop("w", None)
         assert torch.equal(net._wt("w"), net.wb["w"].flip(1).transpose(0, 2).contiguous())
+
+
+# the first convolution from the volume itself: the same instructions on the same bf16 values as the gathered tensor's
+# 1-tap convolution, so the same bits; one tile, tiles across x rows, slices and samples, thin volumes.
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb,nz,ny,nx,relu,biased", [(1, 1, 1, 128, True, True), (1, 16, 16, 16, True, True),
+                                                     (2, 5, 16, 24, False, True), (3, 64, 48, 80, True, False),
+                                                     (1, 2, 64, 1, True, True)])
+def test_conv_first_matches_gathered_taps(nb, nz, ny, nx, relu, biased):
+    import torch
+    from ctgb import unet
+    g = torch.Generator(device="cuda").manual_seed(nz + nx)
+    vol = torch.randn((nb, nz, ny, nx), device="cuda", generator=g)
+    w = torch.randn((32, 1, 32), device="cuda", generator=g)
+    w[:, :, 27:] = 0
+    w = w.to(torch.bfloat16)
+    bias = torch.randn(32, device="cuda", generator=g) if biased else None
+    out = unet.conv_first(vol, w, bias, relu)
+    assert unet.status() == 0
+    taps = unet.im2col27(vol).reshape(1, 1, -1, 128, 32)      # as rows of 128 voxels: a shape the 1-tap kernel takes
+    assert torch.equal(out.reshape(-1), unet.conv3d(taps, w, bias, relu=relu, ntaps=1).reshape(-1))
