@@ -374,10 +374,10 @@ def run_ours(args):
     kern = {
         "cone_fp_kernel": {"ms": t_fp * 1e3, "algorithmic_bytes": fp_bytes,
                            "achieved_gbs": fp_bytes / t_fp / 1e9, "segments": segs},
-        "cone_bp_kernel+pack_quads": {"ms": t_bp * 1e3, "algorithmic_bytes": bp_bytes,
+        "cone_bp_kernel+pack+setup": {"ms": t_bp * 1e3, "algorithmic_bytes": bp_bytes,
                                       "achieved_gbs": bp_bytes / t_bp / 1e9},
     }
-    dom = "cone_fp_kernel" if t_fp >= t_bp else "cone_bp_kernel+pack_quads"
+    dom = "cone_fp_kernel" if t_fp >= t_bp else "cone_bp_kernel+pack+setup"
     ach = kern[dom]["achieved_gbs"]
     full_case = args.size == "full" and not args.views
     tr = traffic.get(dom.split("+")[0]) if full_case else None
@@ -415,11 +415,11 @@ def run_ours(args):
             "config": {"workload": line_workload,
                        "parallelism": (f"views split over {world} ranks, NCCL all-reduce of the volume" if sharded
                                        else f"replicas x{world}"),
-                       "l2": "inputs larger than L2 (512 MiB volume, 566 MB sinogram, 2.3 GB packed quads)",
+                       "l2": "inputs larger than L2 (512 MiB volume, 566 MB sinogram, 1.1 GB packed pairs)",
                        "phantom": "12 random ellipsoids, seed 2"},
             "roofline": roofline, "kernels": kern, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks,
             "parity": parity,
-            # per step: transpose_ts, cone_fp, cone_fixup, then pack_quads + cone_bp per view chunk
+            # per step: transpose_ts, cone_fp, cone_fixup, then pack_pairs + cone_bp_setup + cone_bp per view chunk
             "gpu_launches": plan.launches_per_pair() * args.steps, "sirt_tv_learned_vs_plain": warm}
     print(json.dumps(line), flush=True)
     if dist:

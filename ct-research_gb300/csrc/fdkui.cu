@@ -309,10 +309,7 @@ fdkui_setup_kernel(const UIGeom g, const UIView *__restrict__ views, const doubl
 // `last`, into the display.
 // 8 blocks per SM (64 registers): 48.0 ms for filter and backprojection of 936 x 80 x
 // 800 into 512 x 512 x 50, against 52.2 / 56.8 / 63.2 ms at 6 / 5 / 4.
-#ifndef CT_UI_MINB
-#define CT_UI_MINB 8
-#endif
-__global__ void __launch_bounds__(128, CT_UI_MINB)
+__global__ void __launch_bounds__(128, 8)
 fdkui_bp_kernel(const UIGeom g, const UICol *__restrict__ rec, const float *__restrict__ xif,
                 const float *__restrict__ rcov, float2 *__restrict__ part, double *__restrict__ disp, int v0, int nv,
                 bool first, bool last) {

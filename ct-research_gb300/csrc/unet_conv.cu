@@ -16,20 +16,22 @@
 //   activation, rounds to bf16 and splits the channels over one or two outputs.
 //   conv_march_kernel is the same convolution for few channels: it keeps the
 //   filters in shared memory and reads each input slice once.
-// * conv_wgrad_cl_kernel (weight gradient): the channels-last tensors as they are,
-//   see below.  conv_wgrad_kernel, for volumes that its tiles do not fit: rows = (tap, input channel), columns
-//   = output channels, K = voxels in 64-voxel slices (128-byte rows, 128-byte
-//   swizzle).  Activations and output gradients are read channel-major
-//   [n][c][z][y*x]; x offsets come from three x-shifted copies (so the
-//   innermost TMA coordinate stays on the 16-byte grid), y and z offsets move
-//   the box.  Split-K over voxel ranges; partial sums are added to an FP32
-//   gradient with atomics.
+// * conv_first_kernel: the one-channel input's 27 taps built in shared memory.
+// * conv_wgrad_cl_kernel (weight gradient): the channels-last tensors as they
+//   are, see below.  conv_wgrad_kernel, for volumes that its tiles do not fit:
+//   rows = (tap, input channel), columns = output channels, K = voxels in
+//   64-voxel slices (128-byte rows, 128-byte swizzle).  Activations and output
+//   gradients are read channel-major [n][c][z][y*x]; x offsets come from three
+//   x-shifted copies (so the innermost TMA coordinate stays on the 16-byte
+//   grid), y and z offsets move the box.  Split-K over voxel ranges; partial
+//   sums are added to an FP32 gradient with atomics.
 //
-// A warp-specialised pipeline per CTA: warp 0 issues TMA loads into a
-// 3- or 4-stage ring, warp 1 the MMAs (one elected lane of a converged warp each),
-// and after the last MMA all four warps read the accumulator from TMEM (tcgen05.ld) for the epilogue.  Every
-// mbarrier wait is bounded by a 2 s timer; a timeout sets a device error flag
-// (read by ct_unet_status), drains the loads in flight and frees TMEM.
+// A warp-specialised pipeline per CTA: warp 0 issues TMA loads into a 3- or
+// 4-stage ring, warp 1 the MMAs (one elected lane of a converged warp each), and
+// after the last MMA all four warps read the accumulator from TMEM (tcgen05.ld)
+// for the epilogue.  Every mbarrier wait is bounded by a 2 s timer; a timeout
+// sets a device error flag (read by ct_unet_status), the loads in flight are
+// waited for and TMEM is freed.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -228,8 +230,10 @@ struct Ctrl {
     uint64_t empty[kStages];
     uint64_t done;
     uint32_t tmem;
-    int abort;
 };
+
+// A wait gave up: each role then ends on its own waits, all bounded.
+__device__ __forceinline__ void flag_error(int code) { atomicOr(&g_unet_err, code); }
 
 __device__ __forceinline__ void tap_offsets(int tap, int ntaps, int &dz, int &dy, int &dx) {
     if (ntaps == 27) {
@@ -241,14 +245,7 @@ __device__ __forceinline__ void tap_offsets(int tap, int ntaps, int &dz, int &dy
     }
 }
 
-__device__ __forceinline__ void fail(Ctrl *c, int code) {
-    atomicOr(&g_unet_err, code);
-    *reinterpret_cast<volatile int *>(&c->abort) = 1;
-}
-
-__device__ __forceinline__ bool aborted(Ctrl *c) { return *reinterpret_cast<volatile int *>(&c->abort) != 0; }
-
-// After an abort: wait (bounded) for the loads issued into each of the S stages.
+// Wait (bounded) until every load into the S stages has landed: no CTA leaves with one in flight, whichever wait gave up.
 template <int S>
 __device__ void drain_loads(Ctrl *c, int issued) {
     for (int s = 0; s < S && s < issued; ++s) {
@@ -301,7 +298,7 @@ __device__ __forceinline__ void mma_loop(Ctrl *c, uint8_t *ring, uint32_t tmem, 
             ph ^= 1;
         }
     }
-    if (!ok) fail(c, 2);
+    if (!ok) flag_error(2);
     if (elect_one()) umma_commit(&c->done);
 }
 
@@ -328,6 +325,8 @@ struct FwdArgs {
     __nv_bfloat16 *out1, *out2;
     int co1, co2;            // channels written to out1 / out2 (co1 + co2 = N)
     const __nv_bfloat16 *mask1, *mask2;   // ReLU-derivative masks (same layout as out1 / out2) or null
+    const float *head_w, *head_b, *base;  // conv_march_kernel's HEAD mode: 32 weights, bias, added volume or null
+    float *head_out;
 };
 
 // ReLU-derivative mask values of columns c0 .. c0 + 15 of a voxel.
@@ -410,7 +409,6 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
             mbar_init(&c->empty[s], 1);
         }
         mbar_init(&c->done, 1);
-        c->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) tmem_alloc(&c->tmem, N);
@@ -461,8 +459,8 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
                 }
             }
         }
-        if (!ok) fail(c, 1);
-        if (aborted(c)) drain_loads<S>(c, issued);
+        if (!ok) flag_error(1);
+        drain_loads<S>(c, issued);
     } else if (warp == 1) {
         mma_loop<N, S, a_bytes, ng, kYBx * kRowBytes>(c, ring, tmem, a.ksteps);
     }
@@ -470,7 +468,7 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__
 
     // epilogue: thread = tile row = voxel
     const bool ok = mbar_wait(&c->done, 0);
-    if (!ok) fail(c, 4);
+    if (!ok) flag_error(4);
     tc_fence_after();
     const int r = warp * 32 + lane;
     const int rxy = a.bx * a.by;
@@ -563,7 +561,11 @@ __device__ __forceinline__ MarchItem march_item(const MarchArgs &a, long long i)
     return it;
 }
 
-template <int N, int NCH>                                  // outputs, 32-channel chunks of the input
+// N outputs, NCH 32-channel chunks of the input.  HEAD (N = 32): instead of the 32
+// channels, their 1 x 1 convolution to one, added to `base`: the bf16 values and the
+// order of the sum are those of storing them and reading them back, without that
+// gigabyte at 256^3: 635 + 194 us as two launches, @HD@ as one.
+template <int N, int NCH, bool HEAD>
 __global__ void __launch_bounds__(192 * kMGroups, 1)
 conv_march_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mx2,
                   const __grid_constant__ CUtensorMap mw, const MarchArgs a) {
@@ -647,7 +649,7 @@ conv_march_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant
                 }
             }
         }
-        if (!ok && lane == 0) atomicOr(&g_unet_err, 1);
+        if (!ok && lane == 0) flag_error(1);
         // every load has landed before the CTA may leave: the last use of stage j
         mbar_wait(&ctrl->wfull, 0);
         for (int j = 0; j < used; ++j) mbar_wait(&c->full[j], j < s ? ph : ph ^ 1);
@@ -717,21 +719,31 @@ conv_march_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant
             }
             obase += it.z1 - it.z0;
         }
-        if (!ok && lane == 0) atomicOr(&g_unet_err, 2);
+        if (!ok && lane == 0) flag_error(2);
         if (elect_one()) umma_commit(&c->done);
     } else {
         const int r = (warp & 3) * 32 + lane;
         const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         unsigned o = 0;
         bool ok = true;
+        float hw[HEAD ? 32 : 1];
+        if (HEAD) {
+#pragma unroll
+            for (int j = 0; j < (HEAD ? 32 : 1); ++j) hw[j] = __ldg(a.f.head_w + j);
+        }
         for (long long i = item0; ok && i < a.items; i += istep) {
             const MarchItem it = march_item(a, i);
             long long vox = ((static_cast<long long>(it.n) * nz + it.z0) * a.f.ny + it.y0 + r / kYBx) * a.f.nx + it.x0 +
                             r % kYBx;
             for (int z = it.z0; z < it.z1; ++z, ++o, vox += static_cast<long long>(a.f.ny) * a.f.nx) {
                 Mask16 m[N / 16];
+                float sum = 0.0f;
+                if (HEAD) {
+                    sum = __ldg(a.f.head_b) + (a.f.base ? __ldg(a.f.base + vox) : 0.0f);
+                } else {
 #pragma unroll
-                for (int j = 0; j < N / 16; ++j) m[j] = load_mask(a.f, vox, n0 + 16 * j);
+                    for (int j = 0; j < N / 16; ++j) m[j] = load_mask(a.f, vox, n0 + 16 * j);
+                }
                 ok = __all_sync(0xffffffffu, mbar_wait(&c->accfull[o % R], (o / R) & 1));
                 if (!ok) break;
                 tc_fence_after();
@@ -746,14 +758,24 @@ conv_march_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant
                             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&c->accempty[o % R]))
                                          : "memory");
                     }
-                    store16(a.f, vox, n0 + 16 * j, v, m[j]);
+                    if (HEAD) {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            float x = a.f.bias ? v[e] + __ldg(a.f.bias + 16 * j + e) : v[e];
+                            if (a.f.relu) x = fmaxf(x, 0.0f);
+                            sum = fmaf(hw[HEAD ? 16 * j + e : 0], __bfloat162float(__float2bfloat16_rn(x)), sum);
+                        }
+                    } else {
+                        store16(a.f, vox, n0 + 16 * j, v, m[j]);
+                    }
                 }
+                if (HEAD) a.f.head_out[vox] = sum;
             }
         }
-        if (!ok && lane == 0) atomicOr(&g_unet_err, 4);
+        if (!ok && lane == 0) flag_error(4);
     }
     __syncwarp();
-    if (!mbar_wait(&c->done, 0)) atomicOr(&g_unet_err, 4);
+    if (!mbar_wait(&c->done, 0)) flag_error(4);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -894,7 +916,7 @@ conv_first_kernel(const FirstArgs a) {
             }
         }
     }
-    if (!ok && r == 0) atomicOr(&g_unet_err, 4);
+    if (!ok && r == 0) flag_error(4);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -934,7 +956,6 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap mxm, const __grid_constant
             mbar_init(&c->empty[s], 1);
         }
         mbar_init(&c->done, 1);
-        c->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) tmem_alloc(&c->tmem, N);
@@ -980,15 +1001,15 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap mxm, const __grid_constant
                 }
             }
         }
-        if (!ok) fail(c, 1);
-        if (aborted(c)) drain_loads<kWStages>(c, k);
+        if (!ok) flag_error(1);
+        drain_loads<kWStages>(c, k);
     } else if (warp == 1) {
         mma_loop<N, kWStages, a_bytes, 1, 0, kWRowBytes>(c, ring, tmem, ksteps);
     }
     __syncwarp();
 
     const bool ok = mbar_wait(&c->done, 0);
-    if (!ok) fail(c, 4);
+    if (!ok) flag_error(4);
     tc_fence_after();
     const int r = warp * 32 + lane;
     const int tap = tap0 + r / a.rows_per_tap, ci = ci0 + r % a.rows_per_tap;
@@ -1143,7 +1164,7 @@ conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_const
                 }
             }
         }
-        if (!ok && lane == 0) atomicOr(&g_unet_err, 1);
+        if (!ok && lane == 0) flag_error(1);
         // every load has landed before the CTA may leave: the last use of stage j
         for (int j = 0; j < used; ++j) mbar_wait(&c->full[j], j < s ? ph : ph ^ 1);
     } else if (warp == 5) {
@@ -1201,7 +1222,7 @@ conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_const
                 }
             }
         }
-        if (!ok && lane == 0) atomicOr(&g_unet_err, 2);
+        if (!ok && lane == 0) flag_error(2);
         if (elect_one()) umma_commit(&c->done);
     } else if (warp < NX) {                                // warp = dx + 1, lane = input channel
         long long tiles = 0;
@@ -1233,10 +1254,10 @@ conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_const
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&c->accempty[j])) : "memory");
             }
         }
-        if (!ok && lane == 0) atomicOr(&g_unet_err, 4);
+        if (!ok && lane == 0) flag_error(4);
     }
     __syncwarp();
-    if (!mbar_wait(&c->done, 0)) atomicOr(&g_unet_err, 4);
+    if (!mbar_wait(&c->done, 0)) flag_error(4);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1344,7 +1365,7 @@ constexpr size_t march_smem() {
 
 // Slices per item: the groups of the persistent CTAs share ceil(items / groups) items each, and an item of zc outputs
 // reads zc + 2 slices; the zc with the fewest slices read by the busiest group, the longer one of equals.
-template <int N, int NCH>
+template <int N, int NCH, bool HEAD = false>
 int launch_march(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &mw, const FwdArgs &f, int nb,
                  cudaStream_t st) {
     MarchArgs a{};
@@ -1366,11 +1387,11 @@ int launch_march(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap
     constexpr size_t smem = march_smem<N, NCH>();
     static bool attr = false;
     if (!attr) {
-        CT_CUDA(cudaFuncSetAttribute(conv_march_kernel<N, NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        CT_CUDA(cudaFuncSetAttribute(conv_march_kernel<N, NCH, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "conv_march smem");
         attr = true;
     }
-    conv_march_kernel<N, NCH><<<(unsigned)((std::min(a.items, groups) + kMGroups - 1) / kMGroups * a.parts), 192 * kMGroups, smem, st>>>(m1, m2, mw, a);
+    conv_march_kernel<N, NCH, HEAD><<<(unsigned)((std::min(a.items, groups) + kMGroups - 1) / kMGroups * a.parts), 192 * kMGroups, smem, st>>>(m1, m2, mw, a);
     CT_LAUNCH_CHECK("conv_march_kernel");
     return CT_OK;
 }
@@ -1595,6 +1616,35 @@ int ct_unet_conv3d_wgrad_cl(const void *x1, int c1, const void *x2, int c2, cons
     cudaStream_t st = as_stream(stream);
     return ntaps == 27 ? launch_wgrad_cl<27>(m1, m2, md, a, px, py, ctas, st)
                        : launch_wgrad_cl<1>(m1, m2, md, a, px, py, ctas, st);
+}
+
+int ct_unet_conv3d_head(const void *x, int nb, int nz, int ny, int nx, const void *w, const float *bias, int relu,
+                        const float *head_w, const float *head_b, const float *base, float *out, void *stream) {
+    CT_REQUIRE(x && w && head_w && head_b && out, "conv3d_head: null pointer");
+    CT_REQUIRE(nb > 0 && nz > 0 && ny > 0 && nx > 0 && nx % kYBx == 0 && ny % kYBy == 0,
+               "conv3d_head: x must be a multiple of 8, y of 16");
+    CT_REQUIRE(aligned16(x) && aligned16(w), "conv3d_head: pointers must be 16-byte aligned");
+    const long long tiles = (long long)nb * nz * (ny / kYBy) * (nx / kYBx);
+    CT_REQUIRE(tiles < (1ll << 31), "conv3d_head: too many tiles");
+    CUtensorMap m, mw;
+    int s;
+    if ((s = map_ndhwc(&m, x, 32, nx, ny, nz, nb, kYBx, kYBy + 2, 1))) return s;
+    const uint64_t dims[3] = {32, 27, 32}, st[2] = {64, 27 * 64};
+    const uint32_t box[3] = {32, 1, 32};
+    if ((s = make_map(&mw, w, 3, dims, st, box))) return s;
+    FwdArgs a{};
+    a.c1 = 32;
+    a.nx = nx;
+    a.ny = ny;
+    a.nz = nz;
+    a.bias = bias;
+    a.relu = relu;
+    a.co1 = 32;
+    a.head_w = head_w;
+    a.head_b = head_b;
+    a.base = base;
+    a.head_out = out;
+    return launch_march<32, 1, true>(m, m, mw, a, nb, as_stream(stream));
 }
 
 int ct_unet_conv_first(const float *vol, int nb, int nz, int ny, int nx, const void *w, const float *bias, int relu,

@@ -88,6 +88,7 @@ SIGNATURES = {
     "ct_unet_adam": (_i, [_vp, _vp, _vp, _vp, _vp, _ll, _d, _d, _d, _d, _d, _d, _vp]),
     "ct_unet_flip_weights": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "ct_unet_conv_first": (_i, [_vp, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp]),
+    "ct_unet_conv3d_head": (_i, [_vp, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp]),
     "ct_unet_conv3d_wgrad_cl": (_i, [_vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp]),
     "ct_unet_status": (_i, [C.POINTER(_i)]),
     "ct_unet_wait_selftest": (_i, [_ll, _vp]),

@@ -180,6 +180,15 @@ def head(f, w, b, base):
     return out
 
 
+def conv3d_head(x, w, bias, relu, head_w, head_b, base):
+    """head(conv3d(x, w, bias, relu), head_w, head_b, base) for 32 channels, without the stored activation."""
+    out = torch.empty(x.shape[:-1], dtype=torch.float32, device=x.device)
+    n, z, y, xx, _ = x.shape
+    _lib.call("ct_unet_conv3d_head", _tptr(x), n, z, y, xx, _tptr(w), _p(bias), int(relu), _tptr(head_w), _tptr(head_b),
+              _p(base), _tptr(out), _stream())
+    return out
+
+
 def head_bwd(dout, f, w, dw, db):
     df = torch.empty_like(f)
     _lib.call("ct_unet_head_bwd", _tptr(dout), _tptr(f), _tptr(w), _tptr(df), _tptr(dw), _tptr(db), dout.numel(),
@@ -314,8 +323,12 @@ class UNet3D:
         a["c1"] = self._conv("u1", a["d2"], ntaps=1)
         a["up1"] = up2(a["c1"])
         a["d1a"] = self._conv("d1a", a["e1"], a["up1"], ntaps=27)
-        a["d1"] = self._conv("d1b", a["d1a"], ntaps=27)
-        out = head(a["d1"], self.params["head.w"], self.params["head.b"], x)
+        if keep:
+            a["d1"] = self._conv("d1b", a["d1a"], ntaps=27)
+            out = head(a["d1"], self.params["head.w"], self.params["head.b"], x)
+        else:
+            out = conv3d_head(a["d1a"], self.wb["d1b"], self.params["d1b.b"], _RELU["d1b"], self.params["head.w"],
+                              self.params["head.b"], x)
         self.cache = a if keep else None
         return out
 

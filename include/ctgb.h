@@ -439,6 +439,10 @@ int ct_unet_shift_t(const void *d_in, int c, int nb, int nz, int ny, int nx, voi
  * dw += sum_v dout f, db += sum_v dout. */
 int ct_unet_head(const void *d_f, const float *d_w, const float *d_b, const float *d_base, float *d_out,
                  long long nvox, void *stream);
+/* The head of a 3x3x3 convolution of 32 channels to 32 (w bf16 [32][27][32],
+ * bias, ReLU) without storing its output: x a multiple of 8, y of 16. */
+int ct_unet_conv3d_head(const void *d_x, int nb, int nz, int ny, int nx, const void *d_w, const float *d_bias, int relu,
+                        const float *d_head_w, const float *d_head_b, const float *d_base, float *d_out, void *stream);
 int ct_unet_head_bwd(const float *d_dout, const void *d_f, const float *d_w, void *d_df, float *d_dw, float *d_db,
                      long long nvox, void *stream);
 /* db[c] += sum_v dy[v][c] (bias gradient); c divides 256. */

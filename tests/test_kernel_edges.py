@@ -408,3 +408,20 @@ def test_conv_first_matches_gathered_taps(nb, nz, ny, nx, relu, biased):
     assert unet.status() == 0
     taps = unet.im2col27(vol).reshape(1, 1, -1, 128, 32)      # as rows of 128 voxels: a shape the 1-tap kernel takes
     assert torch.equal(out.reshape(-1), unet.conv3d(taps, w, bias, relu=relu, ntaps=1).reshape(-1))
+
+
+# the head taken from the convolution's accumulators: the same bf16 values summed in the same order as from the stored
+# activation, so the same bits; one slice, fewer slices than accumulators, several items per group, no base.
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb,nz,ny,nx,base", [(1, 1, 16, 8, True), (2, 5, 32, 24, False), (2, 37, 64, 72, True)])
+def test_conv_head_without_stored_activation(nb, nz, ny, nx, base):
+    import torch
+    from ctgb import unet
+    g = torch.Generator(device="cuda").manual_seed(nz)
+    x = torch.randn((nb, nz, ny, nx, 32), device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn((32, 27, 32), device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    bias, hw, hb = (torch.randn(k, device="cuda", generator=g) for k in (32, 32, 1))
+    b = torch.randn((nb, nz, ny, nx), device="cuda", generator=g) if base else None
+    out = unet.conv3d_head(x, w, bias, True, hw, hb, b)
+    assert unet.status() == 0
+    assert torch.equal(out, unet.head(unet.conv3d(x, w, bias, relu=True), hw, hb, b))
