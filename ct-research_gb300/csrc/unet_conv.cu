@@ -564,7 +564,8 @@ __device__ __forceinline__ MarchItem march_item(const MarchArgs &a, long long i)
 // N outputs, NCH 32-channel chunks of the input.  HEAD (N = 32): instead of the 32
 // channels, their 1 x 1 convolution to one, added to `base`: the bf16 values and the
 // order of the sum are those of storing them and reading them back, without that
-// gigabyte at 256^3: 635 + 194 us as two launches, @HD@ as one.
+// gigabyte at 256^3: 635 + 194 us as two launches, about 580 as one (a whole forward
+// pass 6.60 -> 6.35 ms).
 template <int N, int NCH, bool HEAD>
 __global__ void __launch_bounds__(192 * kMGroups, 1)
 conv_march_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mx2,
