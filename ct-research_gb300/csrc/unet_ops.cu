@@ -99,9 +99,11 @@ __global__ void pool2_kernel(const bf16 *__restrict__ in, bf16 *__restrict__ out
 
 // dx[child] = dy where the child is the first maximum of its window and that
 // maximum is > 0, else 0: the pooled activations are ReLU outputs, so this is
-// also the ReLU derivative of the pooling path
+// also the ReLU derivative of the pooling path.  With `skip` (the skip connection's
+// gradient) dx = skip + that, rounded once: a pass of its own read and wrote it again.
 __global__ void pool2_bwd_kernel(const bf16 *__restrict__ x, const bf16 *__restrict__ y, const bf16 *__restrict__ dy,
-                                 bf16 *__restrict__ dx, int c8, int cx, int cy, int cz, long long n) {
+                                 const bf16 *__restrict__ skip, bf16 *__restrict__ dx, int c8, int cx, int cy, int cz,
+                                 long long n) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
     const long long cv = i / c8;
@@ -122,6 +124,11 @@ __global__ void pool2_bwd_kernel(const bf16 *__restrict__ x, const bf16 *__restr
             const bool hit = !taken[j] && f[j] == m[j];
             o[j] = (hit && m[j] > 0.0f) ? d[j] : 0.0f;
             taken[j] = taken[j] || hit;
+        }
+        if (skip) {
+            unpack8(__ldg(reinterpret_cast<const uint4 *>(skip) + ch[k] * c8 + g), f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += f[j];
         }
         reinterpret_cast<uint4 *>(dx)[ch[k] * c8 + g] = pack8(o);
     }
@@ -357,21 +364,43 @@ colsum8_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long 
     if (threadIdx.x < c) atomicAdd(db + threadIdx.x, red[threadIdx.x % 8][threadIdx.x / 8]);   // whole lines at once
 }
 
-// One Adam step of a parameter and its bf16 copy (null: none).  Twelve
-// element-wise passes of separate launches in one: bound by memory at the large
-// parameters, by the launch at the small ones.
+// One Adam step of many parameters and their bf16 copies (null: none), 1024
+// elements of one of them per block.  Twelve element-wise passes per parameter in
+// one launch for all: bound by memory at the large parameters, and the small ones
+// (biases of 32 to 256) share its launch.
+constexpr int kAdamTensors = 48, kAdamBlock = 1024;
+
+struct AdamArgs {
+    float *p[kAdamTensors];
+    const float *g[kAdamTensors];
+    float *m[kAdamTensors], *v[kAdamTensors];
+    bf16 *wb[kAdamTensors];
+    long long n[kAdamTensors];
+    unsigned first[kAdamTensors + 1];   // a tensor's first block; the block count at the end
+    int count;
+    float b1, a1, b2, a2, inv1, inv2, lr, eps;
+};
+
 __global__ void __launch_bounds__(256)
-adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-            bf16 *__restrict__ wb, long long n, float b1, float a1, float b2, float a2, float inv1, float inv2, float lr,
-            float eps) {
-    const long long i = blockIdx.x * 256ll + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i], mi = fmaf(a1, gi, m[i] * b1), vi = fmaf(a2 * gi, gi, v[i] * b2);
-    const float pi = fmaf(-lr, (mi * inv1) / (sqrtf(vi * inv2) + eps), p[i]);
-    m[i] = mi;
-    v[i] = vi;
-    p[i] = pi;
-    if (wb) wb[i] = __float2bfloat16(pi);
+adam_kernel(const __grid_constant__ AdamArgs a) {
+    int t = 0;
+    for (int h = 32; h > 0; h >>= 1)                       // the last tensor that starts at or before this block
+        if (t + h < a.count && a.first[t + h] <= blockIdx.x) t += h;
+    const long long i0 = static_cast<long long>(blockIdx.x - a.first[t]) * kAdamBlock + threadIdx.x;
+    float *p = a.p[t], *m = a.m[t], *v = a.v[t];
+    const float *g = a.g[t];
+    bf16 *wb = a.wb[t];
+#pragma unroll
+    for (int u = 0; u < kAdamBlock / 256; ++u) {
+        const long long i = i0 + u * 256;
+        if (i >= a.n[t]) break;
+        const float gi = g[i], mi = fmaf(a.a1, gi, m[i] * a.b1), vi = fmaf(a.a2 * gi, gi, v[i] * a.b2);
+        const float pi = fmaf(-a.lr, (mi * a.inv1) / (sqrtf(vi * a.inv2) + a.eps), p[i]);
+        m[i] = mi;
+        v[i] = vi;
+        p[i] = pi;
+        if (wb) wb[i] = __float2bfloat16(pi);
+    }
 }
 
 // Weights of the data gradient: [cout][taps][cin] -> [cin][taps reversed][cout],
@@ -430,16 +459,21 @@ int ct_unet_pool2(const void *in, void *out, int c, int nb, int nz, int ny, int 
     return CT_OK;
 }
 
-int ct_unet_pool2_bwd(const void *x, const void *y, const void *dy, void *dx, int c, int nb, int nz, int ny, int nx,
-                      void *stream) {
+int ct_unet_pool2_bwd_add(const void *x, const void *y, const void *dy, const void *skip, void *dx, int c, int nb, int nz,
+                          int ny, int nx, void *stream) {
     long long n;
     if (int s = pool_args(x, dx, c, nb, nz, ny, nx, n)) return s;
-    CT_REQUIRE(y && dy && al16(y) && al16(dy), "pool2_bwd: null or unaligned pointer");
+    CT_REQUIRE(y && dy && al16(y) && al16(dy) && al16(skip), "pool2_bwd: null or unaligned pointer");
     pool2_bwd_kernel<<<blocks_for(n, 256), 256, 0, as_stream(stream)>>>(
         static_cast<const bf16 *>(x), static_cast<const bf16 *>(y), static_cast<const bf16 *>(dy),
-        static_cast<bf16 *>(dx), c / 8, nx, ny, nz * nb, n);
+        static_cast<const bf16 *>(skip), static_cast<bf16 *>(dx), c / 8, nx, ny, nz * nb, n);
     CT_LAUNCH_CHECK("pool2_bwd_kernel");
     return CT_OK;
+}
+
+int ct_unet_pool2_bwd(const void *x, const void *y, const void *dy, void *dx, int c, int nb, int nz, int ny, int nx,
+                      void *stream) {
+    return ct_unet_pool2_bwd_add(x, y, dy, nullptr, dx, c, nb, nz, ny, nx, stream);
 }
 
 int ct_unet_up2(const void *in, void *out, int c, int nb, int nz, int ny, int nx, void *stream) {
@@ -525,14 +559,36 @@ int ct_unet_colsum(const void *dy, int c, long long nvox, float *db, void *strea
     return CT_OK;
 }
 
-int ct_unet_adam(float *p, const float *g, float *m, float *v, void *wb, long long n, double b1, double b2, double c1,
-                 double c2, double lr, double eps, void *stream) {
-    CT_REQUIRE(p && g && m && v, "adam: null pointer");
-    CT_REQUIRE(n > 0 && (n + 255) / 256 < (1ll << 31), "adam: bad element count");
-    adam_kernel<<<blocks_for(n, 256), 256, 0, as_stream(stream)>>>(
-        p, g, m, v, static_cast<bf16 *>(wb), n, (float)b1, (float)(1.0 - b1), (float)b2, (float)(1.0 - b2),
-        1.0f / (float)c1, 1.0f / (float)c2, (float)lr, (float)eps);
-    CT_LAUNCH_CHECK("adam_kernel");
+int ct_unet_adam(int count, float *const *p, const float *const *g, float *const *m, float *const *v, void *const *wb,
+                 const long long *n, double b1, double b2, double c1, double c2, double lr, double eps, void *stream) {
+    CT_REQUIRE(count > 0 && p && g && m && v && wb && n, "adam: null pointer or no tensors");
+    for (int i = 0; i < count; ++i) {
+        CT_REQUIRE(p[i] && g[i] && m[i] && v[i], "adam: null pointer");
+        CT_REQUIRE(n[i] > 0 && n[i] < (1ll << 31) * (kAdamBlock / kAdamTensors), "adam: bad element count");
+    }
+    for (int i0 = 0; i0 < count; i0 += kAdamTensors) {
+        AdamArgs a{};
+        a.count = std::min(kAdamTensors, count - i0);
+        for (int j = 0; j < a.count; ++j) {
+            a.p[j] = p[i0 + j];
+            a.g[j] = g[i0 + j];
+            a.m[j] = m[i0 + j];
+            a.v[j] = v[i0 + j];
+            a.wb[j] = static_cast<bf16 *>(wb[i0 + j]);
+            a.n[j] = n[i0 + j];
+            a.first[j + 1] = a.first[j] + blocks_for(a.n[j], kAdamBlock);
+        }
+        a.b1 = (float)b1;
+        a.a1 = (float)(1.0 - b1);
+        a.b2 = (float)b2;
+        a.a2 = (float)(1.0 - b2);
+        a.inv1 = 1.0f / (float)c1;
+        a.inv2 = 1.0f / (float)c2;
+        a.lr = (float)lr;
+        a.eps = (float)eps;
+        adam_kernel<<<a.first[a.count], 256, 0, as_stream(stream)>>>(a);
+        CT_LAUNCH_CHECK("adam_kernel");
+    }
     return CT_OK;
 }
 

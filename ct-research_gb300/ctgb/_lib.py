@@ -85,7 +85,8 @@ SIGNATURES = {
     "ct_tv_flow_asd": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _f, _f, _vp]),
     "ct_unet_conv3d": (_i, [_vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _i, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _vp]),
     "ct_unet_conv3d_wgrad": (_i, [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp]),
-    "ct_unet_adam": (_i, [_vp, _vp, _vp, _vp, _vp, _ll, _d, _d, _d, _d, _d, _d, _vp]),
+    "ct_unet_adam": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _d, _d, _d, _d, _d, _d, _vp]),
+    "ct_unet_pool2_bwd_add": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "ct_unet_flip_weights": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "ct_unet_conv_first": (_i, [_vp, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp]),
     "ct_unet_conv3d_head": (_i, [_vp, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp]),

@@ -153,10 +153,11 @@ def pool2(t):
     return out
 
 
-def pool2_bwd(x, y, dy):
+def pool2_bwd(x, y, dy, skip=None):
+    """Gradient of pool2, added to ``skip`` if given."""
     n, z, yy, xx, c = y.shape
     dx = torch.empty_like(x)
-    _lib.call("ct_unet_pool2_bwd", _tptr(x), _tptr(y), _tptr(dy), _tptr(dx), c, n, z, yy, xx, _stream())
+    _lib.call("ct_unet_pool2_bwd_add", _tptr(x), _tptr(y), _tptr(dy), _p(skip), _tptr(dx), c, n, z, yy, xx, _stream())
     return dx
 
 
@@ -380,17 +381,17 @@ class UNet3D:
         dp3 = conv3d(db1, self._wt("b1"))
         # enc3: the skip path is masked by e3 > 0 in its epilogue; the pooling
         # gradient reaches only window maxima that are > 0
-        de3 = de3_skip + pool2_bwd(a["e3"], a["p3"], dp3)
+        de3 = pool2_bwd(a["e3"], a["p3"], dp3, de3_skip)
         wgrad("e3b", [a["e3a"]], de3, 27)
         de3a = conv3d(de3, self._wt("e3b"), masks=(a["e3a"], None))
         wgrad("e3a", [a["p2"]], de3a, 27)
         dp2 = conv3d(de3a, self._wt("e3a"))
-        de2 = de2_skip + pool2_bwd(a["e2"], a["p2"], dp2)
+        de2 = pool2_bwd(a["e2"], a["p2"], dp2, de2_skip)
         wgrad("e2b", [a["e2a"]], de2, 27)
         de2a = conv3d(de2, self._wt("e2b"), masks=(a["e2a"], None))
         wgrad("e2a", [a["p1"]], de2a, 27)
         dp1 = conv3d(de2a, self._wt("e2a"))
-        de1 = de1_skip + pool2_bwd(a["e1"], a["p1"], dp1)
+        de1 = pool2_bwd(a["e1"], a["p1"], dp1, de1_skip)
         wgrad("e1b", [a["e1a"]], de1, 27)
         de1a = conv3d(de1, self._wt("e1b"), masks=(a["e1a"], None))
         wgrad("e1a", [a["g"]], de1a, 1)
@@ -403,7 +404,7 @@ class UNet3D:
         lr = float(s.lr if lr is None else lr)
         c1 = 1.0 - s.b1 ** s.t
         c2 = 1.0 - s.b2 ** s.t
-        wb = {}
+        wb, fused = {}, []                       # (p, g, m, v, bf16 copy or None) of one launch
         for k, p in self.params.items():
             g = grads[k]
             for st in (s.m, s.v):
@@ -415,14 +416,17 @@ class UNet3D:
                    and t.device == p.device for t in (p, g, m, v)):
                 if w:
                     wb[w] = torch.empty(p.shape, dtype=BF16, device=p.device)
-                _lib.call("ct_unet_adam", _tptr(p), _tptr(g), _tptr(m), _tptr(v), _p(wb.get(w)), p.numel(), s.b1, s.b2,
-                          c1, c2, lr, s.eps, _stream())
+                fused.append((p, g, m, v, wb.get(w)))
             else:
                 m.mul_(s.b1).add_(g, alpha=1 - s.b1)
                 v.mul_(s.b2).addcmul_(g, g, value=1 - s.b2)
                 p.addcdiv_(m / c1, (v / c2).sqrt_().add_(s.eps), value=-lr)
                 if w:
                     wb[w] = p.to(BF16).contiguous()
+        if fused:
+            cols = [(C.c_void_p * len(fused))(*[None if t is None else t.data_ptr() for t in col]) for col in zip(*fused)]
+            sizes = (C.c_longlong * len(fused))(*[t[0].numel() for t in fused])
+            _lib.call("ct_unet_adam", len(fused), *cols, sizes, s.b1, s.b2, c1, c2, lr, s.eps, _stream())
         self.wb, self.wt = wb, {}
 
 

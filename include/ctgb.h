@@ -399,10 +399,12 @@ int ct_unet_conv3d_wgrad(const void *d_xm, const void *d_x0, const void *d_xp, i
  * voxels. */
 int ct_unet_conv3d_wgrad_cl(const void *d_x1, int c1, const void *d_x2, int c2, const void *d_dy, int cout, int nb,
                             int nz, int ny, int nx, int ntaps, int kper, float *d_dw, void *stream);
-/* One Adam step of n FP32 parameters: m = b1 m + (1 - b1) g, v = b2 v + (1 - b2)
- * g^2, p -= lr (m / c1) / (sqrt(v / c2) + eps); wb, if not null, gets p in bf16. */
-int ct_unet_adam(float *d_p, const float *d_g, float *d_m, float *d_v, void *d_wb, long long n, double b1, double b2,
-                 double c1, double c2, double lr, double eps, void *stream);
+/* One Adam step of `count` FP32 tensors (host arrays of device pointers; tensor i has n[i] elements):
+ * m = b1 m + (1 - b1) g, v = b2 v + (1 - b2) g^2, p -= lr (m / c1) / (sqrt(v / c2) + eps); wb[i], if not null, gets
+ * p[i] in bf16. */
+int ct_unet_adam(int count, float *const *d_p, const float *const *d_g, float *const *d_m, float *const *d_v,
+                 void *const *d_wb, const long long *n, double b1, double b2, double c1, double c2, double lr,
+                 double eps, void *stream);
 /* bf16 weights [cout][taps][cin] to those of the data gradient, [cin][taps][cout] with the taps reversed. */
 int ct_unet_flip_weights(const void *d_w, void *d_out, int cout, int taps, int cin, void *stream);
 /* Reads and clears the device flag of the convolutions' bounded waits:
@@ -428,6 +430,9 @@ int ct_unet_conv_first(const float *d_vol, int nb, int nz, int ny, int nx, const
 int ct_unet_pool2(const void *d_in, void *d_out, int c, int nb, int nz, int ny, int nx, void *stream);
 int ct_unet_pool2_bwd(const void *d_x, const void *d_y, const void *d_dy, void *d_dx, int c, int nb, int nz, int ny,
                       int nx, void *stream);
+/* The same added to d_skip (dx's layout). */
+int ct_unet_pool2_bwd_add(const void *d_x, const void *d_y, const void *d_dy, const void *d_skip, void *d_dx, int c,
+                          int nb, int nz, int ny, int nx, void *stream);
 int ct_unet_up2(const void *d_in, void *d_out, int c, int nb, int nz, int ny, int nx, void *stream);
 int ct_unet_up2_bwd(const void *d_dout, void *d_din, int c, int nb, int nz, int ny, int nx, void *stream);
 /* Channel-major copies of a channels-last activation at channel offset coff

@@ -425,3 +425,29 @@ def test_conv_head_without_stored_activation(nb, nz, ny, nx, base):
     out = unet.conv3d_head(x, w, bias, True, hw, hb, b)
     assert unet.status() == 0
     assert torch.equal(out, unet.head(unet.conv3d(x, w, bias, relu=True), hw, hb, b))
+
+
+# one Adam launch for many tensors: more than one launch's table, sizes around a block's 1024 elements; against the
+# element-wise expressions (a dozen FP32 roundings apart).  Pooling gradient added to a skip gradient: the same bits as
+# the two passes.
+@pytest.mark.gpu
+def test_adam_of_many_tensors_and_pool_gradient_sum():
+    import torch
+    from ctgb import unet
+    g = torch.Generator(device="cuda").manual_seed(5)
+    sizes = [1, 3, 1023, 1024, 1025, 2048, 5000] * 8
+    net, twin = unet.UNet3D(), unet.UNet3D()
+    net.params = {f"{i}.w": torch.randn(n, device="cuda", generator=g) for i, n in enumerate(sizes)}
+    twin.params = {k: v.clone() for k, v in net.params.items()}
+    for _ in range(2):
+        gr = {k: torch.randn(v.shape, device="cuda", generator=g) for k, v in net.params.items()}
+        net.adam_step(gr, lr=1e-2)
+        twin.adam_step({k: torch.stack((v, v), -1)[..., 0] for k, v in gr.items()}, lr=1e-2)
+    for k, v in net.params.items():
+        assert bool(((v - twin.params[k]).abs() <= 24 * 2.0 ** -24 * (v.abs() + 1)).all()), k
+        assert torch.equal(net.wb[k[:-2]], v.to(torch.bfloat16))
+    x = torch.relu(torch.randn((2, 4, 6, 8, 40), device="cuda", generator=g)).to(torch.bfloat16)
+    y = unet.pool2(x)
+    dy = torch.randn(y.shape, device="cuda", generator=g).to(torch.bfloat16)
+    skip = torch.randn(x.shape, device="cuda", generator=g).to(torch.bfloat16)
+    assert torch.equal(unet.pool2_bwd(x, y, dy, skip), skip + unet.pool2_bwd(x, y, dy))
