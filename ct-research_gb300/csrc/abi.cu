@@ -212,7 +212,7 @@ using namespace ct;
 struct ct_cone_plan {
     ConeGeom g{};
     DevBuf trig, vsrc, P, xi, xtab, vorder, trigf, vsrcf, Pd, xid;
-    DevBuf pairs, bptab, rcov, G, wtab, norms, volT, volS, cols, pwt, win, scan, bpsum;
+    DevBuf pairs, rcov, G, wtab, norms, volT, volS, cols, pwt, win, scan, bpsum;
     double cols_res[3] = {0, 0, 0};   // voxel pitch the column table was built for
     GrazeBuf graze;
     int bp_chunk = 0;   // views per backprojection chunk; 0: automatic (cone_bp_chunk_views)
@@ -226,7 +226,7 @@ struct ct_cone_plan {
     ~ct_cone_plan() {
         trig.release(); vsrc.release(); P.release(); xi.release(); xtab.release(); vorder.release();
         trigf.release(); vsrcf.release(); Pd.release(); xid.release();
-        pairs.release(); bptab.release(); rcov.release(); G.release(); wtab.release(); norms.release(); graze.release();
+        pairs.release(); rcov.release(); G.release(); wtab.release(); norms.release(); graze.release();
         volT.release(); volS.release(); cols.release(); pwt.release(); win.release(); scan.release(); bpsum.release();
     }
 };
@@ -424,7 +424,7 @@ int ct_cone_plan_set_short_scan(ct_cone_plan *plan, int enable) {
 
 size_t ct_cone_plan_workspace_bytes(const ct_cone_plan *plan) {
     if (!plan) return 0;
-    return plan->pairs.bytes + plan->bptab.bytes + plan->rcov.bytes + plan->G.bytes + plan->wtab.bytes + plan->norms.bytes +
+    return plan->pairs.bytes + plan->rcov.bytes + plan->G.bytes + plan->wtab.bytes + plan->norms.bytes +
            plan->graze.buf.bytes + plan->volT.bytes + plan->volS.bytes + plan->cols.bytes + plan->bpsum.bytes;
 }
 
@@ -513,6 +513,15 @@ static int cone_bp_table_views(const ct_cone_plan *plan, int chunk) {
     return (int)std::max<size_t>(1, std::min<size_t>(chunk, kBpTableBytes / per_view));
 }
 
+// The workspace of a chunk of views: its pairs and, behind them, its records (one
+// allocation: a plan's first backprojection waits for it).
+static int cone_bp_work(ct_cone_plan *plan, int chunk, void **tab) {
+    const size_t pairs = (cone_bp_pairs_bytes(plan->g, chunk) + 255) & ~static_cast<size_t>(255);
+    if (int s = plan->pairs.ensure(pairs + cone_bp_table_bytes(plan->g, chunk))) return s;
+    *tab = plan->pairs.as<char>() + pairs;
+    return CT_OK;
+}
+
 // Backprojection in chunks of cone_bp_chunk_views views (fewer where their
 // records would not fit): every chunk is packed into pairs and backprojected,
 // its sums added to the volume (or, for the fused SIRT update, to a partial-sum
@@ -524,8 +533,8 @@ static int cone_bp_common(ct_cone_plan *plan, const float *d_proj, float *d_vol,
     const int chunk = cone_bp_table_views(plan, cone_bp_chunk_views(plan));
     const int nchunks = (g.nb + chunk - 1) / chunk;
     int s;
-    if ((s = plan->pairs.ensure(cone_bp_pairs_bytes(g, chunk))) || (s = plan->bptab.ensure(cone_bp_table_bytes(g, chunk))))
-        return s;
+    void *tab;
+    if ((s = cone_bp_work(plan, chunk, &tab))) return s;
     float *part = nullptr;
     if (update && nchunks > 1) {
         if ((s = plan->bpsum.ensure(sizeof(float) * (size_t)g.nt * g.ns * g.nz))) return s;
@@ -537,7 +546,7 @@ static int cone_bp_common(ct_cone_plan *plan, const float *d_proj, float *d_vol,
         if ((s = cone_bp_pack(g, d_proj, plan->pairs.as<float2>(), v0, nv, st))) return s;
         const float *prev = c == 0 ? nullptr : (update ? part : d_vol);
         float *out = (update && !last) ? part : d_vol;
-        if ((s = cone_bp_launch(g, plan->pairs.as<float2>(), plan->bptab.ptr, false, v0, nv, prev, out, weighting, colsum,
+        if ((s = cone_bp_launch(g, plan->pairs.as<float2>(), tab, false, v0, nv, prev, out, weighting, colsum,
                                 eps, lambda, lo, hi, update && last, st)))
             return s;
     }
@@ -1070,9 +1079,8 @@ static int cone_bp_dropin(float *Display, const float *R, const float *xi, const
         const int nchunks = (nb + bchunk - 1) / bchunk;
         const int ztile = cone_bp_ztile(pl->g), ntiles = (nz + ztile - 1) / ztile;
         const int nslab = std::min(kDropinSlabs, ntiles);
-        if ((s = dropin_streams(st, nchunks + nslab)) || (s = pl->pairs.ensure(cone_bp_pairs_bytes(pl->g, bchunk))) ||
-            (s = pl->bptab.ensure(cone_bp_table_bytes(pl->g, bchunk))))
-            return s;
+        void *tab;
+        if ((s = dropin_streams(st, nchunks + nslab)) || (s = cone_bp_work(pl, bchunk, &tab))) return s;
         const size_t per_view = (size_t)np * nx;
         for (int c = 0; c < nchunks; ++c) {
             const int v0 = c * bchunk, n = std::min(bchunk, nb - v0);
@@ -1088,7 +1096,7 @@ static int cone_bp_dropin(float *Display, const float *R, const float *xi, const
             if ((s = cone_bp_pack(pl->g, st.proj.as<float>(), pl->pairs.as<float2>(), v0, n, st.cs))) return s;
             for (int k = 0; k < (last ? nslab : 1); ++k) {
                 const int t0 = last ? k * ntiles / nslab : 0, t1 = last ? (k + 1) * ntiles / nslab : ntiles;
-                if ((s = cone_bp_launch(pl->g, pl->pairs.as<float2>(), pl->bptab.ptr, k > 0, v0, n,
+                if ((s = cone_bp_launch(pl->g, pl->pairs.as<float2>(), tab, k > 0, v0, n,
                                         c == 0 ? nullptr : st.vol.as<float>(), st.vol.as<float>(), 0, nullptr, 0.f, 0.f,
                                         0.f, 0.f, false, st.cs, t0, t1 - t0)))
                     return s;

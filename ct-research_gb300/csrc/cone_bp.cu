@@ -45,15 +45,23 @@ constexpr int BP_BX = 32;          // t per block (one warp)
 constexpr int BP_BY = 4;           // s per block
 // z per thread (register accumulators) and the blocks per SM its registers aim at.
 // 32 z share a column-view's record best: 45.2 ms at 512^3 / 360 views and 4 blocks
-// (57 at 5, 50 at 6), 47.7 with 16 z and 8 blocks; where 32 z leave the GPU with
-// few waves of blocks 16 z fill it (SIRT3D of 151 x 133 x 97: 5.2 -> 3.8 ms).
-constexpr int kZLong = 32, kZShort = 16;
-constexpr int bp_min_blocks(int zc) { return zc == kZLong ? 4 : 8; }
+// (57 at 5, 50 at 6), 47.7 with 16 z and 8 blocks.  A thread sums its views one after
+// the other, so a small scan, whose blocks do not fill the GPU several times over, takes
+// fewer z per thread: more threads, and fewer of them off the fast path at the
+// ends of a column.  us of a backprojection with 16 / 8 / 4 z: 150 x 140 x 110 and 120
+// views (1225 blocks at 16 z) 839 / 519 / 610; 64 x 60 x 50 and 90 views (210 at
+// 8 z) 434 / 196 / 78; of an FDK of 180 x 170 x 140 and 120 views (2322 at 16 z) 877 / 908
+// with 16 / 8 z, of 80 x 70 x 50 and 200 views (378 at 8 z) 517 / 222 / 219.  The lines lie
+// between these.  At 8 z, 4 / 5 / 6 / 8 blocks: SIRT3D of 151 x 133 x 97 in 3.33 / 3.37 /
+// 3.42 / 3.48 ms (3.81 with 16 z).
+constexpr int kZLong = 32, kZShort = 16, kZTiny = 8, kZLeast = 4;
+constexpr int bp_min_blocks(int zc) { return zc == kZShort ? 8 : 4; }
 
 int bp_zc(const ConeGeom &g) {
-    const long long blocks = (long long)((g.nt + BP_BX - 1) / BP_BX) * ((g.ns + BP_BY - 1) / BP_BY) *
-                             ((g.nz + kZLong - 1) / kZLong);
-    return blocks < 3LL * bp_min_blocks(kZLong) * sm_count() ? kZShort : kZLong;
+    const long long cols = (long long)((g.nt + BP_BX - 1) / BP_BX) * ((g.ns + BP_BY - 1) / BP_BY), sms = sm_count();
+    if (cols * ((g.nz + kZLong - 1) / kZLong) >= 12 * sms) return kZLong;
+    if (cols * ((g.nz + kZShort - 1) / kZShort) >= 12 * sms) return kZShort;
+    return cols * ((g.nz + kZTiny - 1) / kZTiny) >= 3 * sms ? kZTiny : kZLeast;
 }
 
 // Pairs of n consecutive samples; the last sample of a row pairs with 0.
@@ -578,9 +586,11 @@ int cone_bp_launch(const ConeGeom &g, const float2 *Q, void *tab, bool tab_ready
 #define CT_BP_RUN(W, U, Z)                                                                                        \
     cone_bp_kernel<W, U, Z><<<grid, block, smem, st>>>(gk, Q, ta, tb, v0, nv, prev, out, colsum, eps, lambda, lo, \
                                                        hi, t, zbase)
-#define CT_BP_CASE(W, U)                     \
+#define CT_BP_CASE(W, U)                            \
     if (zc == kZLong) CT_BP_RUN(W, U, kZLong); \
-    else CT_BP_RUN(W, U, kZShort)
+    else if (zc == kZShort) CT_BP_RUN(W, U, kZShort); \
+    else if (zc == kZTiny) CT_BP_RUN(W, U, kZTiny); \
+    else CT_BP_RUN(W, U, kZLeast)
         if (update) {
             if (weighting == W_CHORD) { CT_BP_CASE(W_CHORD, true); }
             else if (weighting == W_FDK_ZERO) { CT_BP_CASE(W_FDK_ZERO, true); }

@@ -451,3 +451,13 @@ def test_adam_of_many_tensors_and_pool_gradient_sum():
     dy = torch.randn(y.shape, device="cuda", generator=g).to(torch.bfloat16)
     skip = torch.randn(x.shape, device="cuda", generator=g).to(torch.bfloat16)
     assert torch.equal(unet.pool2_bwd(x, y, dy, skip), skip + unet.pool2_bwd(x, y, dy))
+
+
+# 8 z per thread (enough blocks at 8, too few at 16), a last tile of one and of three slices, and 4 z with a last tile
+# of one: the bounds of the other tile sizes' test above
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,views,det,rows,down,dist", [
+    ((100, 100, 41), 5, (130, 60), 0.9, False, 3.0), ((97, 101, 43), 4, (120, 90), 1.4, True, 3.0),
+    ((40, 30, 9), 6, (60, 24), 0.8, False, 2.0)])
+def test_cone_backprojection_small_scans(oracle, shape, views, det, rows, down, dist):
+    test_cone_backprojection_tiles_and_row_steps(oracle, shape, views, det, rows, down, dist)
