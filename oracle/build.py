@@ -112,7 +112,7 @@ def _extract_device_consts(text: str) -> list[str]:
 def build_ref(force: bool = False) -> list[Path]:
     """Compile the reference kernels as host code into oracle/_ref/ (checker only)."""
     root = reference_root()
-    if not root.is_dir():
+    if not root.is_dir() or not any(root.iterdir()):   # absent, or a mount point with nothing in it
         return []
     REF_OUT.mkdir(exist_ok=True)
     shim = (HERE / "shim" / "cuda_host_shim.h").read_text()
