@@ -367,7 +367,7 @@ colsum8_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long 
 // One Adam step of many parameters and their bf16 copies (null: none), 1024
 // elements of one of them per block.  Twelve element-wise passes per parameter in
 // one launch for all: bound by memory at the large parameters, and the small ones
-// (biases of 32 to 256) share its launch.
+// (biases of 32 to 256) share its launch.  Its roundings are those of the twelve passes.
 constexpr int kAdamTensors = 48, kAdamBlock = 1024;
 
 struct AdamArgs {
@@ -394,7 +394,7 @@ adam_kernel(const __grid_constant__ AdamArgs a) {
     for (int u = 0; u < kAdamBlock / 256; ++u) {
         const long long i = i0 + u * 256;
         if (i >= a.n[t]) break;
-        const float gi = g[i], mi = fmaf(a.a1, gi, m[i] * a.b1), vi = fmaf(a.a2 * gi, gi, v[i] * a.b2);
+        const float gi = g[i], mi = fmaf(a.a1, gi, m[i] * a.b1), vi = fmaf(a.a2, gi * gi, v[i] * a.b2);
         const float pi = fmaf(-a.lr, (mi * a.inv1) / (sqrtf(vi * a.inv2) + a.eps), p[i]);
         m[i] = mi;
         v[i] = vi;
