@@ -302,15 +302,24 @@ head_bwd_kernel(const float *__restrict__ dout, const bf16 *__restrict__ f, cons
     }
 }
 
-// db[c] += sum_v dy[v][c]; block of 256 threads = 256 / c voxel lanes x c channels
+// db[c] += sum_v dy[v][c]; block of 256 threads = 256 / c voxel lanes x c channels.  A
+// thread adds its voxels in order and lane 0 the lanes in order: Adam divides a
+// gradient by its own size, so another order of these sums shows in later steps.
 __global__ void __launch_bounds__(256)
 colsum_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long long nvox) {
     const int lanes = 256 / c;
     const int ch = threadIdx.x % c, l = threadIdx.x / c;
+    const long long step = static_cast<long long>(gridDim.x) * lanes;
     float s = 0.0f;
-    for (long long v = blockIdx.x * static_cast<long long>(lanes) + l; v < nvox;
-         v += static_cast<long long>(gridDim.x) * lanes)
-        s += __bfloat162float(dy[v * c + ch]);
+    long long v = blockIdx.x * static_cast<long long>(lanes) + l;
+    for (; v + 7 * step < nvox; v += 8 * step) {           // eight loads in flight
+        bf16 q[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) q[u] = dy[(v + u * step) * c + ch];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += __bfloat162float(q[u]);
+    }
+    for (; v < nvox; v += step) s += __bfloat162float(dy[v * c + ch]);
     __shared__ float red[256];
     red[threadIdx.x] = s;
     __syncthreads();
@@ -318,50 +327,6 @@ colsum_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long l
         for (int k = 1; k < lanes; ++k) s += red[k * c + ch];
         atomicAdd(db + ch, s);
     }
-}
-
-// The same where a voxel's channels come in whole 16-byte groups: 8 channels per
-// thread, lanes of a block summed in a tree, one atomic per block and channel
-// with a block's channels side by side (a thread adding its 8 itself makes eight
-// times the requests: 56 us instead of 15 for 64 channels).  128^3 x 32 channels
-// (134 MB): 35 us against 43 with 2-byte loads; 64^3 x 128: 5.7 against 9.3.
-__global__ void __launch_bounds__(256)
-colsum8_kernel(const bf16 *__restrict__ dy, float *__restrict__ db, int c, long long nvox) {
-    const int c8 = c / 8, lanes = 256 / c8;
-    const int g = threadIdx.x % c8, l = threadIdx.x / c8;
-    float s[8] = {};
-    const uint4 *src = reinterpret_cast<const uint4 *>(dy) + g;
-    const long long step = static_cast<long long>(gridDim.x) * lanes;
-    long long v = blockIdx.x * static_cast<long long>(lanes) + l;
-    for (; v + 3 * step < nvox; v += 4 * step) {           // four loads in flight
-        uint4 q[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = __ldg(src + (v + u * step) * c8);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            float f[8];
-            unpack8(q[u], f);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) s[j] += f[j];
-        }
-    }
-    for (; v < nvox; v += step) {
-        float f[8];
-        unpack8(__ldg(src + v * c8), f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s[j] += f[j];
-    }
-    __shared__ float red[8][256];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[j][threadIdx.x] = s[j];
-    for (int h = lanes / 2; h > 0; h /= 2) {
-        __syncthreads();
-        if (l < h)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) red[j][threadIdx.x] += red[j][threadIdx.x + h * c8];
-    }
-    __syncthreads();
-    if (threadIdx.x < c) atomicAdd(db + threadIdx.x, red[threadIdx.x % 8][threadIdx.x / 8]);   // whole lines at once
 }
 
 // One Adam step of many parameters and their bf16 copies (null: none), 1024
@@ -544,14 +509,6 @@ int ct_unet_colsum(const void *dy, int c, long long nvox, float *db, void *strea
     CT_REQUIRE(dy && db, "colsum: null pointer");
     CT_REQUIRE(c > 0 && c <= 256 && 256 % c == 0, "colsum: channels must divide 256");
     CT_REQUIRE(nvox > 0, "colsum: bad voxel count");
-    if (c % 8 == 0 && al16(dy)) {
-        // about four voxels per lane and block at least: an atomic per block and channel
-        const unsigned blocks = static_cast<unsigned>(
-            std::min<long long>((nvox + 1024LL / (c / 8) - 1) / (1024 / (c / 8)), 8LL * sm_count()));
-        colsum8_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const bf16 *>(dy), db, c, nvox);
-        CT_LAUNCH_CHECK("colsum8_kernel");
-        return CT_OK;
-    }
     const long long lanes = 256 / c;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((nvox + lanes - 1) / lanes, 8LL * sm_count()));
     colsum_kernel<<<grid, 256, 0, as_stream(stream)>>>(static_cast<const bf16 *>(dy), db, c, nvox);

@@ -5,6 +5,21 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+# One block of the channel sums: its voxels added one after the other, in FP32
+@pytest.mark.parametrize("c", [8, 32, 64, 128])
+def test_channel_sums_keep_their_order(c):
+    import torch
+    from ctgb import unet
+    g = torch.Generator(device="cuda").manual_seed(c)
+    x = torch.randn((256 // c, c), device="cuda", generator=g).to(torch.bfloat16)
+    db = torch.zeros(c, device="cuda")
+    unet.colsum(x, db)
+    ref = torch.zeros(c, device="cuda")
+    for row in x.float():
+        ref = ref + row
+    assert torch.equal(db, ref)
+
+
 # The fused Adam pass is bit for bit torch's expressions
 def test_adam_bits():
     import torch
