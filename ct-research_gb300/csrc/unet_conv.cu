@@ -18,7 +18,8 @@
 //   filters in shared memory and reads each input slice once.
 // * conv_first_kernel: the one-channel input's 27 taps built in shared memory.
 // * conv_wgrad_cl_kernel (weight gradient): the channels-last tensors as they
-//   are, see below.  conv_wgrad_kernel, for volumes that its tiles do not fit:
+//   are, see below.  conv_wgrad_kernel, for volumes that its segments do not fit
+//   and for 128 x 128 channels and more:
 //   rows = (tap, input channel), columns = output channels, K = voxels in
 //   64-voxel slices (128-byte rows, 128-byte swizzle).  Activations and output
 //   gradients are read channel-major [n][c][z][y*x]; x offsets come from three
@@ -1035,37 +1036,36 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap mxm, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------
-// Weight gradient straight from channels-last tensors, 32 input x 32 output
-// channels per CTA.
+// Weight gradient straight from channels-last tensors: 32 input x 32 output
+// channels and the nine taps of one dz per item.
 //
 // conv_wgrad_kernel wants its K dimension (voxels) contiguous, so the tensors
-// are first copied channel-major, X three times; each of its boxes then
-// gathers 128-byte rows that lie a whole volume apart, and 4 taps x 32 channels against
-// 32 outputs need 7 passes over the volume.  Here the 8 x 16 voxel tiles of the
-// channels-last tensors are the operands as they are (MN-major: 32 channels of
-// a voxel contiguous, voxels along K).  M = 3 boxes of X, one per dx, of 32 channels each (a fourth
-// quarter of M reads what follows them and is dropped); N = the three
-// dy: three atoms that start one tile row (8 voxels, 512 bytes) apart in one
-// box of dY with a halo row on either side.  A CTA walks its columns along z and multiplies X of
-// slice z by dY of z + 1, z, z - 1 into three accumulators (dz = -1, 0, 1): each
-// slice of either tensor is fetched once per column, all 27 taps from 34 KB per 128 voxels
-// instead of 280.  X is zero outside the volume, so every tap's sum over
-// the tiles of X is complete.
+// are first copied channel-major, X three times, and each of its boxes gathers
+// 128-byte rows that lie a whole volume apart.  Here the channels-last tensors are the
+// operands as they are (MN-major: 32 channels of a voxel contiguous, voxels along
+// K).  A K step is 16 consecutive voxels of X.  M = 3 boxes of X, one per dx, of 32 channels
+// each (a fourth quarter of M reads what follows them and is dropped); N = the
+// three dy: the voxels of dY one row before, at and one row after those of X, which
+// lie one row apart in a ring of dY.  (Its first two rows are fetched a second time
+// behind its end: a product split at the end costs 88 cycles of operand reads
+// instead of 56, in 4 of 7 steps of 128-voxel rows.)  The CTA walks X in memory order in
+// segments (rows or parts of one), so each row of either tensor is fetched once per dz.
 //
-// Partial sums are added to dw after every `flush` tiles, so an FP32 sum is as long
-// as with conv_wgrad_kernel's kper, and its error is the same (128^3: 1.88e-6
-// of the norm for both, 32^3: 2.1e-7 against 7.8e-7).
+// The sums are conv_wgrad_kernel's: a partial sum takes the same kper * 64 voxels of
+// dY, every tap meets them in the same order and groups of 16, and it is added
+// to dw the same way.  Adam divides a gradient by its own size, so a weight whose
+// gradient is near zero follows its last bits, and one bf16 weight more or less
+// moves the next step's gradients by 1e-3 of their norm.  (8 x 16 voxel tiles walked
+// along z, with one fetch of X for all dz, took three quarters of the time, but sum in
+// another order.)
 //
-// GB300, with the copies that conv_wgrad_kernel needs (before / after): 128^3,
-// 32 x 32 channels 948 / 125 us, 64 x 32 1805 / 232, 64 x 64 2291 / 444; 64^3, 64 x 64 138 / 81,
-// 128 x 128 328 / 274, 256 x 128 595 / 566; 32^3, 256 x 256 164 / 157.  No channel count was found
-// at which the copies pay, so conv_wgrad_kernel only serves volumes whose y is
-// not a multiple of the tile's 16.  What remains is the issuing thread's
-// waits and commits (about as long as the 24 instructions of 56 cycles per
-// tile) and, at many channels, 3 of 4 useful rows.
+// Bound by shared memory: 224 cycles of operand reads and 140 of TMA writes per 64
+// voxels of one dz.  GB300, with the copies that conv_wgrad_kernel needs (before /
+// after): 128^3, 32 x 32 channels 935 / 161 us, 64 x 32 1789 / 296; 64^3, 64 x 64 131 / 86,
+// 128 x 64 225 / 162; 32^3, 64 x 128 40 / 35, but 128 x 128 54 / 59 (there every row of
+// conv_wgrad_kernel's products is of use); 16^3, 256 x 256 38 / 53.
 // ---------------------------------------------------------------------------
-constexpr int kClStages = 6;
-constexpr uint32_t kClBox = kYBx * kYBy * kRowBytes;       // 128 voxels x 32 channels
+constexpr int kClStages = 16;
 
 struct ClCtrl {
     uint64_t full[kClStages];
@@ -1077,38 +1077,32 @@ struct ClCtrl {
 };
 
 struct ClArgs {
-    int c1, cin, cout;
-    int nz, tx, ty;
-    int zc, nzc;             // slices per item, items along z
-    int flush;               // tiles per partial sum
-    long long items;
+    int c1, cin, nz;
+    int seg, bx, by;         // K steps of a segment; its x and y extent
+    int nseg, spp;           // segments side by side along x, and per plane
+    int boxes;               // 32-channel boxes of X per stage: the three dx, or (one tap) channel chunks
+    int stages;              // of X
+    int steps, chain;        // K steps of the volume and of a partial sum
+    int items;
     float *dw;               // [cout][taps][cin], FP32, accumulated
 };
 
-template <int TAPS>
-__host__ __device__ constexpr uint32_t cl_stage() {
-    return TAPS == 27 ? 3 * kClBox + kYABytes : 2 * kClBox;
-}
-
-template <int TAPS>
-constexpr size_t cl_smem() {
-    return 1024 + kClStages * cl_stage<TAPS>() + sizeof(ClCtrl);
-}
-
-// grid (CTAs, 32-channel chunks of X, 32-channel chunks of dY)
+// grid (CTAs, 32-channel chunks of X (`boxes` of them for one tap), 32-channel chunks of dY)
 template <int TAPS>
 __global__ void __launch_bounds__(192, 1)
 conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mx2,
                      const __grid_constant__ CUtensorMap mdy, const ClArgs a) {
-    constexpr int S = kClStages, NZ = TAPS == 27 ? 3 : 1, NX = NZ;   // dz blocks, boxes of X
-    constexpr int N = 32 * NZ, H = TAPS == 27 ? 1 : 0;               // columns of a block, halo of dY
-    constexpr uint32_t stage = cl_stage<TAPS>(), xbytes = NX * kClBox, dbytes = stage - xbytes;
-    constexpr uint32_t cols = TAPS == 27 ? 512 : 32;
+    constexpr int NZ = TAPS == 27 ? 3 : 1;                 // dz per partial sum, dy per item
+    constexpr uint32_t cols = TAPS == 27 ? 128 : 32;       // 32 NZ used
     extern __shared__ uint8_t smem_raw[];
     uint8_t *ring = align1024(smem_raw);
-    ClCtrl *c = reinterpret_cast<ClCtrl *>(ring + S * stage);
+    const int h = TAPS == 27 ? a.nseg : 0;                 // segments from a voxel to the next row's
+    const int S = a.stages, W = S + 2 * h;                 // stages of X, segments in the ring of dY (and 2 h twice)
+    const uint32_t box = a.seg * 16 * kRowBytes, xstage = a.boxes * box;
+    uint8_t *yring = ring + S * xstage;
+    ClCtrl *c = reinterpret_cast<ClCtrl *>(yring + (W + 2 * h) * box);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int ci0 = blockIdx.y * 32, co0 = blockIdx.z * 32;
+    const int ci0 = blockIdx.y * 32 * (TAPS == 27 ? 1 : a.boxes), co0 = blockIdx.z * 32;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
@@ -1116,7 +1110,7 @@ conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_const
             mbar_init(&c->empty[s], 1);
         }
         mbar_init(&c->accfull, 1);
-        for (int j = 0; j < 3; ++j) mbar_init(&c->accempty[j], NX);
+        for (int e = 0; e < NZ; ++e) mbar_init(&c->accempty[e], a.boxes);
         mbar_init(&c->done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1126,44 +1120,61 @@ conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_const
     tc_fence_after();
     const uint32_t tmem = c->tmem;
 
-    // item i: slices z0 .. z1 - 1 of a tile column
-    auto item = [&](long long i, int &x0, int &y0, int &z0, int &z1, int &n) {
-        x0 = static_cast<int>(i % a.tx) * kYBx;
-        i /= a.tx;
-        y0 = static_cast<int>(i % a.ty) * kYBy;
-        i /= a.ty;
-        z0 = static_cast<int>(i % a.nzc) * a.zc;
-        z1 = min(z0 + a.zc, a.nz);
-        n = static_cast<int>(i / a.nzc);
+    // item i: K steps v0 .. v1 - 1 of dY in memory order, the taps of one dz
+    auto item = [&](int i, int &v0, int &v1) {
+        v0 = i / NZ * a.chain;
+        v1 = min(v0 + a.chain, a.steps);
+        return TAPS == 27 ? i % 3 - 1 : 0;
     };
-    int x0, y0, z0, z1, n;
+    // Its segments ka .. kb - 1 of one plane, from segment sg of all planes.  The steps of such a run are the
+    // segments k of X from ka - h to kb - 1 + h; dY of segment k + h comes with X of segment k.
+    auto run = [&](int sg, int v1, int &plane, int &ka, int &kb) {
+        plane = sg / a.spp;
+        ka = sg - plane * a.spp;
+        kb = min((v1 + a.seg - 1) / a.seg - plane * a.spp, a.spp);
+    };
+    int v0, v1, plane, ka, kb;
 
     if (warp == 4) {
-        int s = 0, used = 0;                               // stage, stages filled so far (up to S)
+        int s = 0, used = 0, w = 0;                        // stage, stages filled so far (up to S), slot of dY
         uint32_t ph = 0;
         bool ok = true;
-        for (long long i = blockIdx.x; ok && i < a.items; i += gridDim.x) {
-            item(i, x0, y0, z0, z1, n);
-            for (int z = z0 - H; z < z1 + H; ++z) {        // stage: dY of slice z, X of it where it is the item's
-                if (used == S) ok = __all_sync(0xffffffffu, mbar_wait(&c->empty[s], ph ^ 1));
-                if (!ok) break;
-                if (elect_one()) {
-                    const bool x = z >= z0 && z < z1;
-                    uint8_t *sa = ring + s * stage;
-                    mbar_expect_tx(&c->full[s], dbytes + (x ? xbytes : 0));
-                    tma_load5(sa + xbytes, &mdy, &c->full[s], co0, x0, y0 - H, z, n);
-                    if (x) {
-#pragma unroll
-                        for (int j = 0; j < NX; ++j)
-                            tma_load5(sa + j * kClBox, ci0 < a.c1 ? &mx1 : &mx2, &c->full[s],
-                                      ci0 < a.c1 ? ci0 : ci0 - a.c1, x0 + j - H, y0, z, n);
+        for (int i = blockIdx.x; ok && i < a.items; i += gridDim.x) {
+            const int dz = item(i, v0, v1);
+            for (int sg = v0 / a.seg; ok && sg * a.seg < v1; sg += kb - ka) {
+                run(sg, v1, plane, ka, kb);
+                const int n = plane / a.nz, z = plane - n * a.nz;
+                int row = (ka - h + a.nseg) / a.nseg - 1;  // ka - h >= -nseg
+                int x0 = (ka - h - row * a.nseg) * a.bx, y0 = row * a.by;
+                for (int k = ka - h; k < kb + h; ++k) {
+                    // step k's stage is free: so is the slot, whose dY the step before that stage's was the last to read
+                    if (used == S) ok = __all_sync(0xffffffffu, mbar_wait(&c->empty[s], ph ^ 1));
+                    if (!ok) break;
+                    if (elect_one()) {
+                        const bool dy = k + h >= ka && k + h < kb, twice = dy && w < 2 * h;
+                        mbar_expect_tx(&c->full[s], xstage + (dy ? box : 0) + (twice ? box : 0));
+                        for (int j = 0; j < a.boxes; ++j) {
+                            const int ch = TAPS == 27 ? ci0 : ci0 + 32 * j;
+                            const bool second = ch >= a.c1;
+                            tma_load5(ring + s * xstage + j * box, second ? &mx2 : &mx1, &c->full[s],
+                                      second ? ch - a.c1 : ch, TAPS == 27 ? x0 + j - 1 : x0, y0, z + dz, n);
+                        }
+                        const int yd = TAPS == 27 ? y0 + a.by : y0;
+                        if (dy) tma_load5(yring + w * box, &mdy, &c->full[s], co0, x0, yd, z, n);
+                        if (twice) tma_load5(yring + (W + w) * box, &mdy, &c->full[s], co0, x0, yd, z, n);
                     }
-                }
-                __syncwarp();
-                used = min(used + 1, S);
-                if (++s == S) {
-                    s = 0;
-                    ph ^= 1;
+                    __syncwarp();
+                    x0 += a.bx;
+                    if (x0 == a.nseg * a.bx) {
+                        x0 = 0;
+                        y0 += a.by;
+                    }
+                    used = min(used + 1, S);
+                    if (++w == W) w = 0;
+                    if (++s == S) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
             }
         }
@@ -1171,90 +1182,97 @@ conv_wgrad_cl_kernel(const __grid_constant__ CUtensorMap mx1, const __grid_const
         // every load has landed before the CTA may leave: the last use of stage j
         for (int j = 0; j < used; ++j) mbar_wait(&c->full[j], j < s ? ph : ph ^ 1);
     } else if (warp == 5) {
-        const uint64_t xd = sw64_mn_desc(smem_u32(ring), TAPS == 27 ? kClBox : 512);
-        const uint64_t yd = sw64_mn_desc(smem_u32(ring) + xbytes, 512);
-        int s = 0, p1 = 0, p2 = 0;                         // stages of this slice and the two before it
-        int tiles = 0;                                     // since the last partial sum was handed over
+        // in K steps (1024 bytes): a row, and the part of it in a segment
+        const int row = a.nseg * a.bx / 16, line = a.bx / 16;
+        const uint64_t xd = sw64_mn_desc(smem_u32(ring), a.boxes > 1 ? box : 512);
+        const uint64_t yd = sw64_mn_desc(smem_u32(yring), row * 1024);
+        int s = 0, w = 0;
         uint32_t ph = 0, sums = 0;
         bool ok = true;
-        for (long long i = blockIdx.x; ok && i < a.items; i += gridDim.x) {
-            item(i, x0, y0, z0, z1, n);
-            for (int z = z0 - H; z < z1 + H; ++z) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&c->full[s], ph));
-                if (!ok) break;
-                const int zx = z - H;                      // the slice of X that has all its dY now
-                if (zx >= z0) {
+        for (int i = blockIdx.x; ok && i < a.items; i += gridDim.x) {
+            item(i, v0, v1);
+            for (int sg = v0 / a.seg; ok && sg * a.seg < v1; sg += kb - ka) {
+                run(sg, v1, plane, ka, kb);
+                const int pv = plane * a.spp * a.seg;                  // the plane's first K step
+                const bool start = v0 >= pv;                           // the sum starts in this run
+                const int pa = start ? v0 - pv : 0, pb = min(v1 - pv, a.spp * a.seg);   // the sum's dY in this plane
+                for (int k = ka - h; k < kb + h; ++k) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&c->full[s], ph));
+                    if (!ok) break;
                     tc_fence_after();
+                    const uint64_t xb = xd + static_cast<uint64_t>(s) * (xstage / 16);
+                    const int y0 = (w >= h ? w - h : w - h + W) * a.seg;   // where dY of the same voxels is
+                    // the segment's rows (or part of one): what holds for a row's first K step holds for all.  dY of
+                    // p + (e - 1) row is met for dy = 1 - e.
+                    for (int r = 0; r < a.seg; r += line) {
+                        const int p = k * a.seg + r;
+                        int e = TAPS == 1 ? 1 : (p >= pa + row ? 0 : (p >= pa ? 1 : (p >= pa - row ? 2 : 3)));
+                        const int ee = TAPS == 1 ? 2 : (p + row < pb ? 3 : (p < pb ? 2 : (p - row < pb ? 1 : 0)));
+                        while (e < ee) {
+                            // a sum's first K step for e starts its accumulator, once it has been read
+                            const bool first = start && p + (e - 1) * row == pa;
+                            if (first && sums)
+                                ok = __all_sync(0xffffffffu, mbar_wait(&c->accempty[TAPS == 1 ? 0 : e], (sums - 1) & 1));
+                            if (!ok) break;
+                            tc_fence_after();
+                            const int len = first ? 1 : ee - e;
+                            const int y = y0 + r + (e - 1) * row;
+                            if (elect_one()) {
+                                const uint64_t xg = xb + r * 64, yg = yd + (y < 0 ? y + W * a.seg : y) * 64;
+                                const uint32_t d = tmem + (TAPS == 1 ? 0 : e * 32);
+                                const uint32_t id = idesc_bf16_mn(kTileM, 32) + (len - 1) * (4u << 17);
 #pragma unroll
-                    for (int j = 0; j < NZ; ++j) {         // dz = j - 1: dY of slice zx - dz
-                        if (tiles == 0 && sums) ok = __all_sync(0xffffffffu, mbar_wait(&c->accempty[j], (sums - 1) & 1));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-                            const int sx = H ? p1 : s, sy = H ? (j == 0 ? s : (j == 1 ? p1 : p2)) : s;
-                            const uint64_t ad = xd + static_cast<uint64_t>(sx) * (stage / 16);
-                            const uint64_t bd = yd + static_cast<uint64_t>(sy) * (stage / 16);
-#pragma unroll
-                            for (int kk = 0; kk < kYBx * kYBy / 16; ++kk)
-                                umma_bf16(tmem + j * N, ad + kk * 64, bd + kk * 64, idesc_bf16_mn(kTileM, N),
-                                          tiles | kk);
+                                for (int g = 0; g < 4; ++g)
+                                    if (g < line) umma_bf16(d, xg + g * 64, yg + g * 64, id, g > 0 || !first);
+                            }
+                            __syncwarp();
+                            e += len;
                         }
-                        __syncwarp();
+                        if (!ok) break;
                     }
                     if (!ok) break;
-                    const bool last = zx == z1 - 1, full = ++tiles == a.flush || (last && i + gridDim.x >= a.items);
                     if (elect_one()) {
-                        if (H) {
-                            umma_commit(&c->empty[p2]);
-                            if (last) umma_commit(&c->empty[p1]);
-                        }
-                        if (!H || last) umma_commit(&c->empty[s]);
-                        if (full) umma_commit(&c->accfull);
+                        umma_commit(&c->empty[s]);
+                        if (k == kb + h - 1 && pv + kb * a.seg >= v1) umma_commit(&c->accfull);
                     }
                     __syncwarp();
-                    if (full) {
-                        tiles = 0;
-                        ++sums;
+                    if (++w == W) w = 0;
+                    if (++s == S) {
+                        s = 0;
+                        ph ^= 1;
                     }
                 }
-                p2 = p1;
-                p1 = s;
-                if (++s == S) {
-                    s = 0;
-                    ph ^= 1;
-                }
             }
+            ++sums;
         }
         if (!ok && lane == 0) flag_error(2);
         if (elect_one()) umma_commit(&c->done);
-    } else if (warp < NX) {                                // warp = dx + 1, lane = input channel
-        long long tiles = 0;
-        for (long long i = blockIdx.x; i < a.items; i += gridDim.x) {
-            item(i, x0, y0, z0, z1, n);
-            tiles += z1 - z0;
-        }
-        const long long sums = (tiles + a.flush - 1) / a.flush, cstride = static_cast<long long>(TAPS) * a.cin;
+    } else if (warp < a.boxes) {                           // warp = dx + 1 (or channel chunk), lane = input channel
+        const long long cstride = static_cast<long long>(TAPS) * a.cin;
         const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+        uint32_t sums = 0;
         bool ok = true;
-        for (long long q = 0; q < sums; ++q) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&c->accfull, static_cast<uint32_t>(q & 1)));
+        for (int i = blockIdx.x; i < a.items; i += gridDim.x, ++sums) {
+            const int dz = item(i, v0, v1);
+            ok = __all_sync(0xffffffffu, mbar_wait(&c->accfull, sums & 1));
             if (!ok) break;
             tc_fence_after();
 #pragma unroll 1
-            for (int j = 0; j < NZ; ++j) {
-#pragma unroll 1
-                for (int b = 0; b < 2 * NZ; ++b) {         // 16 output channels of dy = 1 - b / 2
-                    float v[16];
-                    tmem_ld16(trow + j * N + b * 16, v);
-                    const int tap = TAPS == 27 ? j * 9 + (2 - b / 2) * 3 + warp : 0;
-                    float *dst = a.dw + (co0 + b % 2 * 16) * cstride + static_cast<long long>(tap) * a.cin + ci0 + lane;
+            for (int e = NZ - 1; e >= 0; --e) {            // in the order in which the next sum wants them
+                const int tap = TAPS == 27 ? (dz + 1) * 9 + (2 - e) * 3 + warp : 0;
+                const int ci = ci0 + lane + (TAPS == 27 ? 0 : 32 * warp);
+                float *dst = a.dw + co0 * cstride + static_cast<long long>(tap) * a.cin + ci;
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) atomicAdd(dst + e * cstride, v[e]);
+                for (int b = 0; b < 32; b += 16) {
+                    float v[16];
+                    tmem_ld16(trow + e * 32 + b, v);
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) atomicAdd(dst + (b + q) * cstride, v[q]);
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0)
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&c->accempty[j])) : "memory");
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&c->accempty[e])) : "memory");
             }
         }
         if (!ok && lane == 0) flag_error(4);
@@ -1414,17 +1432,32 @@ int launch_wgrad(const CUtensorMap &mm, const CUtensorMap &m0, const CUtensorMap
     return CT_OK;
 }
 
+// Bytes of a CTA's rings and control block, and the stages of X that fit beside `per_sm` CTAs on an SM (1 KB of each is
+// the system's).
+size_t cl_smem(const ClArgs &a, int h, int stages) {
+    return 1024 + (size_t)a.seg * 16 * kRowBytes * (stages * a.boxes + stages + 4 * h) + sizeof(ClCtrl);
+}
+
+int cl_stages(const ClArgs &a, int h, int per_sm) {
+    int s = 0;
+    while (s < kClStages && cl_smem(a, h, s + 1) <= (228u / per_sm - 1) * 1024) ++s;
+    return s;
+}
+
 template <int TAPS>
-int launch_wgrad_cl(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &md, const ClArgs &a, int chunks_x,
-                    int chunks_y, unsigned ctas, cudaStream_t st) {
-    constexpr size_t smem = cl_smem<TAPS>();
-    static bool attr = false;
-    if (!attr) {
-        CT_CUDA(cudaFuncSetAttribute(conv_wgrad_cl_kernel<TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "conv_wgrad_cl smem");
-        attr = true;
-    }
-    conv_wgrad_cl_kernel<TAPS><<<dim3(ctas, chunks_x, chunks_y), 192, smem, st>>>(m1, m2, md, a);
+int launch_wgrad_cl(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &md, ClArgs a, int cout, cudaStream_t st) {
+    const int h = TAPS == 27 ? a.nseg : 0;
+    // CTAs per SM, one's waits under the others' instructions: 3 where each can load two segments ahead, else 2.  128^3,
+    // 32 x 32 channels (2 stages with 3 CTAs): 161 / 178 / 179 us with 2 / 3 / 4; 64^3, 64 x 64 (3 stages): 89 / 86 / 136;
+    // 32^3, 128 x 128: 66 / 59 / 73.
+    int per_sm = cl_stages(a, h, 3) >= 3 ? 3 : (cl_stages(a, h, 2) >= 2 ? 2 : 1);
+    a.stages = cl_stages(a, h, per_sm);
+    const size_t smem = cl_smem(a, h, a.stages);
+    CT_CUDA(cudaFuncSetAttribute(conv_wgrad_cl_kernel<TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+            "conv_wgrad_cl smem");
+    const int gy = a.cin / (TAPS == 27 ? 32 : 32 * a.boxes), gz = cout / 32;
+    const int ctas = std::max(1, per_sm * sm_count() / (gy * gz));
+    conv_wgrad_cl_kernel<TAPS><<<dim3((unsigned)std::min(a.items, ctas), gy, gz), 192, smem, st>>>(m1, m2, md, a);
     CT_LAUNCH_CHECK("conv_wgrad_cl_kernel");
     return CT_OK;
 }
@@ -1581,44 +1614,43 @@ int ct_unet_conv3d_wgrad_cl(const void *x1, int c1, const void *x2, int c2, cons
     CT_REQUIRE(c1 > 0 && c1 % 32 == 0 && c2 >= 0 && c2 % 32 == 0 && cout > 0 && cout % 32 == 0 &&
                    c1 <= 32 * 65535 - c2 && cout <= 32 * 65535,
                "conv3d_wgrad_cl: channels must be positive multiples of 32");
-    CT_REQUIRE(nb > 0 && nz > 0 && ny > 0 && nx > 0 && nx % kYBx == 0 && ny % kYBy == 0 && (long long)nx * ny < (1ll << 30),
-               "conv3d_wgrad_cl: x must be a multiple of 8, y of 16");
+    CT_REQUIRE(nb > 0 && nz > 0 && ny > 0 && nx > 0 && (long long)nx * ny < (1ll << 30),
+               "conv3d_wgrad_cl: empty volume, or a plane too large");
     CT_REQUIRE(kper > 0, "conv3d_wgrad_cl: kper must be positive");
     CT_REQUIRE(aligned16(x1) && aligned16(dy) && (!x2 || aligned16(x2)),
                "conv3d_wgrad_cl: pointers must be 16-byte aligned");
-    CT_REQUIRE(((long long)nb * nz * ((nx * ny + kWK - 1) / kWK) + kper - 1) / kper <= 65535,
-               "conv3d_wgrad_cl: too many K splits (raise kper)");
-    CUtensorMap m1, m2, md;
-    int s;
-    if ((s = map_ndhwc(&m1, x1, c1, nx, ny, nz, nb, kYBx, kYBy, 1))) return s;
-    if ((s = map_ndhwc(&m2, c2 ? x2 : x1, c2 ? c2 : c1, nx, ny, nz, nb, kYBx, kYBy, 1))) return s;
-    if ((s = map_ndhwc(&md, dy, cout, nx, ny, nz, nb, kYBx, ntaps == 27 ? kYBy + 2 : kYBy, 1))) return s;
+    // Segments: 64 voxels, in whole rows where x is 16 or 32, or the largest power of two that
+    // divides x: partial sums (of 64 voxels) then end with one.
     ClArgs a{};
+    a.by = nx == 16 || nx == 32 ? 64 / nx : 1;
+    a.bx = std::min(nx & -nx, 64);
+    CT_REQUIRE(nx % 16 == 0 && ny % a.by == 0 && nx * ny % kWK == 0,
+               "conv3d_wgrad_cl: x must be a multiple of 16 and x * y of 64");
+    const int seg = a.bx * a.by;
+    a.seg = seg / 16;
+    a.nseg = nx / a.bx;
+    a.spp = nx * ny / seg;
     a.c1 = c1;
     a.cin = c1 + c2;
-    a.cout = cout;
     a.nz = nz;
-    a.tx = nx / kYBx;
-    a.ty = ny / kYBy;
-    a.flush = std::max(1, kper / 2);                       // tiles of 128 voxels, slices of 64
+    a.boxes = 3;
+    if (ntaps == 1)
+        for (a.boxes = 2; a.cin / 32 % a.boxes;) --a.boxes;
+    CT_REQUIRE(cl_stages(a, ntaps == 27 ? a.nseg : 0, 1) >= 2, "conv3d_wgrad_cl: rows too long");
+    const long long vox = (long long)nb * nz * ny * nx, ksplit = (vox / kWK + kper - 1) / kper;
+    CT_REQUIRE(ksplit <= 65535, "conv3d_wgrad_cl: too many K splits (raise kper)");
+    CT_REQUIRE(vox / 16 < (1ll << 30), "conv3d_wgrad_cl: volume too large");
+    a.steps = (int)(vox / 16);
+    a.chain = (int)std::min<long long>(4ll * kper, a.steps);
+    a.items = (int)ksplit * (ntaps == 27 ? 3 : 1);
     a.dw = dw;
-    // slices per item: the fewest steps of the busiest CTA, as the z-marching forward kernel chooses them
-    const int px = a.cin / 32, py = cout / 32;
-    const long long columns = (long long)nb * a.tx * a.ty, sms = std::max(1, sm_count() / (px * py));
-    long long best = -1;
-    for (int parts = 1; parts <= nz; ++parts) {
-        const int zc = (nz + parts - 1) / parts;
-        const long long items = columns * ((nz + zc - 1) / zc), cost = (items + sms - 1) / sms * (zc + 1);
-        if (best >= 0 && cost >= best) continue;
-        best = cost;
-        a.zc = zc;
-        a.items = items;
-    }
-    a.nzc = (nz + a.zc - 1) / a.zc;
-    const unsigned ctas = (unsigned)std::min(a.items, sms);
+    CUtensorMap m1, m2, md;
+    int s;
+    if ((s = map_ndhwc(&m1, x1, c1, nx, ny, nz, nb, a.bx, a.by, 1))) return s;
+    if ((s = map_ndhwc(&m2, c2 ? x2 : x1, c2 ? c2 : c1, nx, ny, nz, nb, a.bx, a.by, 1))) return s;
+    if ((s = map_ndhwc(&md, dy, cout, nx, ny, nz, nb, a.bx, a.by, 1))) return s;
     cudaStream_t st = as_stream(stream);
-    return ntaps == 27 ? launch_wgrad_cl<27>(m1, m2, md, a, px, py, ctas, st)
-                       : launch_wgrad_cl<1>(m1, m2, md, a, px, py, ctas, st);
+    return ntaps == 27 ? launch_wgrad_cl<27>(m1, m2, md, a, cout, st) : launch_wgrad_cl<1>(m1, m2, md, a, cout, st);
 }
 
 int ct_unet_conv3d_head(const void *x, int nb, int nz, int ny, int nx, const void *w, const float *bias, int relu,

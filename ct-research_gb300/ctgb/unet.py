@@ -100,11 +100,18 @@ def shift_copies(xs, ntaps=27):
     return xm, x0, xp
 
 
-def _wgrad_cl(cs, cout, y, x):
-    """Whether a weight gradient can read the channels-last tensors: whole 32-channel chunks and 8 x 16 voxel tiles
-    (faster than the channel-major copies at every channel count measured: 128^3, 32 x 32: 125 against 948 us,
-    32^3, 256 x 256: 157 against 164)."""
-    return len(cs) <= 2 and all(c % 32 == 0 for c in cs) and cout in (32, 64, 128, 256) and x % 8 == 0 and y % 16 == 0
+def _wgrad_cl(cs, cout, y, x, taps=27):
+    """Whether a weight gradient reads the channels-last tensors, which takes whole 32-channel chunks, rows of whole K steps
+    (16 voxels), partial sums (64) that end with one, and rings that hold the rows around a segment.  From 128 input and
+    128 output channels on the channel-major copies are faster (both give the same sums): 32^3, 128 x 128: 54 against 59 us,
+    16^3, 256 x 256: 38 against 53; 64 x 128 at 32^3 40 against 35, 128 x 64 at 64^3 225 against 162."""
+    if len(cs) > 2 or any(c % 32 for c in cs) or cout not in (32, 64, 128, 256) or x % 16 or x * y % 64:
+        return False
+    if taps == 27 and sum(cs) >= 128 and cout >= 128:
+        return False
+    if x <= 32:
+        return y % (64 // x) == 0
+    return 64 * (8 * min(x & -x, 64) + 4 * x) <= 230000
 
 
 def conv3d_wgrad(xs, dy, ntaps=27, kper=None, out=None):
@@ -118,7 +125,7 @@ def conv3d_wgrad(xs, dy, ntaps=27, kper=None, out=None):
     if kper is None:
         chunks = n * z * y * x // 64
         kper = max(16, -(-chunks // 1024))
-    if _wgrad_cl(cs, cout, y, x):
+    if _wgrad_cl(cs, cout, y, x, ntaps):
         x2 = xs[1] if len(xs) > 1 else None
         _lib.call("ct_unet_conv3d_wgrad_cl", _tptr(xs[0]), cs[0], _p(x2), cin - cs[0], _tptr(dy), cout, n, z, y, x,
                   ntaps, int(kper), _tptr(dw), _stream())

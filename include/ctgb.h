@@ -395,8 +395,8 @@ int ct_unet_conv3d_wgrad(const void *d_xm, const void *d_x0, const void *d_xp, i
                          int nb, int nz, int ny, int nx, int ntaps, int kper, float *d_dw, void *stream);
 /* The same gradient from the channels-last tensors themselves: X the concat of
  * d_x1 [v][c1] and d_x2 [v][c2] (c2 may be 0), dY [v][cout].  Channels multiples
- * of 32, x a multiple of 8, y of 16; partial sums of kper / 2 tiles of 128
- * voxels. */
+ * of 32, x of 16, x y of 64 (x = 16: y of 4, x = 32: y of 2), rows of up to about
+ * 700 voxels; the same partial sums, in the same order. */
 int ct_unet_conv3d_wgrad_cl(const void *d_x1, int c1, const void *d_x2, int c2, const void *d_dy, int cout, int nb,
                             int nz, int ny, int nx, int ntaps, int kper, float *d_dw, void *stream);
 /* One Adam step of `count` FP32 tensors (host arrays of device pointers; tensor i has n[i] elements):
