@@ -56,7 +56,8 @@ __device__ __forceinline__ int tile_pos(int k, int nfull, bool resid_first) {
 // 5.7; FBP of 720 rows of 1024 0.64 -> 0.49 ms (the filter 0.31 -> 0.17).
 //
 // grid: rows x split, each block a run of the row's outputs (split > 1 where the
-// rows alone would leave the GPU idle).
+// rows alone would leave the GPU idle).  A row filtered in place takes one block, which
+// has read the whole row before it writes.
 __global__ void __launch_bounds__(FT)
 row_filter_kernel(const RowFilter f, const float *__restrict__ R, float *__restrict__ out, int split) {
     extern __shared__ float4 sm4[];
@@ -269,9 +270,11 @@ int row_filter_launch(const RowFilter &f, const float *R, float *out, cudaStream
     // outputs then lie in one P-tile); where the rows give fewer than 8 warps per
     // scheduler, a block per warp
     const int warps = ((f.np + FJ - 1) / FJ + 31) / 32;
+    const size_t n = (size_t)f.nrow * f.np;
+    const bool in_place = R < out + n && out < R + n;      // the input's rows overlap the output's
     int per_block = std::min(warps, 4);
-    if (!f.win && (long long)f.nrow * warps < 32LL * sm_count()) per_block = 1;
-    const int split = f.win ? 1 : (warps + per_block - 1) / per_block;
+    if (!f.win && !in_place && (long long)f.nrow * warps < 32LL * sm_count()) per_block = 1;
+    const int split = f.win || in_place ? 1 : (warps + per_block - 1) / per_block;
     CT_REQUIRE((long long)f.nrow * split < (1LL << 31), "row filter: too many rows");
     row_filter_kernel<<<(unsigned)((long long)f.nrow * split), 32 * per_block, smem, st>>>(f, R, out, split);
     CT_LAUNCH_CHECK("row_filter_kernel");

@@ -1,0 +1,21 @@
+"""Forms of a call that a kernel's split, its range tests or its kept state must not change: operands that share memory,
+steps of either sign, uneven detector samples, calls on other streams, threads and after a device reset."""
+import pytest
+
+
+# The row filter in place: rows of several blocks (600, 1300 columns), few short rows (200 columns, a block per warp),
+# rows of one block, the smoothing window, and launch order on rows above its limit
+@pytest.mark.gpu
+@pytest.mark.parametrize("views,rows,cols,window", [(9, 7, 768, 0), (3, 2, 200, 0), (4, 3, 1300, 5), (40, 64, 128, 0),
+                                                    (2, 1, 2100, 0)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_row_filter_in_place(views, rows, cols, window, mode):
+    import torch
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry, centred_domain, view_angles
+    geom = ConeGeometry(8, 8, 8, (8.0, 8.0, 8.0), view_angles(views), centred_domain(cols, 0.05),
+                        centred_domain(rows, 0.1), 80.0)
+    plan = ConePlan(geom, fdk_filter=mode).set_filter("shepp-logan", window)
+    R = torch.rand((views, rows, cols), device="cuda")
+    ref = plan.fdk_filter(R)
+    assert torch.equal(plan.fdk_filter(R, out=R), ref)
