@@ -7,7 +7,7 @@ import pytest
 # rows of one block, the smoothing window, and launch order on rows above its limit
 @pytest.mark.gpu
 @pytest.mark.parametrize("views,rows,cols,window", [(9, 7, 768, 0), (3, 2, 200, 0), (4, 3, 1300, 5), (40, 64, 128, 0),
-                                                    (2, 1, 2100, 0)])
+                                                    (2, 2, 2100, 0)])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_row_filter_in_place(views, rows, cols, window, mode):
     import torch
