@@ -157,14 +157,15 @@ __global__ void __launch_bounds__(256)
 tv_apply_kernel(float *__restrict__ x, const float *__restrict__ g, long long n, float step, float lo,
                 const double *__restrict__ sumsq) {
     // one warp's FP64 root and division per block (in every warp they kept the FP64 pipe busy for half of the pass)
-    __shared__ float sh;
+    __shared__ float scale;
+    __shared__ bool moves;
     if (threadIdx.x < 32) {
         const double ss = *sumsq;
-        sh = ss > 0.0 ? (float)(step * sqrt((double)n / ss)) : -1.0f;
+        moves = ss > 0.0;
+        scale = (float)(step * sqrt((double)n / ss));
     }
     __syncthreads();
-    if (!(sh >= 0.0f)) return;
-    tv_move(x, g, n, sh, lo);
+    if (moves) tv_move(x, g, n, scale, lo);
 }
 
 // tv_apply_kernel with the ASD-POCS step on the device: state = (alpha, dp2, dg2)
@@ -173,14 +174,15 @@ tv_apply_kernel(float *__restrict__ x, const float *__restrict__ g, long long n,
 __global__ void __launch_bounds__(256)
 tv_apply_asd_kernel(float *__restrict__ x, const float *__restrict__ g, long long n, float lo,
                     const double *__restrict__ sumsq, const double *__restrict__ state) {
-    __shared__ float sh;
+    __shared__ float scale;
+    __shared__ bool moves;
     if (threadIdx.x < 32) {
         const double ss = *sumsq, dp2 = state[1];
-        sh = (ss > 0.0 && dp2 > 0.0) ? (float)(state[0] * sqrt(dp2 / ss)) : -1.0f;
+        moves = ss > 0.0 && dp2 > 0.0;
+        scale = (float)(state[0] * sqrt(dp2 / ss));
     }
     __syncthreads();
-    if (!(sh >= 0.0f)) return;
-    tv_move(x, g, n, sh, lo);
+    if (moves) tv_move(x, g, n, scale, lo);
 }
 
 // alpha <- alpha * alpha_red when the TV phase moved x more than r_max times the data step

@@ -19,3 +19,23 @@ def test_row_filter_in_place(views, rows, cols, window, mode):
     R = torch.rand((views, rows, cols), device="cuda")
     ref = plan.fdk_filter(R)
     assert torch.equal(plan.fdk_filter(R, out=R), ref)
+
+
+# A negative step moves against the flow, as written: from the same start the two moves are opposite (FP32 rounding of
+# values near 0.5: 6e-8 of them, against moves of 0.05).  The ASD-POCS phase with a negative alpha likewise.
+@pytest.mark.gpu
+def test_tv_flow_steps_of_either_sign():
+    import torch
+    from ctgb.device import tv_flow, tv_flow_asd
+    x0 = 0.5 + 0.2 * torch.randn((9, 20, 33), device="cuda")
+    up, down = tv_flow(x0.clone(), 1, -0.05, lo=-1e9), tv_flow(x0.clone(), 1, 0.05, lo=-1e9)
+    assert float((down - x0).abs().max()) > 0.01
+    assert float((up + down - 2 * x0).abs().max()) <= 4e-7
+    got = []
+    for alpha in (-0.2, 0.2):
+        x, prev = x0.clone(), x0 + 0.1
+        state = torch.tensor([alpha, 0.0, 0.0], dtype=torch.float64, device="cuda")
+        tv_flow_asd(x, prev, torch.empty_like(x), torch.zeros(2, dtype=torch.float64, device="cuda"), state, 1, lo=-1e9)
+        got.append(x - x0)
+    assert float(got[1].abs().max()) > 0.001
+    assert float((got[0] + got[1]).abs().max()) <= 4e-7
