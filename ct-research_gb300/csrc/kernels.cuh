@@ -26,8 +26,10 @@ struct FanGeom {
     double ires[2], ext[2];
     float2 res_ff[2], hsize_ff[2], D_ff, ipint_ff;
     // distance of a bin boundary, in bins, within which the backprojector's FP32
-    // detector coordinate does not decide the bin
+    // detector coordinate does not decide the bin; bins 1 .. inner lie on the detector
+    // whole
     float near_q;
+    int inner;
     // the walk set-up of every ray (fan_ray_table_launch), or null: computed per ray
     const struct FanRay *ray_tab;
     long long grazing;       // grazing rays of ray_tab
@@ -78,6 +80,11 @@ inline void fan_geom_derive(FanGeom &g) {
     const double q = err * ulp / g.pint + 2.0 * ulp * g.np;
     const bool grid = g.np <= (1 << 22) && (double)g.maxp - g.minp <= ((double)g.np - 0.5) * g.pint;
     g.near_q = grid && q < 0.5 ? (float)q : 1.0f;
+    // The implied grid (the first spacing) can run past the last sample, where uneven or
+    // rounded samples lie closer: a uniform domain of 8192 float samples is up to 2 bins
+    // shorter.  Bins that reach past it, the first and the last take the exact path.
+    const double len = ((double)g.maxp - g.minp) / (double)g.pint;
+    g.inner = len < g.np ? std::max(0, std::min(g.np - 3, (int)std::floor(len) - 1)) : std::max(g.np - 3, 0);
 }
 
 // Detector-row filter job (filter.cu).

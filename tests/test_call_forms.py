@@ -1,6 +1,9 @@
 """Forms of a call that a kernel's split, its range tests or its kept state must not change: operands that share memory,
 steps of either sign, uneven detector samples, calls on other streams, threads and after a device reset."""
+import numpy as np
 import pytest
+
+from conftest import rel_l2
 
 
 # The row filter in place: rows of several blocks (600, 1300 columns), few short rows (200 columns, a block per warp),
@@ -39,3 +42,34 @@ def test_tv_flow_steps_of_either_sign():
         got.append(x - x0)
     assert float(got[1].abs().max()) > 0.001
     assert float((got[0] + got[1]).abs().max()) <= 4e-7
+
+
+# A detector that the image's shadow passes, with a first spacing wider than the rest (the grid it implies runs 0.7 to 22
+# bins past the last sample, as 12000 even float samples' does by 4): pixel-views past the last sample get nothing.
+# FP32 against the reference's FP64 arithmetic on smooth rows: rel-L2 <= 1e-5, as for even samples.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,views,bins,down,first", [(64, 64, 90, False, 1.02), (64, 40, 333, True, 1.02),
+                                                     (65, 37, 90, True, 1.5), (64, 40, 50, False, 2.0)])
+def test_fan_backprojection_past_uneven_samples(oracle, n, views, bins, down, first):
+    import torch
+    from ctgb.batch import FanBatch
+    from ctgb.device import FanPlan
+    from ctgb.geometry import FanGeometry
+    half = 0.35 * n
+    step = np.full(bins - 1, 1.0)
+    step[0] = first
+    P = np.concatenate([[0.0], np.cumsum(step)])
+    P = (P / P[-1] * 2 - 1) * half
+    P = -P if down else P
+    beta = np.arange(1, views + 1) * (2 * np.pi / views)
+    size, D = np.array([float(n), float(n)]), 2.5 * n
+    phase = np.random.default_rng(bins).uniform(0, 6, (views, 1))
+    R = (1.5 + np.cos(phase + np.linspace(0, 5, bins)[None, :])).astype(np.float32)
+    b32, p32 = beta.astype(np.float32), P.astype(np.float32)
+    geom = FanGeometry(n, n, tuple(size), beta, P, D)
+    plan, d = FanPlan(geom), torch.from_numpy(R).cuda()
+    got = plan.bp(d)
+    assert rel_l2(got.cpu().numpy(), oracle.fan_bp(R, b32, p32, size, (n, n), D)) <= 1e-5
+    filt = oracle.fbpfan_filter(R, p32, D, mode=0)
+    assert rel_l2(plan.fbp(d, filter_mode=0).cpu().numpy(), oracle.fbpfan_bp(filt, b32, p32, size, (n, n), D)) <= 1e-5
+    assert torch.equal(FanBatch([geom]).bp(d.reshape(-1)), got.reshape(-1))
