@@ -329,6 +329,8 @@ int ct_cone_plan_create(ct_cone_plan **out, int nt, int ns, int nz, const double
     g.x0 = xi[0];
     g.psgn = (np > 1 && P[np - 1] < P[0]) ? -1.0f : 1.0f;
     g.xsgn = (nx > 1 && xi[nx - 1] < xi[0]) ? -1.0f : 1.0f;
+    g.wmin = 1.0f;
+    for (int i = 0; i + 1 < np; ++i) g.wmin = std::min(g.wmin, std::fabs(P[i + 1] - P[i]) / g.pint);
     // the reference evaluates sin/cos of the float angle with the
     // single-precision overloads (ProjectionCone_3D.cu:26-28)
     std::vector<double2> tr(nb);

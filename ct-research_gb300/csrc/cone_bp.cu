@@ -432,8 +432,8 @@ cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__
             l1 = izc * rz * ilc;
             l2 = 0.5f * qq * rz * rz * ilc * ilc * ilc;
             const float hl = hspan * ilc;
-            // the weights sum to 2 mts to the samples' drift: 10% of margin
-            fast = fast && 0.55f * izmax * (wa + wb) < hz && fabsf(izc) * ilc * hl * hl * hl < 2e-7f;
+            // the weights sum to at least 2 mts wmin, to 10% of margin
+            fast = fast && g.bp_zlim * izmax * (wa + wb) < hz && fabsf(izc) * ilc * hl * hl * hl < 2e-7f;
         }
         if (fast) {
             auto add = [&](int k, unsigned x, unsigned f, float top, float bot) {

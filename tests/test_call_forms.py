@@ -73,3 +73,24 @@ def test_fan_backprojection_past_uneven_samples(oracle, n, views, bins, down, fi
     filt = oracle.fbpfan_filter(R, p32, D, mode=0)
     assert rel_l2(plan.fbp(d, filter_mode=0).cpu().numpy(), oracle.fbpfan_bp(filt, b32, p32, size, (n, n), D)) <= 1e-5
     assert torch.equal(FanBatch([geom]).bp(d.reshape(-1)), got.reshape(-1))
+
+
+# Detector columns that lie closer than the first two, so that a voxel's column weights sum to less than 1, under a
+# volume of flat voxels whose z faces limit most chords: FP32 against the reference's FP64 arithmetic
+@pytest.mark.gpu
+@pytest.mark.parametrize("rest,down", [(0.5, False), (0.8, True), (0.05, False)])
+def test_cone_backprojection_uneven_columns(oracle, rest, down):
+    import torch
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry
+    nt, ns, nz, cols, rows, views = 16, 12, 400, 60, 80, 7
+    P = np.concatenate([[0.0, 1.0], 1.0 + rest * np.arange(1, cols - 1)])
+    P = (P / P[-1] * 2 - 1) * 14.0
+    P = -P if down else P
+    xi = (np.arange(rows) - (rows - 1) / 2) * (56.0 / rows)
+    beta = np.arange(1, views + 1) * (2 * np.pi / views)
+    size, D = (16.0, 12.0, 40.0), 100.0
+    g = ConeGeometry(nt, ns, nz, size, beta, P, xi, D)
+    R = np.random.default_rng(cols).random(g.sino_shape).astype(np.float32)
+    got = ConePlan(g).bp(torch.from_numpy(R).cuda()).cpu().numpy()
+    assert rel_l2(got, oracle.cone_bp(R, g.beta, g.P, g.xi, size, D, (nz, ns, nt))) <= 1e-5
