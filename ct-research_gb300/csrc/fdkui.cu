@@ -384,7 +384,7 @@ fdkui_bp_kernel(const UIGeom g, const UICol *__restrict__ rec, const float *__re
 // ---------------------------------------------------------------------------
 struct UIState {
     DevBuf beta, gama, tang, dgam, xi, xif, taps, views, rcov, R, disp, cosw, rec, part;
-    // the end of the last call that used cosw, rec or part, and its device
+    // the end of the last call, which used the tables and workspaces, and its device
     cudaEvent_t used = nullptr;
     int dev = -1;
     void release() {
@@ -397,6 +397,21 @@ struct UIState {
         for (DevBuf *b : {&beta, &gama, &tang, &dgam, &xi, &xif, &taps, &views, &rcov, &R, &disp, &cosw, &rec,
                           &part})
             b->release();
+    }
+    // Buffers of the current device.
+    int begin() {
+        int d = 0;
+        CT_CUDA(cudaGetDevice(&d), "cudaGetDevice");
+        if (dev != d) release();
+        dev = d;
+        if (!used) CT_CUDA(cudaEventCreateWithFlags(&used, cudaEventDisableTiming), "FDKUI: event");
+        return CT_OK;
+    }
+    // The kernels of the last call have read the tables and left the workspaces, on whatever
+    // stream it ran (the copies of the tables do not wait for a non-blocking one).
+    int wait() {
+        CT_CUDA(cudaEventSynchronize(used), "FDKUI: tables in use");
+        return CT_OK;
     }
 };
 std::mutex g_ui_mutex;
@@ -489,11 +504,10 @@ int ui_upload(UIState &S, const UIGeom &g, const double *xi, const double *gama,
         tg[k] = ff_split_host(std::tan(gama[k]));
         if (k + 1 < g.lg) dg[k] = (float)(gama[k + 1] - gama[k]);
     }
+    const std::vector<float2> taps = filter ? ui_taps(g, xi) : std::vector<float2>();
     int s;
-    if (filter) {
-        const std::vector<float2> taps = ui_taps(g, xi);
-        if ((s = upload(S.taps, taps.data(), taps.size()))) return s;
-    }
+    if ((s = S.wait())) return s;
+    if (filter && (s = upload(S.taps, taps.data(), taps.size()))) return s;
     if ((s = upload(S.tang, tg.data(), tg.size())) || (s = upload(S.dgam, dg.data(), dg.size()))) return s;
     if ((s = upload(S.beta, beta, (size_t)g.lb)) || (s = upload(S.gama, gama, (size_t)g.lg)) ||
         (s = upload(S.xi, xi, (size_t)g.lx)) || (s = upload(S.xif, xf.data(), xf.size())) ||
@@ -502,30 +516,12 @@ int ui_upload(UIState &S, const UIGeom &g, const double *xi, const double *gama,
     return CT_OK;
 }
 
-// The workspaces (cosw, rec, part) for a call on `st`: it waits for the last one
-// that used them, on whatever stream; before they grow, so does the host.
-int ui_workspace(UIState &S, bool grow, cudaStream_t st) {
-    int dev = 0;
-    CT_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
-    if (S.used && (grow || S.dev != dev)) CT_CUDA(cudaEventSynchronize(S.used), "FDKUI: workspace in use");
-    if (S.used && S.dev != dev) {
-        cudaEventDestroy(S.used);
-        S.used = nullptr;
-    }
-    if (!S.used) CT_CUDA(cudaEventCreateWithFlags(&S.used, cudaEventDisableTiming), "FDKUI: event");
-    else CT_CUDA(cudaStreamWaitEvent(st, S.used, 0), "FDKUI: workspace wait");
-    S.dev = dev;
-    return CT_OK;
-}
-
 int ui_filter(UIState &S, const UIGeom &g, const double *d_R, float *d_rcov, cudaStream_t st) {
     const size_t smem = sizeof(float) * 2 * (size_t)(((g.lg + 3) & ~3) + ((2 * g.lg - 1 + 18) & ~3));
     if (smem > 48 * 1024)
         CT_CUDA(cudaFuncSetAttribute(fdkui_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "fdkui filter smem attribute");
-    const size_t need = sizeof(double) * (size_t)g.lx * g.lg;
-    int s;
-    if ((s = ui_workspace(S, need > S.cosw.bytes, st)) || (s = S.cosw.ensure(need))) return s;
+    if (int s = S.cosw.ensure(sizeof(double) * (size_t)g.lx * g.lg)) return s;
     fdkui_cos_kernel<<<(unsigned)(((long long)g.lx * g.lg + 255) / 256), 256, 0, st>>>(
         g, S.gama.as<double>(), S.xi.as<double>(), S.cosw.as<double>());
     CT_LAUNCH_CHECK("fdkui_cos_kernel");
@@ -549,9 +545,7 @@ int ui_bp(UIState &S, const UIGeom &g, const float *d_rcov, double *d_disp, cuda
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>(g.lb, kUIRecBytes / (sizeof(UICol) * ncol)));
     const size_t need_rec = sizeof(UICol) * ncol * chunk, need_part = chunk < g.lb ? sizeof(float2) * ncol * g.nz : 0;
     int s;
-    if ((s = ui_workspace(S, need_rec > S.rec.bytes || need_part > S.part.bytes, st)) || (s = S.rec.ensure(need_rec)) ||
-        (s = S.part.ensure(need_part)))
-        return s;
+    if ((s = S.rec.ensure(need_rec)) || (s = S.part.ensure(need_part))) return s;
     for (int v0 = 0; v0 < g.lb; v0 += chunk) {
         const int nv = std::min(chunk, g.lb - v0);
         int per = 8;
@@ -594,7 +588,8 @@ int ct_fdkui_filter(const double *d_R, float *d_Rcov, const double *Xigamadomain
     if (s) return s;
     std::lock_guard<std::mutex> lk(g_ui_mutex);
     UIState &S = ui_state();
-    if ((s = ui_upload(S, g, Xigamadomain, Gamadomain, BetaScanRange, true))) return s;
+    if ((s = S.begin()) || (s = ui_upload(S, g, Xigamadomain, Gamadomain, BetaScanRange, true)))
+        return s;
     return ui_filter(S, g, d_R, d_Rcov, as_stream(stream));
 }
 
@@ -608,7 +603,8 @@ int ct_fdkui_bp(const float *d_Rcov, double *d_Display, const double *Xigamadoma
     if (s) return s;
     std::lock_guard<std::mutex> lk(g_ui_mutex);
     UIState &S = ui_state();
-    if ((s = ui_upload(S, g, Xigamadomain, Gamadomain, BetaScanRange, false))) return s;
+    if ((s = S.begin()) || (s = ui_upload(S, g, Xigamadomain, Gamadomain, BetaScanRange, false)))
+        return s;
     return ui_bp(S, g, d_Rcov, d_Display, as_stream(stream));
 }
 
@@ -623,7 +619,7 @@ int ct_FDKUI(double *Display, const double *R, const double *Xigamadomain, const
     std::lock_guard<std::mutex> lk(g_ui_mutex);
     UIState &S = ui_state();
     const size_t nr = (size_t)LGama * LBeta * LXigama, nd = (size_t)Size[0] * Size[1] * z_length;
-    if ((s = ui_upload(S, g, Xigamadomain, Gamadomain, BetaScanRange, true)) || (s = S.R.ensure(nr * sizeof(double))) ||
+    if ((s = S.begin()) || (s = ui_upload(S, g, Xigamadomain, Gamadomain, BetaScanRange, true)) || (s = S.R.ensure(nr * sizeof(double))) ||
         (s = S.rcov.ensure(nr * sizeof(float))) || (s = S.disp.ensure(nd * sizeof(double))))
         return s;
     CT_CUDA(cudaMemcpy(S.R.ptr, R, nr * sizeof(double), cudaMemcpyHostToDevice), "H2D projections");

@@ -94,3 +94,32 @@ def test_cone_backprojection_uneven_columns(oracle, rest, down):
     R = np.random.default_rng(cols).random(g.sino_shape).astype(np.float32)
     got = ConePlan(g).bp(torch.from_numpy(R).cuda()).cpu().numpy()
     assert rel_l2(got, oracle.cone_bp(R, g.beta, g.P, g.xi, size, D, (nz, ns, nt))) <= 1e-5
+
+
+# The curved-detector stages of two scans queued one behind the other on a stream of their own, which the copies of the
+# second scan's tables do not wait for: each gives what it gives alone
+@pytest.mark.gpu
+def test_curved_fdk_scans_back_to_back_on_a_stream():
+    import torch
+    from ctgb.device import fdkui_bp, fdkui_filter
+
+    def scan(lg, lx, nb, dg):
+        gama = (np.arange(lg) - (lg - 1) / 2) * dg
+        fan = abs(gama[-1] - gama[0])
+        return dict(gama=gama, xi=(np.arange(lx) - (lx - 1) / 2) * 1.5, beta=np.arange(nb) * ((np.pi + fan) / (nb - 1)),
+                    fan=fan, R=torch.rand((nb, lx, lg), dtype=torch.float64, device="cuda"))
+
+    def run(c):
+        rows = fdkui_filter(c["R"], c["xi"], c["gama"], c["beta"], 0.0, c["fan"], 110.0, 200.0)
+        rows.nan_to_num_(0.0, 0.0, 0.0)
+        return rows, fdkui_bp(rows, c["xi"], c["gama"], c["beta"], 110.0, 200.0, np.array([96, 96, 21], np.int32), 20)
+
+    a, b = scan(700, 24, 300, 0.0012), scan(700, 24, 300, 0.0011)
+    alone = [run(a), run(b)]
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        got = [run(c) for c in (a, b, a, b)]
+    s.synchronize()
+    for k, (rows, disp) in enumerate(got):
+        assert torch.equal(rows, alone[k % 2][0]) and torch.equal(disp, alone[k % 2][1])
