@@ -6,8 +6,11 @@
 // helpers; they stage host data through device buffers that persist between
 // calls (the reference allocates, copies and resets the device on every call,
 // ProjectionCone_3D.cu:433-520 and ProjectionCone_3D.cpp:53).
+#include <cuda.h>
+
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -673,6 +676,16 @@ struct ct_fan_plan {
     std::vector<float> hPf, hbf;
     FilterOpts filt;
     double wsum = 0.0;
+    size_t bytes() const {
+        size_t n = graze.buf.bytes;
+        for (const DevBuf *b : {&trig_d, &Pd, &trig_f, &Pf, &G, &wtab, &rcov, &pwt, &win, &scan, &rays}) n += b->bytes;
+        return n;
+    }
+    // The device memory is gone (a reset): nothing to free.
+    void forget() {
+        for (DevBuf *b : {&trig_d, &Pd, &trig_f, &Pf, &G, &wtab, &rcov, &pwt, &win, &scan, &rays}) *b = DevBuf();
+        graze = GrazeBuf();
+    }
     ~ct_fan_plan() {
         rays.release();
         trig_d.release(); Pd.release(); trig_f.release(); Pf.release();
@@ -1142,125 +1155,174 @@ int ct_FDKpro(float *Display, const float *R, const float *Xigamadomain, const f
 
 // 2D entry points: small problems, where a plan's ~10 allocations and frees and its
 // tables cost more than the kernels (250 of 330 us for an FBP of 256^2 / 360
-// views).  The last kDropinPlans plans stay, with their workspaces, found again by
-// the contents of their geometry (as cached_cone_plan's), and the two data
-// buffers; g_dropin_mutex covers a whole call, ct_dropin_release frees all.
+// views).  The last kDropinPlans plans stay, each with its workspaces and data buffers,
+// found again by the contents of their geometry.  A call has its plan to itself: calls of
+// several threads run side by side, and what a failed one used is not kept.  A plan
+// serves the context that made it; after a device reset (the reference's gateways
+// reset after every call) that context's id is gone, and the plan with it.
 namespace {
 
 constexpr int kDropinPlans = 4;
+constexpr size_t kDropinBytes = size_t(512) << 20;   // device memory of the plans kept
+
+// Id of the current device's context, unique over the life of the process; 0 if there is none to be had.
+unsigned long long context_id() {
+    using Fn = CUresult (*)(CUcontext, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<Fn>(p);
+    }();
+    unsigned long long id = 0;
+    if (!fn || cudaFree(nullptr) != cudaSuccess || fn(nullptr, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
 
 struct Dropin2D {
-    struct Entry {
-        ct_fan_plan *pl = nullptr;
-        std::vector<double> ang, P;
-        unsigned long long used = 0;
-    };
-    Entry plans[kDropinPlans];
+    ct_fan_plan *pl = nullptr;
     DevBuf in, out;
-    unsigned long long calls = 0;
+    std::vector<double> ang, P;
     int dev = -1;
-    void release() {
-        for (Entry &e : plans) {
-            delete e.pl;
-            e = Entry();
+    unsigned long long ctx = 0;
+
+    Dropin2D() = default;
+    Dropin2D(const Dropin2D &) = delete;
+    Dropin2D &operator=(const Dropin2D &) = delete;
+    ~Dropin2D() {
+        int d = 0;
+        if (cudaGetDevice(&d) == cudaSuccess && d != dev && dev >= 0) cudaSetDevice(dev);
+        if (context_id() != ctx) {      // its memory went with the context
+            if (pl) pl->forget();
+            in = out = DevBuf();
         }
+        delete pl;
         in.release();
         out.release();
+        if (d != dev && dev >= 0) cudaSetDevice(d);
     }
-    // The buffers of another device are freed; those of a device that was reset since
-    // (its addresses then no longer are device memory) are forgotten.
-    int check_device() {
-        int d = 0;
-        CT_CUDA(cudaGetDevice(&d), "cudaGetDevice");
-        if (in.ptr) {
-            cudaPointerAttributes a;
-            const bool gone = cudaPointerGetAttributes(&a, in.ptr) != cudaSuccess || a.type != cudaMemoryTypeDevice;
-            if (gone) {
-                (void)cudaGetLastError();
-                for (Entry &e : plans) e = Entry();      // its device memory went with the reset
-                in = out = DevBuf();
-            } else if (d != dev) {
-                release();
-            }
-        }
-        dev = d;
-        return CT_OK;
-    }
+    size_t bytes() const { return in.bytes + out.bytes + (pl ? pl->bytes() : 0); }
 };
-Dropin2D &dropin2d() {
-    static Dropin2D st;
-    return st;
+
+std::mutex g_dropin2d_mutex;                             // the two below
+unsigned long long g_dropin2d_releases = 0;
+std::vector<std::unique_ptr<Dropin2D>> &dropin2d_idle()  // the one used last at the end
+{
+    static std::vector<std::unique_ptr<Dropin2D>> v;
+    return v;
 }
 
-// A plan of this geometry, kept from an earlier call or made in the place of the
-// one that was used least recently.  res: the pixel pitch the caller passed.
-int cached_fan_plan(ct_fan_plan **out, int nt, int ns, const double size2[2], const double res[2], const double *ang,
-                    int nb, const double *P, int np, double D, int parallel) {
-    Dropin2D &st = dropin2d();
-    Dropin2D::Entry *old = &st.plans[0];
-    for (Dropin2D::Entry &e : st.plans) {
-        if (e.used < old->used) old = &e;
-        if (!e.pl) continue;
-        const FanGeom &g = e.pl->g;
-        if (g.nt == nt && g.ns == ns && g.nb == nb && g.np == np && g.D == D && g.parallel == parallel &&
-            g.size[0] == size2[0] && g.size[1] == size2[1] && g.res[0] == res[0] && g.res[1] == res[1] && ang && P &&
-            !std::memcmp(e.ang.data(), ang, sizeof(double) * nb) && !std::memcmp(e.P.data(), P, sizeof(double) * np)) {
-            e.used = ++st.calls;
-            *out = e.pl;
-            return CT_OK;
-        }
+// Drops the idle plans (all, or with `max` given those beyond that many and kDropinBytes); the caller frees them
+// outside the lock.
+std::vector<std::unique_ptr<Dropin2D>> dropin2d_evict(size_t max) {
+    std::vector<std::unique_ptr<Dropin2D>> &idle = dropin2d_idle(), gone;
+    size_t bytes = 0;
+    for (auto &e : idle) bytes += e->bytes();
+    while (!idle.empty() && (idle.size() > max || bytes > kDropinBytes)) {
+        bytes -= idle.front()->bytes();
+        gone.push_back(std::move(idle.front()));
+        idle.erase(idle.begin());
     }
-    ct_fan_plan *pl = nullptr;
-    int s = fan_plan_make(&pl, nt, ns, size2, ang, nb, P, np, D, parallel);
-    if (s) return s;
-    pl->g.res[0] = res[0];
-    pl->g.res[1] = res[1];
-    delete old->pl;
-    old->pl = pl;
-    old->ang.assign(ang, ang + nb);
-    old->P.assign(P, P + np);
-    old->used = ++st.calls;
-    *out = pl;
-    return CT_OK;
-}
-
-// which: 0 forward projection into doubles, 1 backprojection, 2 FBP.
-int fan2d_run(int which, const void *in, void *out, int nt, int ns, const double size2[2], const double res[2],
-              const double *ang, int nb, const double *P, int np, double D, int parallel, int filter_mode) {
-    std::lock_guard<std::mutex> lk(g_dropin_mutex);
-    Dropin2D &st = dropin2d();
-    ct_fan_plan *pl;
-    int s;
-    if ((s = st.check_device()) ||
-        (s = cached_fan_plan(&pl, nt, ns, size2, res, ang, nb, P, np, D, parallel)))
-        return s;
-    const FanGeom &g = pl->g;
-    const size_t nimg = (size_t)nt * ns, nsino = (size_t)nb * np;
-    const bool fp = which == 0;
-    const size_t bytes_in = (fp ? nimg : nsino) * sizeof(float);
-    const size_t bytes_out = fp ? nsino * sizeof(double) : nimg * sizeof(float);
-    if ((s = st.in.ensure(bytes_in)) || (s = st.out.ensure(bytes_out))) return s;
-    CT_CUDA(cudaMemcpy(st.in.ptr, in, bytes_in, cudaMemcpyHostToDevice), "H2D");
-    if (fp) {
-        GrazeList gl;
-        if ((s = graze_list(pl->graze, gl, (long long)nsino, 0)) ||
-            (s = fan_fp_launch(g, st.in.as<float>(), st.out.ptr, nullptr, nullptr, 0.f, nullptr, 3, gl, 0)))
-            return s;
-    } else if (which == 1) {
-        if ((s = fan_bp_launch(g, st.in.as<float>(), st.out.as<float>(), 0, nullptr, 0, 0, 0, 0, false, 0))) return s;
-    } else if ((s = ct_fan_fbp(pl, st.in.as<float>(), st.out.as<float>(), filter_mode, nullptr))) {
-        return s;
-    }
-    CT_CUDA(cudaMemcpy(out, st.out.ptr, bytes_out, cudaMemcpyDeviceToHost), "D2H");
-    return CT_OK;
+    return gone;
 }
 
 }  // namespace
 
 static void dropin2d_release() {
-    std::lock_guard<std::mutex> lk(g_dropin_mutex);
-    dropin2d().release();
+    std::vector<std::unique_ptr<Dropin2D>> gone;
+    std::lock_guard<std::mutex> lk(g_dropin2d_mutex);
+    ++g_dropin2d_releases;
+    gone = dropin2d_evict(0);
 }
+
+namespace {
+
+// which: 0 forward projection into doubles, 1 backprojection, 2 FBP, with e's plan.
+int fan2d_call(Dropin2D &e, int which, const void *in, void *out, int filter_mode) {
+    ct_fan_plan *pl = e.pl;
+    const FanGeom &g = pl->g;
+    const size_t nimg = (size_t)g.nt * g.ns, nsino = (size_t)g.nb * g.np;
+    const bool fp = which == 0;
+    const size_t bytes_in = (fp ? nimg : nsino) * sizeof(float);
+    const size_t bytes_out = fp ? nsino * sizeof(double) : nimg * sizeof(float);
+    int s;
+    if ((s = e.in.ensure(bytes_in)) || (s = e.out.ensure(bytes_out))) return s;
+    CT_CUDA(cudaMemcpy(e.in.ptr, in, bytes_in, cudaMemcpyHostToDevice), "H2D");
+    if (fp) {
+        GrazeList gl;
+        if ((s = graze_list(pl->graze, gl, (long long)nsino, 0)) ||
+            (s = fan_fp_launch(g, e.in.as<float>(), e.out.ptr, nullptr, nullptr, 0.f, nullptr, 3, gl, 0)))
+            return s;
+    } else if (which == 1) {
+        if ((s = fan_bp_launch(g, e.in.as<float>(), e.out.as<float>(), 0, nullptr, 0, 0, 0, 0, false, 0))) return s;
+    } else if ((s = ct_fan_fbp(pl, e.in.as<float>(), e.out.as<float>(), filter_mode, nullptr))) {
+        return s;
+    }
+    CT_CUDA(cudaMemcpy(out, e.out.ptr, bytes_out, cudaMemcpyDeviceToHost), "D2H");
+    return CT_OK;
+}
+
+// The call with a kept plan of this geometry or a new one.  res: the pixel pitch the caller passed.
+int fan2d_run(int which, const void *in, void *out, int nt, int ns, const double size2[2], const double res[2],
+              const double *ang, int nb, const double *P, int np, double D, int parallel, int filter_mode) {
+    const unsigned long long ctx = context_id();
+    std::unique_ptr<Dropin2D> e;
+    unsigned long long releases;
+    {
+        std::lock_guard<std::mutex> lk(g_dropin2d_mutex);
+        releases = g_dropin2d_releases;
+        auto &idle = dropin2d_idle();
+        for (size_t i = idle.size(); ctx && ang && P && i-- > 0;) {
+            const FanGeom &g = idle[i]->pl->g;
+            if (idle[i]->ctx == ctx && g.nt == nt && g.ns == ns && g.nb == nb && g.np == np && g.D == D &&
+                g.parallel == parallel && g.size[0] == size2[0] && g.size[1] == size2[1] && g.res[0] == res[0] &&
+                g.res[1] == res[1] && !std::memcmp(idle[i]->ang.data(), ang, sizeof(double) * nb) &&
+                !std::memcmp(idle[i]->P.data(), P, sizeof(double) * np)) {
+                e = std::move(idle[i]);
+                idle.erase(idle.begin() + i);
+                break;
+            }
+        }
+    }
+    int s = CT_OK;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        if (!e) {
+            e.reset(new Dropin2D);
+            e->ctx = ctx;
+            CT_CUDA(cudaGetDevice(&e->dev), "cudaGetDevice");
+            if (!(s = fan_plan_make(&e->pl, nt, ns, size2, ang, nb, P, np, D, parallel))) {
+                e->pl->g.res[0] = res[0];
+                e->pl->g.res[1] = res[1];
+                e->ang.assign(ang, ang + nb);
+                e->P.assign(P, P + np);
+            }
+        }
+        if (!s) s = fan2d_call(*e, which, in, out, filter_mode);
+        if (s != CT_ERR_OOM || attempt) break;
+        // once more without what is kept
+        e.reset();
+        dropin2d_release();
+        {
+            std::lock_guard<std::mutex> lk(g_dropin2d_mutex);
+            releases = g_dropin2d_releases;
+        }
+        s = CT_OK;
+    }
+    if (s || !ctx) return s;
+    std::vector<std::unique_ptr<Dropin2D>> gone;
+    {
+        std::lock_guard<std::mutex> lk(g_dropin2d_mutex);
+        if (releases == g_dropin2d_releases) {
+            dropin2d_idle().push_back(std::move(e));
+            gone = dropin2d_evict(kDropinPlans);
+        }
+    }
+    return CT_OK;
+}
+
+}  // namespace
 
 int ct_ProjectionFan_2D(const float *Pic, double *Projection, const double *BetaScanRange, const double *Pdomain,
                         int t_length, int s_length, double Center_t, double Center_s, int LBeta, int LP,

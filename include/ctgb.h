@@ -42,10 +42,11 @@ const char *ct_last_error(void);
 const char *ct_version(void);
 /* Frees the device memory that the host-pointer entry points below keep
  * between calls (the cone plan of the last geometry and its staging buffers,
- * the last four 2D plans and theirs, the IterativeFDK and curved-FDK buffers).  Call it before cudaDeviceReset,
- * which the reference's gateways run after every call (ProjectionCone_3D.cpp:53):
- * a reset frees those buffers behind the library's back.  No counterpart in
- * the reference, whose helpers allocate and free on every call. */
+ * the last four 2D plans and theirs up to 512 MiB, the IterativeFDK and
+ * curved-FDK buffers).  Call it before cudaDeviceReset, which the reference's
+ * gateways run after every call (ProjectionCone_3D.cpp:53): a reset frees those
+ * buffers behind the library's back (the 2D plans notice it by themselves).  No
+ * counterpart in the reference, whose helpers allocate and free on every call. */
 int ct_dropin_release(void);
 
 /* ===================================================================== */

@@ -123,3 +123,81 @@ def test_curved_fdk_scans_back_to_back_on_a_stream():
     s.synchronize()
     for k, (rows, disp) in enumerate(got):
         assert torch.equal(rows, alone[k % 2][0]) and torch.equal(disp, alone[k % 2][1])
+
+
+RESET_CHILD = r'''
+import ctypes as C, sys
+import numpy as np
+sys.path[:0] = [sys.argv[1], sys.argv[1] + "/ct-research_gb300"]
+from ctgb import _lib
+lib = _lib.lib()
+rt = C.CDLL("libcudart.so.13")
+rt.cudaMalloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+rt.cudaMemcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+p = lambda a: a.ctypes.data_as(C.c_void_p)
+n, nb, bins = 24, 20, 31
+beta = (np.arange(1, nb + 1) * (2 * np.pi / nb)).astype(np.float32)
+P = np.linspace(-30, 30, bins).astype(np.float32)
+R = np.random.default_rng(1).random((nb, bins)).astype(np.float32)
+size, out = np.array([24.0, 24.0]), []
+for k in range(3):
+    if k:
+        # memory of other owners at the addresses that the reset set free, in the sizes that the call uses
+        blocks = []
+        for nbytes in [4 * nb * bins, 4 * n * n, 512, 2048, 1 << 16, 1 << 20] * 8:
+            d = C.c_void_p()
+            assert rt.cudaMalloc(C.byref(d), nbytes) == 0
+            mark = np.full(nbytes, 0xA5, np.uint8)
+            assert rt.cudaMemcpy(d, p(mark), nbytes, 1) == 0
+            blocks.append((d, nbytes))
+    img = np.zeros((n, n), np.float32)
+    assert lib.ct_FBPfan(p(img), p(R), p(P), p(beta), nb, bins, p(size), n, n, C.c_double(70.0)) == 0, lib.ct_last_error()
+    out.append(img)
+    if k:
+        for d, nbytes in blocks:
+            got = np.empty(nbytes, np.uint8)
+            assert rt.cudaMemcpy(p(got), d, nbytes, 2) == 0
+            assert (got == 0xA5).all(), nbytes
+    assert rt.cudaDeviceReset() == 0
+assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2]) and out[0].any()
+print("kept apart")
+'''
+
+
+# A 2D host-pointer call after a device reset that nobody announced, with the freed addresses in other hands: the same
+# image, and the others' memory untouched
+@pytest.mark.gpu
+def test_2d_calls_after_a_device_reset():
+    import subprocess
+    import sys
+    from pathlib import Path
+    r = subprocess.run([sys.executable, "-c", RESET_CHILD, str(Path(__file__).resolve().parents[1])], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and "kept apart" in r.stdout, r.stdout + r.stderr
+
+
+# 2D calls of eight threads on six scans, two of them alike, with a release among them: every result is the one of a call
+# alone
+@pytest.mark.gpu
+def test_2d_calls_of_several_threads():
+    from concurrent.futures import ThreadPoolExecutor
+    from ctgb import _lib, ops
+    rng = np.random.default_rng(5)
+    scans = []
+    for n, nb, bins in ((24, 20, 31), (33, 17, 40), (24, 20, 31), (200, 90, 300), (64, 50, 91), (24, 21, 31)):
+        P = np.linspace(-0.9 * n, 0.9 * n, bins).astype(np.float32)
+        beta = (np.arange(1, nb + 1) * (2 * np.pi / nb)).astype(np.float32)
+        scans.append((rng.random((nb, bins)).astype(np.float32), beta, P, np.array([float(n)] * 2), n))
+
+    def call(k):
+        R, beta, P, size, n = scans[k % len(scans)]
+        return ops.FBPfan(R.ravel(), beta, P, size, n, n, 3.0 * n), ops.BackprojectionFan2D(R.ravel(), beta, P, size, n, n, 3.0 * n)
+
+    alone = [call(k) for k in range(len(scans))]
+    _lib.call("ct_dropin_release")
+    with ThreadPoolExecutor(8) as ex:
+        for k, got in enumerate(ex.map(call, range(60))):
+            for a, b in zip(got, alone[k % len(scans)]):
+                assert np.array_equal(a, b)
+            if k == 20:
+                _lib.call("ct_dropin_release")
