@@ -433,16 +433,21 @@ size_t ct_cone_plan_workspace_bytes(const ct_cone_plan *plan) {
            plan->graze.buf.bytes + plan->volT.bytes + plan->volS.bytes + plan->cols.bytes + plan->bpsum.bytes;
 }
 
-// Views per backprojection chunk: the caller's setting, else chunks of about
-// kBpChunkBytes at 16 bytes per detector sample, evened out over the scan.
+// Views per backprojection chunk: the caller's setting, up to kBpTableMost of
+// column-view records (1024 views of 1024^2 columns), else chunks of about
+// kBpChunkBytes at 16 bytes per detector sample and of at most kBpTableBytes of
+// records (256 views of 512^2 columns), evened out over the scan.
 // Shorter launches keep the views the resident blocks are working on close
 // together, so their samples stay in L2.
 constexpr size_t kBpChunkBytes = size_t(768) << 20;
+constexpr size_t kBpTableBytes = size_t(2) << 30, kBpTableMost = size_t(32) << 30;
 static int cone_bp_chunk_views(const ct_cone_plan *plan) {
     const ConeGeom &g = plan->g;
-    if (plan->bp_chunk > 0) return std::min(plan->bp_chunk, g.nb);
-    const size_t per_view = 16 * (size_t)g.nx * g.np;
-    const int target = (int)std::max<size_t>(1, std::min<size_t>(g.nb, kBpChunkBytes / std::max<size_t>(per_view, 1)));
+    const size_t per_view = 16 * (size_t)g.nx * g.np, table = cone_bp_table_bytes(g, 1);
+    if (plan->bp_chunk > 0)
+        return (int)std::max<size_t>(1, std::min<size_t>(std::min(plan->bp_chunk, g.nb), kBpTableMost / table));
+    const size_t most = std::min(kBpChunkBytes / per_view, kBpTableBytes / table);
+    const int target = (int)std::max<size_t>(1, std::min<size_t>(g.nb, most));
     const int nch = (g.nb + target - 1) / target;
     return (g.nb + nch - 1) / nch;
 }
@@ -510,14 +515,6 @@ int ct_cone_fp_residual(ct_cone_plan *plan, const float *d_vol, const float *d_b
                           1, gl, as_stream(stream));
 }
 
-// Views whose column-view records are held at a time: at most kBpTableBytes of
-// them (360 x 8 MiB at 512^2 columns).
-constexpr size_t kBpTableBytes = size_t(2) << 30;
-static int cone_bp_table_views(const ct_cone_plan *plan, int chunk) {
-    const size_t per_view = cone_bp_table_bytes(plan->g, 1);
-    return (int)std::max<size_t>(1, std::min<size_t>(chunk, kBpTableBytes / per_view));
-}
-
 // The workspace of a chunk of views: its pairs and, behind them, its records (one
 // allocation: a plan's first backprojection waits for it).
 static int cone_bp_work(ct_cone_plan *plan, int chunk, void **tab) {
@@ -527,15 +524,14 @@ static int cone_bp_work(ct_cone_plan *plan, int chunk, void **tab) {
     return CT_OK;
 }
 
-// Backprojection in chunks of cone_bp_chunk_views views (fewer where their
-// records would not fit): every chunk is packed into pairs and backprojected,
-// its sums added to the volume (or, for the fused SIRT update, to a partial-sum
-// volume that the last chunk folds into the update).
+// Backprojection in chunks of cone_bp_chunk_views views: every chunk is packed
+// into pairs and backprojected, its sums added to the volume (or, for the fused
+// SIRT update, to a partial-sum volume that the last chunk folds into the update).
 static int cone_bp_common(ct_cone_plan *plan, const float *d_proj, float *d_vol, int weighting,
                           const float *colsum, float eps, float lambda, float lo, float hi, bool update,
                           cudaStream_t st) {
     const ConeGeom &g = plan->g;
-    const int chunk = cone_bp_table_views(plan, cone_bp_chunk_views(plan));
+    const int chunk = cone_bp_chunk_views(plan);
     const int nchunks = (g.nb + chunk - 1) / chunk;
     int s;
     void *tab;
@@ -1086,7 +1082,7 @@ static int cone_bp_dropin(float *Display, const float *R, const float *xi, const
     DropinState &st = dropin();
     const size_t nv = (size_t)nt * ns * nz, npj = (size_t)nb * np * nx;
     if ((s = st.vol.ensure(nv * sizeof(float))) || (s = st.proj.ensure(npj * sizeof(float)))) return s;
-    const int bchunk = cone_bp_table_views(pl, std::min(cone_bp_chunk_views(pl), kDropinChunk * 2));
+    const int bchunk = std::min(cone_bp_chunk_views(pl), kDropinChunk * 2);
     if (!fdk && nb > bchunk && np >= 2 && nx >= 2 && host_pinned(R) && host_pinned(Display)) {
         // pinned buffers: copy view chunks (the backprojector's own chunks) in,
         // each backprojected (and added to the volume) while the next one arrives;

@@ -174,10 +174,11 @@ int ct_cone_plan_set_short_scan(ct_cone_plan *plan, int enable);
 size_t ct_cone_plan_workspace_bytes(const ct_cone_plan *plan);
 /* Views per chunk of the backprojectors (ct_cone_bp, ct_cone_bp_update,
  * ct_cone_fdk_bp): each chunk's detector data is packed and backprojected on
- * its own and its sums added to the volume; the packed data needs 16 bytes per
- * detector sample of one chunk.  0 (the default): automatic, chunks of about
- * 768 MiB of packed data evened out over the scan (shorter launches keep the
- * packed views in L2); a value >= the view count: one pass.  Results differ
+ * its own and its sums added to the volume; a chunk needs 8 bytes per detector
+ * sample for the packed data and 32 per volume column and view for its set-up.
+ * 0 (the default): automatic, chunks of about 384 MiB of packed data and at most
+ * 2 GiB of set-up evened out over the scan (shorter launches keep the packed
+ * views in L2); a value >= the view count: one pass, up to 32 GiB of set-up.  Results differ
  * from one pass only by float rounding of the partial sums.  get returns the
  * chunk in effect.  No counterpart in the reference. */
 int ct_cone_plan_set_bp_chunk(ct_cone_plan *plan, int views);

@@ -201,3 +201,26 @@ def test_2d_calls_of_several_threads():
                 assert np.array_equal(a, b)
             if k == 20:
                 _lib.call("ct_dropin_release")
+
+
+# The chunk that is reported is the one in effect: automatic chunks where the set-up's records bound them (64 views of
+# 1024^2 columns, evened out), and a set value up to the view count, in one pass
+@pytest.mark.gpu
+def test_backprojection_chunk_in_effect():
+    import torch
+    from ctgb import _lib
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry, centred_domain, view_angles
+    lib = _lib.lib()
+    geom = ConeGeometry(1024, 1024, 3, (100.0, 100.0, 0.3), view_angles(100), centred_domain(60, 3.0),
+                        centred_domain(6, 0.2), 400.0)
+    R, got = torch.rand(geom.sino_shape, device="cuda"), []
+    for views, chunk, launches in ((0, 50, 3 + 3 * 2), (100, 100, 6), (1000, 100, 6), (70, 70, 9)):
+        plan = ConePlan(geom).set_bp_chunk(views)
+        assert plan.bp_chunk_views() == chunk and plan.launches_per_pair() == launches
+        got.append(plan.bp(R))
+        size = lib.ct_cone_plan_workspace_bytes(plan._h)
+        need = chunk * (8 * 60 * 6 + 32 * 1024 * 1024)
+        assert need <= size <= need + (1 << 20)
+    for v in got[1:]:
+        assert rel_l2(v.cpu().numpy(), got[0].cpu().numpy()) <= 1e-6
