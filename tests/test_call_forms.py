@@ -224,3 +224,21 @@ def test_backprojection_chunk_in_effect():
         assert need <= size <= need + (1 << 20)
     for v in got[1:]:
         assert rel_l2(v.cpu().numpy(), got[0].cpu().numpy()) <= 1e-6
+
+
+# Columns of many slices: the row quotient is stepped from the set-up's first slice.  On rows that alternate between 0 and
+# 1 an error of the quotient is one of the value; FP32 arithmetic leaves 2^-22 at most.
+@pytest.mark.gpu
+@pytest.mark.parametrize("nz", [500, 60000])
+def test_cone_backprojection_of_tall_columns(oracle, nz):
+    import torch
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry
+    rows, size, D = 6000, (2.0, 2.0, 50.0), 100.0
+    P, xi = np.arange(8) - 3.5, (np.arange(rows) - (rows - 1) / 2) * 0.01
+    for view in range(12):
+        g = ConeGeometry(2, 2, nz, size, np.array([0.3 + 0.5 * view]), P, xi, D)
+        R = np.zeros(g.sino_shape, np.float32)
+        R[:, ::2] = 1.0
+        got = ConePlan(g).bp(torch.from_numpy(R).cuda()).cpu().numpy()
+        assert rel_l2(got, oracle.cone_bp(R, g.beta, g.P, g.xi, size, D, (nz, 2, 2))) <= 2.0 ** -22
