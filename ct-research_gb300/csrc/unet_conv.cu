@@ -1364,16 +1364,17 @@ size_t yring_smem() {
     return 1024 + kYStages * (kYABytes + 3 * N * kRowBytes) + sizeof(Ctrl);
 }
 
+// A kernel's shared memory above 48 KB is granted per device: asked for at each launch.
+int grant_smem(const void *kernel, size_t smem) {
+    CT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "convolution smem");
+    return CT_OK;
+}
+
 template <int N, bool YR>
 int launch_fwd(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap &mw, const FwdArgs &a, int tiles,
                cudaStream_t st) {
     const size_t smem = YR ? yring_smem<N>() : ring_smem<N>();
-    static bool attr = false;
-    if (!attr) {
-        CT_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<N, YR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "conv_fwd smem");
-        attr = true;
-    }
+    if (int e = grant_smem((const void *)conv_fwd_kernel<N, YR>, smem)) return e;
     conv_fwd_kernel<N, YR><<<tiles, 128, smem, st>>>(m1, m2, mw, a);
     CT_LAUNCH_CHECK("conv_fwd_kernel");
     return CT_OK;
@@ -1406,12 +1407,7 @@ int launch_march(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensorMap
     }
     a.nzc = (f.nz + a.zc - 1) / a.zc;
     constexpr size_t smem = march_smem<N, NCH>();
-    static bool attr = false;
-    if (!attr) {
-        CT_CUDA(cudaFuncSetAttribute(conv_march_kernel<N, NCH, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "conv_march smem");
-        attr = true;
-    }
+    if (int e = grant_smem((const void *)conv_march_kernel<N, NCH, HEAD>, smem)) return e;
     conv_march_kernel<N, NCH, HEAD><<<(unsigned)((std::min(a.items, groups) + kMGroups - 1) / kMGroups * a.parts), 192 * kMGroups, smem, st>>>(m1, m2, mw, a);
     CT_LAUNCH_CHECK("conv_march_kernel");
     return CT_OK;
@@ -1421,12 +1417,7 @@ template <int N>
 int launch_wgrad(const CUtensorMap &mm, const CUtensorMap &m0, const CUtensorMap &mp, const CUtensorMap &md,
                  const WgradArgs &a, dim3 grid, cudaStream_t st) {
     const size_t smem = wring_smem<N>();
-    static bool attr = false;
-    if (!attr) {
-        CT_CUDA(cudaFuncSetAttribute(conv_wgrad_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "conv_wgrad smem");
-        attr = true;
-    }
+    if (int e = grant_smem((const void *)conv_wgrad_kernel<N>, smem)) return e;
     conv_wgrad_kernel<N><<<grid, 128, smem, st>>>(mm, m0, mp, md, a);
     CT_LAUNCH_CHECK("conv_wgrad_kernel");
     return CT_OK;
@@ -1453,8 +1444,7 @@ int launch_wgrad_cl(const CUtensorMap &m1, const CUtensorMap &m2, const CUtensor
     int per_sm = cl_stages(a, h, 3) >= 3 ? 3 : (cl_stages(a, h, 2) >= 2 ? 2 : 1);
     a.stages = cl_stages(a, h, per_sm);
     const size_t smem = cl_smem(a, h, a.stages);
-    CT_CUDA(cudaFuncSetAttribute(conv_wgrad_cl_kernel<TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "conv_wgrad_cl smem");
+    if (int e = grant_smem((const void *)conv_wgrad_cl_kernel<TAPS>, smem)) return e;
     const int gy = a.cin / (TAPS == 27 ? 32 : 32 * a.boxes), gz = cout / 32;
     const int ctas = std::max(1, per_sm * sm_count() / (gy * gz));
     conv_wgrad_cl_kernel<TAPS><<<dim3((unsigned)std::min(a.items, ctas), gy, gz), 192, smem, st>>>(m1, m2, md, a);
