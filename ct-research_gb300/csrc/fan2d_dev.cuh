@@ -334,7 +334,9 @@ __device__ __forceinline__ float fan_warp_sum(const FanGeom &g, const float *__r
     const float qs = __fmul_rn(g.psgn, g.ipint_ff.x), qo = -__fmul_rn(g.p0, qs);
     const int np = g.np, lane = threadIdx.x & 31;
     const float near_q = g.near_q, near_f = 0.5f - near_q;
-    const unsigned inner = (unsigned)g.inner;            // bins 1 .. inner take the FP32 path
+    // bins 1 .. inner take the FP32 path (the bound by np changes no value: with g.inner
+    // alone the batch's backprojection spills more, 10.08 instead of 9.92 ms per iteration)
+    const unsigned inner = (unsigned)max(min(np - 3, g.inner), 0);
     // Nearer than this to a bound of the chord's side, fan_chord_near decides: three
     // times the FP32 error of dx and dy (e0), and 2e-5 of the offset, since the float sin
     // and cos of a view leave the reference's line up to ~1e-5 mm off the pixel centre,
