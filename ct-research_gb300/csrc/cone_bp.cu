@@ -372,7 +372,7 @@ cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__
     const float iz0 = ff_from((z0 + 0.5) * g.res[2] - 0.5 * g.size[2]).hi;   // iz of this thread's first z
     // largest |iz| of the thread's z range: decides whether z faces can limit the chord
     const float izmax = fmaxf(fabsf(iz0), fabsf(fmaf((float)(BP_ZC - 1), rz, iz0)));
-    const float wlim = hz / (g.bp_zlim * izmax);
+    const float izw = izmax / g.wmin;  // a column's weights sum to at least 2 mts wmin
     const long long vstride = (long long)g.nx * g.np;
     const long long ncol = (long long)g.nt * g.ns;
     const unsigned last = (unsigned)(g.nx - 2);
@@ -438,8 +438,8 @@ cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__
             l1 = izc * rz * ilc;
             l2 = 0.5f * qq * rz * rz * ilc * ilc * ilc;
             const float hl = hspan * ilc;
-            // the weights sum to at least 2 mts wmin, to 10% of margin
-            fast = fast && wa + wb < wlim && fabsf(izc) * ilc * hl * hl * hl < 2e-7f;
+            // |iz| mts < hz for every z, to 10% of margin
+            fast = fast && 0.55f * izw * (wa + wb) < hz && fabsf(izc) * ilc * hl * hl * hl < 2e-7f;
         }
         if (fast) {
             auto add = [&](int k, unsigned x, unsigned f, float top, float bot) {

@@ -39,7 +39,6 @@ struct ConeGeom {
     float pint, xint, bint;  // |P1-P0|, |xi1-xi0|, |beta1-beta0|
     float minp, maxp, minx, maxx;
     float p0, x0;            // P[0], xi[0]
-    float wmin;              // smallest |P[i+1] - P[i]| / pint: the least sum of a voxel's two column weights
     float psgn, xsgn;        // +1 for ascending domains, -1 for descending
     // Row table of the backprojectors: for x < nx - 1, (x - q(xi[x]), q(xi[x+1]) - x)
     // with q(v) = |v - xi[0]| / xint the reference's row quotient (in double);
@@ -61,7 +60,7 @@ struct ConeGeom {
     // and its float constants: res_z, 1 / res_z, half voxel (t, s, z), size_z / 2,
     // iz at z = 0, D, 1 / D, 1 / PInt
     float bp_rz, bp_irz, bp_ht, bp_hs, bp_hz, bp_czf, bp_xbase, bp_Df, bp_iD, bp_ipintf;
-    float bp_zlim;           // 0.5 / wmin and 10%: a chord is not limited in z where |iz| (wa + wb) bp_zlim < hz
+    float wmin;              // smallest |P[i+1] - P[i]| / pint: the least sum of a voxel's two column weights
 };
 
 // The scalar constants derived from the sizes and the voxel pitch (ext, extf,
@@ -112,7 +111,6 @@ inline void cone_bp_consts(ConeGeom &g) {
     g.bp_Df = (float)g.D;
     g.bp_iD = 1.0f / g.bp_Df;
     g.bp_ipintf = 1.0f / g.pint;
-    g.bp_zlim = 0.55f / g.wmin;
 }
 
 }  // namespace ct
