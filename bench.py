@@ -381,6 +381,7 @@ def run_ours(args):
     ach = kern[dom]["achieved_gbs"]
     full_case = args.size == "full" and not args.views
     tr = traffic.get(dom.split("+")[0]) if full_case else None
+    # `bound`: the rate that frac is taken of.  The backprojector's bytes come from L1 and L2; it is bound by issue
     roofline = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                 "traffic": tr.get("bytes_per_launch") if isinstance(tr, dict) else tr,
                 "traffic_source": ("stored ncu capture of this kernel on this workload, not measured by this run: "

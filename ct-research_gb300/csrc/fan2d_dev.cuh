@@ -311,8 +311,8 @@ constexpr int kFanUnroll = 4;
 // where they occur, with one or two lanes active, they took 60% of the FBP's
 // time and half of the chord weight's.
 //
-// Issue-bound: 46 instructions per pixel-view (FBP) and 60 (chord weight), 67%
-// of the issue slots, against ~160 and 132 of the form this replaced, which divided in IEEE and
+// Issue-bound: 51 instructions per pixel-view (FBP, the queue included) and about 60 (chord
+// weight), 69% of the issue slots, against ~160 and 132 of the form this replaced, which divided in IEEE and
 // built the unit direction of the line.  One approximate reciprocal of
 // Rscan - S serves P / U and the FBP weight 1 / U^2 (the constants multiply the
 // sum once, at the end); the floor is an addition rounded down.  Every rounding

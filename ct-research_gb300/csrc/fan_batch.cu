@@ -34,8 +34,8 @@ __device__ __forceinline__ int find_slice(const BatchSlice *__restrict__ sl, int
 }
 
 template <int MODE>
-// blocks per SM of the batched projection: 4 (32 registers) measured 6.04 ms on
-// 64 uneven slices against 6.17 / 6.32 ms at 3 / 2
+// blocks per SM of the batched projection: a SIRT iteration of 64 uneven slices takes
+// 9.93 / 9.89 / 9.96 ms at 4 (32 registers) / 3 / 2
 #ifndef CT_FANB_FP_MINB
 #define CT_FANB_FP_MINB 4
 #endif
@@ -71,8 +71,8 @@ fan_batch_fp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__r
 }
 
 // blocks of 512 threads per SM the batched backprojection's registers aim at: 2
-// (64 registers): a SIRT iteration of 64 uneven slices 12.2 ms; 12.4 ms with 112
-// registers, 22 ms with 40 (3 blocks: the loop spills)
+// (64 registers): with the three-axis projection before, a SIRT iteration of 64 uneven
+// slices 12.2 ms; 12.4 ms with 112 registers, 22 ms with 40 (3 blocks: the loop spills)
 template <int WMODE, bool UPDATE>
 __global__ void __launch_bounds__(512, 2)
 fan_batch_bp_kernel(const BatchSlice *__restrict__ sl, int nsl, const float *__restrict__ R, float *__restrict__ img,

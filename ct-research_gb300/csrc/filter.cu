@@ -52,8 +52,7 @@ __device__ __forceinline__ int tile_pos(int k, int nfull, bool resid_first) {
 // rounded product and TwoSum.
 //
 // FP32-bound: 16 operations per sample of a thread against 0.5 shared loads.
-// FDK of 256^3 (360 x 384 rows of 512) 16.5 -> 13.35 ms, of which the filter 8.9 ->
-// 5.7; FBP of 720 rows of 1024 0.64 -> 0.49 ms (the filter 0.31 -> 0.17).
+// 360 x 384 rows of 512 (FDK of 256^3) 8.9 -> 5.1 ms, 720 rows of 1024 (FBP) 0.31 -> 0.134 ms.
 //
 // grid: rows x split, each block a run of the row's outputs (split > 1 where the
 // rows alone would leave the GPU idle).  A row filtered in place takes one block, which

@@ -21,8 +21,9 @@ Architecture (4 levels, 32 base channels, 3x3x3 convolutions, ReLU):
 Every convolution, forward and both gradients, runs in ``ct_unet_conv3d`` /
 ``ct_unet_conv3d_wgrad[_cl]`` (bf16 operands, FP32 accumulation in tensor memory);
 pooling, upsampling, the head and the bias gradients are small CUDA kernels of
-the same library.  PyTorch holds the tensors and runs Adam on the FP32 master
-weights.  Activations are bf16 channels-last [n][z][y][x][c].
+the same library, and so is Adam on the FP32 master weights (torch's expressions
+where a tensor is not plain CUDA float32).  PyTorch holds the tensors.  Activations
+are bf16 channels-last [n][z][y][x][c].
 """
 from __future__ import annotations
 
