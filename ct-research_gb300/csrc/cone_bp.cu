@@ -379,7 +379,7 @@ cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__
     constexpr unsigned all = 0xffffffffu >> (32 - BP_ZC);
     const float kc = 0.5f * (BP_ZC - 1);
     const float izc = fmaf(kc, rz, iz0);
-    const float hspan = kc * rz;
+    const float hspan = kc * rz, izq = fabsf(izc) + 0.25f * hspan;
 
     float acc[BP_ZC];
 #pragma unroll
@@ -422,7 +422,8 @@ cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__
         // the affine quotient decide), no z face limits the chord, and the chord length
         // |d| = sqrt(qq + iz^2) is the quadratic in k about the thread's middle z
         // (relative error below 1e-7, bounded by the third-order term
-        // |iz| h^3 / (2 |d|^4), h the half span of the z).
+        // |iz| h^3 / (2 |d|^4) and the fourth, h^4 / (8 |d|^4), which alone is left in the
+        // mid-plane; h the half span of the z).
         bool fast = inmask == all && (unsigned)(int)(r >> 32) <= last &&
                     (unsigned)(int)((r + (BP_ZC - 1) * dqf) >> 32) <= last &&
                     !(WMODE == W_FDK_STICKY && kz < BP_ZC - 1);
@@ -439,7 +440,7 @@ cone_bp_kernel(const ConeGeom g, const float2 *__restrict__ Q, const ColView *__
             l2 = 0.5f * qq * rz * rz * ilc * ilc * ilc;
             const float hl = hspan * ilc;
             // |iz| mts < hz for every z, to 10% of margin
-            fast = fast && 0.55f * izw * (wa + wb) < hz && fabsf(izc) * ilc * hl * hl * hl < 2e-7f;
+            fast = fast && 0.55f * izw * (wa + wb) < hz && izq * ilc * hl * hl * hl < 2e-7f;
         }
         if (fast) {
             auto add = [&](int k, unsigned x, unsigned f, float top, float bot) {

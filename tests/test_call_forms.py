@@ -242,3 +242,21 @@ def test_cone_backprojection_of_tall_columns(oracle, nz):
         R[:, ::2] = 1.0
         got = ConePlan(g).bp(torch.from_numpy(R).cuda()).cpu().numpy()
         assert rel_l2(got, oracle.cone_bp(R, g.beta, g.P, g.xi, size, D, (nz, 2, 2))) <= 2.0 ** -22
+
+
+# Threads whose z lie about the mid-plane of a volume of tall voxels close to the source, where the chord is no quadratic
+# in z: 4, 8 and 32 slices per thread against the reference's FP64 arithmetic
+@pytest.mark.gpu
+@pytest.mark.parametrize("nt,nz,rz", [(3, 20, 2.0), (3, 4, 0.7), (200, 48, 3.0), (130, 40, 1.5), (3, 32, 0.3)])
+def test_cone_backprojection_about_the_mid_plane(oracle, nt, nz, rz):
+    import torch
+    from ctgb.device import ConePlan
+    from ctgb.geometry import ConeGeometry
+    views, cols, rows = 5, 80, 90
+    size, D = (float(nt), float(nt), nz * rz), 1.2 * nt
+    P = (np.arange(cols) - (cols - 1) / 2) * (4.0 * nt / cols)
+    xi = (np.arange(rows) - (rows - 1) / 2) * (9.0 * nz * rz / rows)
+    g = ConeGeometry(nt, nt, nz, size, np.arange(1, views + 1) * (2 * np.pi / views), P, xi, D)
+    R = np.random.default_rng(nz).random(g.sino_shape).astype(np.float32)
+    got = ConePlan(g).bp(torch.from_numpy(R).cuda()).cpu().numpy()
+    assert rel_l2(got, oracle.cone_bp(R, g.beta, g.P, g.xi, size, D, (nz, nt, nt))) <= 1e-6
