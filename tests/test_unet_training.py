@@ -90,8 +90,8 @@ def test_channel_sums_keep_their_order(c):
 
 
 # Two training steps against the same network on the channel-major weight gradients, torch's Adam expressions and torch's
-# sum of the skip gradients.  Each side's FP32 atomics add its partial sums in any order (a few 2^-24 of a gradient), so
-# the first gradients agree to 2e-6; 2e-5 for the second step's, two of whose runs differ by less than 1e-6.
+# sum of the skip gradients.  Each side's FP32 atomics add its partial sums in any order, a few 2^-24 of a gradient: 2e-6.
+# One of 4 million weights may come out a bf16 step away for that; the second step starts from the same ones.
 @pytest.mark.parametrize("shape", [(64, 64, 64), (32, 64, 128)])
 def test_two_training_steps_repeat(shape, monkeypatch):
     import torch
@@ -99,28 +99,22 @@ def test_two_training_steps_repeat(shape, monkeypatch):
     g = torch.Generator(device="cuda").manual_seed(3)
     x = torch.rand(shape, device="cuda", generator=g)
     y = torch.rand(shape, device="cuda", generator=g)
-
-    def steps(plain):
-        net = warmstart.load()
-        got = []
-        with monkeypatch.context() as m:
-            if plain:
-                m.setattr(unet, "_wgrad_cl", lambda *a: False)
-            for _ in range(2):
+    nets = warmstart.load(), warmstart.load()
+    for _ in range(2):
+        grads = []
+        for net, plain in zip(nets, (True, False)):
+            with monkeypatch.context() as m:
+                if plain:
+                    m.setattr(unet, "_wgrad_cl", lambda *a: False)
                 out = net.forward(x, keep=True)
-                grads = net.backward((2.0 / out.numel()) * (out - y))
-                if plain:       # strided gradients take torch's expressions
-                    net.adam_step({k: torch.stack((v, v), -1)[..., 0] for k, v in grads.items()}, lr=1e-5)
-                else:
-                    net.adam_step(grads, lr=1e-5)
-                got.append(grads)
-        return got
-
-    ref = steps(True)
-    for run in (steps(False), steps(False)):
-        for tol, a, b in zip((2e-6, 2e-5), run, ref):
-            for k in a:
-                assert float((a[k] - b[k]).norm()) <= tol * float(b[k].norm()), (tol, k)
+                grads.append(net.backward((2.0 / out.numel()) * (out - y)))
+            # strided gradients take torch's expressions
+            net.adam_step({k: torch.stack((v, v), -1)[..., 0] for k, v in grads[-1].items()} if plain else grads[-1], lr=1e-5)
+        for k, v in grads[0].items():
+            assert float((grads[1][k] - v).norm()) <= 2e-6 * float(v.norm()), k
+        assert sum(int((nets[0].wb[k] != nets[1].wb[k]).sum()) for k in nets[0].wb) <= 8
+        for net in nets:
+            net.load_state_dict({k: v.clone() for k, v in nets[0].params.items()})
 
 
 # The fused Adam pass is bit for bit torch's expressions
